@@ -18,11 +18,6 @@ using namespace gb2;
 #define GB2_VERSION_NUM 100  // 0.1.0
 #define CU GB2_CU
 
-namespace {
-constexpr size_t kCounterBytes = 4096;  // dynamic-queue counters, 128 B apart
-constexpr int kCounterStride = 32;      // ints between the counters of two classes
-}  // namespace
-
 namespace gb2 {
 
 // ---------------------------------------------------------------------------
@@ -229,8 +224,8 @@ __device__ __forceinline__ void count_key(int *counts, int key)
 }
 
 __global__ void k_classify_sw(int64_t n, SeqView q, SeqView r, const int32_t *bands, int32_t band,
-                              int fast_ok, int pack_ok, int wide_ok, int32_t match_pos,
-                              int32_t *keys, int *counts)
+                              int fast_ok, int pack_ok, int narrow_ok, int32_t match_pos,
+                              BandLut lut, int32_t *keys, int *counts)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -250,16 +245,18 @@ __global__ void k_classify_sw(int64_t n, SeqView q, SeqView r, const int32_t *ba
         else if (b == 128)
             cls = 3;
     }
+    const bool short_pack = narrow_ok && hmax <= kPackHmax && (cls == 0 || cls == 1);
     if (ql >= (1 << 21) - 1 || hmax >= (1ll << 22))
         cls = 4;
-    if (pack_ok && hmax <= kPackHmax && (cls == 0 || cls == 1))
+    const int sc = b <= kSplitMaxBand ? lut.v[b] : kNoSplit;
+    if (short_pack)
         cls = cls == 0 ? 5 : 6;
-    else if (wide_ok && hmax <= kWideHmax && cls <= 3)
-        cls = 7 + cls;
-    int64_t lb = ql >> 5;
-    if (lb > kLenBuckets - 1)
-        lb = kLenBuckets - 1;
-    const int key = cls * kLenBuckets + (kLenBuckets - 1 - (int)lb);
+    else if (pack_ok && !(sc & kNoSplit) && (hmax <= kSplitHmax || (sc & kSplitLong)))
+        cls = kSwSplit0 + (sc & kSplitClass);
+    int64_t lb = ql < 4096 ? ql >> 5 : 128 + ((ql - 4096) >> 8);
+    if (lb > kSwBuckets - 1)
+        lb = kSwBuckets - 1;
+    const int key = cls * kSwBuckets + (kSwBuckets - 1 - (int)lb);
     keys[i] = key;
     count_key(counts, key);
 }
@@ -362,6 +359,31 @@ static int classify_band(int32_t b)
 
 namespace gb2 {
 
+int sw_plan(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, const int32_t *d_bands, int32_t band,
+            int64_t n, bool fast, bool pack, bool narrow, int32_t match_pos, const BandLut &lut)
+{
+    const int nb = kSwClasses * kSwBuckets;
+    int rc;
+    if ((rc = ensure(c, x.keys, (size_t)n * 4, x.st)) ||
+        (rc = ensure(c, x.queue, (size_t)n * 4, x.st)) ||
+        (rc = ensure(c, x.counts, (size_t)nb * 4, x.st)) ||
+        (rc = ensure(c, x.seg, (size_t)kSwClasses * 2 * 8, x.st)) ||
+        (rc = ensure(c, x.counters, kCounterBytes, x.st)))
+        return rc;
+    CU(c, cudaMemsetAsync(x.counts.p, 0, (size_t)nb * 4, x.st));
+    CU(c, cudaMemsetAsync(x.counters.p, 0, kCounterBytes, x.st));
+    const int blocks = (int)((n + 255) / 256);
+    k_classify_sw<<<blocks, 256, 0, x.st>>>(n, qv, rv, d_bands, band, fast ? 1 : 0, pack ? 1 : 0,
+                                             narrow ? 1 : 0, match_pos, lut, (int32_t *)x.keys.p,
+                                             (int *)x.counts.p);
+    k_scan<<<1, 1024, 0, x.st>>>((int *)x.counts.p, nb, kSwBuckets, (int64_t *)x.seg.p);
+    k_scatter<<<blocks, 256, 0, x.st>>>(n, (const int32_t *)x.keys.p, (int *)x.counts.p,
+                                         (int32_t *)x.queue.p);
+    CU(c, cudaGetLastError());
+    c->launches += 3;
+    return GB2_OK;
+}
+
 int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,
             const gb2_sw_cfg *cfg, const int32_t *d_bands, const SwPlanInfo &pi, int64_t n,
             gb2_sw_result *d_out, int flags, bool profile)
@@ -375,9 +397,9 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
     const bool force_literal = (flags & GB2_FLAG_GENERIC) != 0;
     const bool batched = (flags & GB2_FLAG_BATCHED) != 0;
     const int variant = (flags >> 8) & 0xff;  // tuning knob (G/K choice), 0 = default
-    // per band class: the caller's variant, else the one installed by the tuner,
-    // else for a small batch (which leaves most SMs idle) the variant with the
-    // most lanes per pair, which shortens each pair's row loop; else the default
+    // int32 kernels, per band class: the caller's variant, else the one installed by
+    // the tuner, else for a small batch (which leaves most SMs idle) the variant with
+    // the most lanes per pair, which shortens each pair's row loop; else the default
     auto var_of = [&](int cls) -> int {
         if (variant)
             return variant;
@@ -409,25 +431,51 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
         return GB2_OK;
     }
     const bool pack = pi.pack_ok && !force_literal && !(flags & GB2_FLAG_INT32);
-    // Wide keys: a small batch leaves most SMs idle and its longest pair's row loop
-    // is the call's critical path, which the int32 kernels with the most lanes per
-    // pair (var_of) shorten; one thread per pair of the packed kernel does not (2,000
-    // mixed-band pairs: 2.4 ms against 4.4; one pair per call: about 1,800 against
-    // 1,100 pairs/s).  GB2_FLAG_PACKED keeps the packed kernel for small batches too.
-    const bool wide =
-        pack && pi.wide_ok && (n > kSwSmallBatch || (flags & GB2_FLAG_PACKED) != 0);
+    const bool split = pack && variant == 0;  // the variants are shapes of the int32 kernels
     const int64_t hbound = (int64_t)match_pos * (std::min(qmax, rmax) + 1);
     const bool pack_lengths = hbound <= kPackHmax;
-    const bool wide_lengths = hbound <= kWideHmax;
+    const bool long_scores = hbound > kSplitHmax;
+    // One thread per pair (sw_pack16_kernel) or the columns split over lanes: the
+    // first issues less per cell, the second finishes a pair sooner.
+    const SplitLoad load = split_load(qv, qmax, n, c->sm_count);
+    auto narrow_wins = [&](int cls, const SplitChoice &ch) {
+        return (cls == 16 || cls == 32) && pack &&
+               (!split || ch.shape < 0 || sw_pack16_cost(cls, load) <= ch.cost);
+    };
     // One band for every pair, pairs in input order: no planning kernels.
     // The batched path takes it too when the lengths are narrow (nothing to
     // sort), with a dynamic pair counter.
     if (pi.uniform_band && (!batched || pi.narrow_lengths)) {
         int cls = (pi.fast_ok && lengths_ok && !force_literal) ? classify_band(cfg->band_width) : 0;
+        const SplitChoice ch = split && cfg->band_width <= kSplitMaxBand
+                                   ? split_choose(p, cfg->band_width, load, false, long_scores)
+                                   : SplitChoice{-1, 0, 0.0};
+        int32_t low = 0, high = -1;
+        if (ch.shape >= 0 && !(pack_lengths && narrow_wins(cls, ch))) {
+            split_rebase(p, ch.shape, ch.lg, &low, &high);
+            int rc;
+            if ((rc = ensure(c, x.counters, kCounterBytes, x.st)))
+                return rc;
+            CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
+            SplitWork w{};
+            w.count = 1;
+            w.lg[0] = ch.lg;
+            w.low[0] = low;
+            w.high[0] = long_scores ? high : -1;
+            w.list[0] = PairList{nullptr, n, nullptr, (int *)x.counters.p};
+            const int64_t per = 4 * (32 >> ch.lg);
+            const int grid = (int)std::min<int64_t>(
+                (n + per - 1) / per,
+                (int64_t)c->sm_count * split_blocks_per_sm(false, ch.shape));
+            cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
+            CU(c, launch_split(false, ch.shape, qv, rv, p, cfg->band_width, nullptr, w, d_out,
+                               grid, x.st));
+            prof_end(c, e0, x.st);
+            c->launches += 1;
+            return GB2_OK;
+        }
         if ((cls == 16 || cls == 32) && pack && pack_lengths)
             cls |= kPack16;
-        else if (cls > 0 && wide && wide_lengths)
-            cls |= kPackWide;
         PairList pl{nullptr, n, nullptr, nullptr};
         int grid = 0;  // one pair per thread, pairs in input order
         if (batched && cls > 0) {  // persistent blocks taking pairs from a counter
@@ -436,7 +484,12 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
                 return rc;
             CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
             pl.counter = (int *)x.counters.p;
-            grid = c->sm_count * sw_blocks_per_sm(cls, var_of(cls));
+            // no more blocks than pairs need: in a batch smaller than one wave the warps of
+            // the SMs that start first would otherwise take every pair (50,000 reads,
+            // band 32: 281 -> 193 us)
+            const int64_t per = sw_pairs_per_block(cls, var_of(cls));
+            grid = (int)std::min<int64_t>((int64_t)c->sm_count * sw_blocks_per_sm(cls, var_of(cls)),
+                                          (n + per - 1) / per);
         }
         cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
         if (cls > 0) {
@@ -454,87 +507,143 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
         return GB2_OK;
     }
 
-    // Device planning: classify + count, scan, scatter.
-    const int nb = kSwClasses * kLenBuckets;
-    int rc;
-    if ((rc = ensure(c, x.keys, (size_t)n * 4, x.st)) ||
-        (rc = ensure(c, x.queue, (size_t)n * 4, x.st)) ||
-        (rc = ensure(c, x.counts, (size_t)nb * 4, x.st)) ||
-        (rc = ensure(c, x.seg, (size_t)kSwClasses * 2 * 8, x.st)) ||
-        (rc = ensure(c, x.counters, kCounterBytes, x.st)))
-        return rc;
-    CU(c, cudaMemsetAsync(x.counts.p, 0, (size_t)nb * 4, x.st));
-    CU(c, cudaMemsetAsync(x.counters.p, 0, kCounterBytes, x.st));
-    const int fast = (pi.fast_ok && !force_literal) ? 1 : 0;
-    const int blocks = (int)((n + 255) / 256);
-    k_classify_sw<<<blocks, 256, 0, x.st>>>(n, qv, rv, d_bands, cfg->band_width, fast,
-                                             pack ? 1 : 0, wide ? 1 : 0, match_pos,
-                                             (int32_t *)x.keys.p, (int *)x.counts.p);
-    k_scan<<<1, 1024, 0, x.st>>>((int *)x.counts.p, nb, kLenBuckets, (int64_t *)x.seg.p);
-    k_scatter<<<blocks, 256, 0, x.st>>>(n, (const int32_t *)x.keys.p, (int *)x.counts.p,
-                                         (int32_t *)x.queue.p);
-    CU(c, cudaGetLastError());
-    c->launches += 3;
-
-    // One persistent launch per class that can hold pairs; classes run
-    // concurrently on the auxiliary streams.
-    static const int cls_band[kSwClasses] = {16, 32, 64, 128, 0, 16 | kPack16, 32 | kPack16,
-                                             16 | kPackWide, 32 | kPackWide, 64 | kPackWide,
-                                             128 | kPackWide};
-    static_assert(kSwClasses * kCounterStride * 4 <= (int)kCounterBytes, "counter space");
-    bool need[kSwClasses] = {false, false, false, false, true, false,
-                             false, false, false, false, false};
-    if (pi.uniform_band) {
-        const int cb = classify_band(cfg->band_width);
-        for (int k = 0; k < 4; ++k)
-            need[k] = fast && cls_band[k] == cb;
-        need[5] = pack && cb == 16;
-        need[6] = pack && cb == 32;
-        for (int k = 0; k < 4; ++k)
-            need[7 + k] = wide && cls_band[k] == cb;
-        // when the batch's longest sequences qualify, every pair lands in one
-        // class: skip the launches that would find nothing
-        if (need[5] || need[6]) {
-            need[0] = need[0] && !pack_lengths;
-            need[1] = need[1] && !pack_lengths;
-            for (int k = 7; k < 9; ++k)
-                need[k] = need[k] && !pack_lengths;
+    // Device planning: classify + count, scan, scatter.  The lane-split class of
+    // every band the call can hold, and which of them exist.
+    const int32_t b_lo = pi.uniform_band ? cfg->band_width : 0;
+    const int32_t b_hi = pi.uniform_band ? cfg->band_width : std::max<int32_t>(pi.max_band, 0);
+    BandLut lut;
+    memset(lut.v, kNoSplit, sizeof lut.v);
+    bool present[kSplitShapes][6] = {};
+    int32_t seg_low[kSplitShapes][6] = {}, seg_high[kSplitShapes][6] = {};
+    bool all_split = split && b_hi <= kSplitMaxBand;  // no pair needs an int32 or literal kernel
+    // One thread per pair for the short pairs of a uniform band only: beside other bands
+    // its launch would wait for, or hold up, the lane-split one.
+    bool narrow = pack && (pi.uniform_band || !split);
+    if (split) {
+        // Per-pair bands run as one launch, so that its warps can take the longest pair
+        // of any band next: the shape with the least time summed over the register
+        // kernels' bands (the host does not know which bands the pairs have).
+        int shape = -1;
+        if (!pi.uniform_band) {
+            double least = 0;
+            for (int s = 0; s < kSplitShapes; ++s) {
+                double sum = 0;
+                for (int32_t b : {16, 32, 64, 128, std::min(b_hi, kSplitMaxBand)}) {
+                    const SplitChoice ch = split_choose(p, std::min(b, b_hi), load, false, false, s);
+                    sum = ch.shape < 0 ? 1e300 : sum + ch.cost;
+                }
+                if (shape < 0 || sum < least) {
+                    shape = s;
+                    least = sum;
+                }
+            }
         }
-        for (int k = 0; k < 4; ++k)
-            if (need[7 + k])
-                need[k] = need[k] && !wide_lengths;
-        need[4] = !(fast && cb > 0 && lengths_ok);
-    } else {
-        for (int k = 0; k < 4; ++k)
-            need[k] = fast && cls_band[k] <= std::max<int32_t>(pi.max_band, 0);
-        need[5] = pack && pi.max_band >= 16;
-        need[6] = pack && pi.max_band >= 32;
-        for (int k = 0; k < 4; ++k)
-            need[7 + k] = wide && (cls_band[k] & 0xff) <= std::max<int32_t>(pi.max_band, 0);
+        for (int32_t b = b_lo; b <= std::min(b_hi, kSplitMaxBand); ++b) {
+            SplitChoice ch = split_choose(p, b, load, false, long_scores, shape);
+            if (ch.shape < 0 && shape >= 0)  // long scores need another shape for this band
+                ch = split_choose(p, b, load, false, long_scores);
+            const bool any_score = long_scores && ch.shape >= 0;
+            if (ch.shape < 0)  // for the pairs whose scores stay below kSplitHmax
+                ch = split_choose(p, b, load, false, false);
+            int32_t low = 0, high = -1;
+            split_rebase(p, ch.shape, ch.lg, &low, &high);
+            lut.v[b] = (uint8_t)(ch.shape * 6 + ch.lg) | (any_score ? kSplitLong : 0);
+            present[ch.shape][ch.lg] = true;
+            seg_low[ch.shape][ch.lg] = low;
+            seg_high[ch.shape][ch.lg] = any_score ? high : -1;
+            if (long_scores && !any_score)
+                all_split = false;
+            if (pi.uniform_band && (b == 16 || b == 32) && !narrow_wins(b, ch))
+                narrow = false;
+        }
+    }
+    const int fast = (pi.fast_ok && !force_literal) ? 1 : 0;
+    int rc = sw_plan(c, x, qv, rv, d_bands, cfg->band_width, n, fast, split, narrow, match_pos, lut);
+    if (rc)
+        return rc;
+
+    // One persistent launch per class of the one-thread and int32 kernels that can
+    // hold pairs and per lane-split shape; they run concurrently on the auxiliary
+    // streams.
+    static const int cls_band[kSwSplit0] = {16, 32, 64, 128, 0, 16 | kPack16, 32 | kPack16};
+    static_assert(kSwClasses * kCounterStride * 4 <= (int)kCounterBytes, "counter space");
+    bool need[kSwSplit0] = {};
+    for (int k = 0; k < 4; ++k)
+        need[k] = fast && !all_split && cls_band[k] >= b_lo && cls_band[k] <= b_hi;
+    need[4] = !all_split;
+    need[5] = narrow && b_lo <= 16 && b_hi >= 16;
+    need[6] = narrow && b_lo <= 32 && b_hi >= 32;
+    if (pi.uniform_band) {
+        // when the batch's longest sequences qualify, every pair lands in one class
+        const int cb = classify_band(cfg->band_width);
+        if ((need[5] || need[6]) && pack_lengths) {
+            for (int k = 0; k < 5; ++k)
+                need[k] = false;
+            memset(present, 0, sizeof present);
+        }
+        if (fast && cb > 0 && lengths_ok)
+            need[4] = false;
     }
     if (need[4] && (rc = ensure_lit()))
         return rc;
     CU(c, cudaEventRecord(x.ev_fork, x.st));
     int used = 0;
     cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
-    for (int k = 0; k < kSwClasses; ++k) {
+    auto next_stream = [&](cudaStream_t &s) -> int {
+        s = x.aux[used % kAux];
+        CU(c, cudaStreamWaitEvent(s, x.ev_fork, 0));
+        return GB2_OK;
+    };
+    auto launched = [&](cudaStream_t s) -> int {
+        CU(c, cudaEventRecord(x.ev_join[used % kAux], s));
+        ++used;
+        c->launches += 1;
+        return GB2_OK;
+    };
+    cudaStream_t s;
+    for (int shape = kSplitShapes - 1; shape >= 0; --shape) {
+        SplitWork w{};
+        for (int lg = 5; lg >= 0; --lg) {
+            if (!present[shape][lg])
+                continue;
+            const int k = kSwSplit0 + shape * 6 + lg, i = w.count++;
+            w.lg[i] = lg;
+            w.low[i] = seg_low[shape][lg];
+            w.high[i] = seg_high[shape][lg];
+            w.list[i] = PairList{(const int32_t *)x.queue.p, 0, (const int64_t *)x.seg.p + 2 * k,
+                                 (int *)x.counters.p + kCounterStride * k};
+        }
+        if (w.count == 0)
+            continue;
+        if ((rc = next_stream(s)))
+            return rc;
+        const int64_t per = 4 * (32 >> w.lg[0]);  // pairs of a block with the most lanes
+        const int grid = (int)std::min<int64_t>(
+            (n + per - 1) / per, (int64_t)c->sm_count * split_blocks_per_sm(false, shape));
+        CU(c, launch_split(false, shape, qv, rv, p, cfg->band_width, d_bands, w, d_out, grid, s));
+        if ((rc = launched(s)))
+            return rc;
+    }
+    for (int k = 0; k < kSwSplit0; ++k) {
         if (!need[k])
             continue;
-        cudaStream_t s = x.aux[used % kAux];
-        CU(c, cudaStreamWaitEvent(s, x.ev_fork, 0));
+        if ((rc = next_stream(s)))
+            return rc;
         PairList pl{(const int32_t *)x.queue.p, 0, (const int64_t *)x.seg.p + 2 * k,
                     (int *)x.counters.p + kCounterStride * k};
         if (k != 4) {
-            const int grid = c->sm_count * sw_blocks_per_sm(cls_band[k], var_of(cls_band[k]));
+            const int64_t per = sw_pairs_per_block(cls_band[k], var_of(cls_band[k]));
+            const int grid = (int)std::min<int64_t>(
+                (int64_t)c->sm_count * sw_blocks_per_sm(cls_band[k], var_of(cls_band[k])),
+                (n + per - 1) / per);
             CU(c, launch_sw(cls_band[k], var_of(cls_band[k]), qv, rv, p, cfg->band_width, d_bands,
                             pl, d_out, nullptr, 0, grid, s));
         } else {
             CU(c, launch_sw(0, 0, qv, rv, p, cfg->band_width, d_bands, pl, d_out,
                             (int64_t *)x.scratch64.p, lit_stride, lit_grid, s));
         }
-        CU(c, cudaEventRecord(x.ev_join[used % kAux], s));
-        ++used;
-        c->launches += 1;
+        if ((rc = launched(s)))
+            return rc;
     }
     for (int i = 0; i < std::min(used, kAux); ++i)
         CU(c, cudaStreamWaitEvent(x.st, x.ev_join[i], 0));
@@ -578,7 +687,6 @@ int sw_validate(gb2_ctx *c, const gb2_sw_cfg *cfg, const int32_t *bands, int64_t
     pi.pack_ok = pi.fast_ok && cfg->mismatch >= goe && cfg->match_score >= cfg->mismatch &&
                  cfg->match_score <= 255 && -goe <= 255 && -cfg->gap_extend <= 255 &&
                  cfg->match_score - cfg->mismatch <= 255;
-    pi.wide_ok = pi.pack_ok && cfg->match_score <= 127;
     pi.max_band = maxb;
     pi.uniform_band = bands == nullptr;
     return GB2_OK;

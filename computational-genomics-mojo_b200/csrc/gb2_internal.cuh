@@ -67,11 +67,9 @@ struct SwParams {
     int32_t match, mismatch, go, ge;
 };
 
-// band_class flags selecting the packed int16x2 kernel: kPack16 with keys for
-// scores up to 511 (bands 16 and 32), kPackWide with group keys for scores up
-// to 4094 (bands 16, 32, 64, 128).
+// band_class flag selecting the packed int16x2 kernel of one thread per pair (bands 16
+// and 32, scores up to kPackHmax).
 constexpr int kPack16 = 0x100;
-constexpr int kPackWide = 0x200;
 
 // Smith-Waterman launch over a list of pair indices (queue == nullptr means
 // pairs [0, n)).  `bands` (device, may be nullptr) overrides `band`.
@@ -81,11 +79,60 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
                       int32_t band, const int32_t *bands, PairList pl, gb2_sw_result *out,
                       int64_t *scratch, int64_t scratch_stride, int grid, cudaStream_t st);
 
+// Any band, a pair's columns split over G = 1 << lg lanes with 2R columns each
+// (sw_split.cu).  Shapes are the register counts R; a launch of one shape takes
+// up to six segments of pairs, one per lane count, each with a counter (zeroed).
+constexpr int kSplitShapes = 8;
+constexpr int32_t kSplitMaxBand = 543;  // R = 17, 32 lanes: 1,088 columns; R = 33: 2,112
+struct SplitWork {
+    int count;
+    int lg[6];
+    // the range the pair's largest value is kept in (see the file's header); high < 0:
+    // scores stay below kSplitHmax and values are never moved
+    int32_t low[6], high[6];
+    PairList list[6];
+};
+struct SplitChoice {
+    int shape, lg;  // shape -1: none fits
+    double cost;    // estimated cycles (for choosing only)
+};
+// What a choice is made for: rows are query lengths.
+struct SplitLoad {
+    int64_t pairs;
+    double mean_rows, max_rows;
+    int sm_count;
+};
+inline SplitLoad split_load(const SeqView &q, int64_t qmax, int64_t n, int sm_count)
+{
+    // the packed words bound the mean length (a layout with gaps or shared words: qmax)
+    const double mean = 32.0 * (double)q.n_words / (double)n;
+    return SplitLoad{n, mean < (double)qmax ? mean : (double)qmax, (double)qmax, sm_count};
+}
+// Estimated cycles of a batch whose warps issue for `issue` cycles per row, or whose
+// longest pair takes `chain` cycles per row; warps per scheduler.
+double split_time(double issue, double chain, double warps, const SplitLoad &l);
+// The shape and lane count for pairs of one band; long_scores: Smith-Waterman scores may
+// pass kSplitHmax.  only_shape >= 0: that shape's lane count, or none.
+SplitChoice split_choose(const SwParams &p, int32_t band, const SplitLoad &l, bool nw,
+                         bool long_scores, int only_shape = -1);
+int split_regs(int shape);
+int split_blocks_per_sm(bool nw, int shape);
+// Whether pairs whose scores pass kSplitHmax may run: the range [low, high] the
+// pair's largest value is kept in (see the file's header) is wide enough.
+bool split_rebase(const SwParams &p, int shape, int lg, int32_t *low, int32_t *high);
+cudaError_t launch_split(bool nw, int shape, SeqView q, SeqView r, SwParams p, int32_t band,
+                         const int32_t *bands, const SplitWork &work, gb2_sw_result *out, int grid,
+                         cudaStream_t st);
+
 // The naive baseline: one 128-thread block per pair, pairs in input order
 // (grid = n), int32 band rows in shared memory (2 * (2 * max_band + 1) ints).
 constexpr int32_t kSwNaiveMaxBand = 4096;
 cudaError_t launch_sw_naive(SeqView q, SeqView r, SwParams p, int32_t band, const int32_t *bands,
                             int32_t max_band, int64_t n, gb2_sw_result *out, cudaStream_t st);
+
+// Estimated cycles of one thread per pair in the packed kernel of band 16 or 32 (the
+// same scale as SplitChoice::cost).
+double sw_pack16_cost(int band, const SplitLoad &l);
 
 // Pairs per 128-thread block, and resident blocks per SM, of a kernel variant.
 int sw_pairs_per_block(int band_class, int variant);

@@ -12,19 +12,25 @@
 namespace gb2 {
 
 constexpr int kAux = 4;            // auxiliary streams for concurrent band classes
-// 16, 32, 64, 128 (int32 registers), literal, packed 16, packed 32 (narrow keys),
-// packed 16, 32, 64, 128 (wide keys)
-constexpr int kSwClasses = 11;
-constexpr int kLenBuckets = 1024;  // length buckets per class
+// 16, 32, 64, 128 (int32 registers), literal, packed 16, packed 32 (one thread per
+// pair), then the lane-split packed kernel: shape * 6 + log2(lanes)
+constexpr int kSwSplit0 = 7;
+constexpr int kSwClasses = kSwSplit0 + gb2::kSplitShapes * 6;
+// length buckets per class: 32 bases each up to 4,096, then 256 bases each
+constexpr int kSwBuckets = 256;
+constexpr int kLenBuckets = 1024;  // WFA length buckets
 constexpr int64_t kSwSmallBatch = 16384;  // SW batches this small take the widest lane split
 constexpr int64_t kInlineScanPairs = 8192;  // host batches this small are scanned inline
 constexpr int64_t kPinChunk = 32ll << 20;
 // Packed int16x2 kernels: every cell they compute (the in-matrix ones, and the
 // row past the query end, which adds at most `match`) stays below these, checked
 // as match * (min(qlen, rlen) + 1): H*128 + column fits 16 bits (narrow keys),
-// H*8 + 7 fits a signed 16-bit half (wide keys).
+// H*8 + 7 fits a signed 16-bit half (the lane-split kernel, which moves its values'
+// base for longer pairs).
 constexpr int64_t kPackHmax = 511;
-constexpr int64_t kWideHmax = 4094;
+constexpr int64_t kSplitHmax = 4094;
+constexpr size_t kCounterBytes = 8192;  // dynamic-queue counters, 128 B apart
+constexpr int kCounterStride = 32;      // ints between the counters of two classes
 constexpr int64_t kWfaScratchCap = 8ll << 30;  // WFA rings of all warps, bytes
 constexpr int64_t kWfaTeamMinLen = 2048;       // shortest WFA pair aligned by a whole block
 constexpr int64_t kTierDumpCap = 1ll << 30;    // bytes of suspended-pair records per transition
@@ -118,7 +124,6 @@ struct GraphCache {
 struct SwPlanInfo {
     bool fast_ok;       // the register kernels apply (sign conditions on the scores)
     bool pack_ok;       // the packed int16x2 kernel applies (scores also small)
-    bool wide_ok;       // ... and with its wide keys (match <= 127)
     int32_t max_band;
     bool uniform_band;  // no per-pair bands
     // set by the caller when every pair's lengths lie in a narrow range: a
@@ -250,6 +255,18 @@ void harvest_profile(gb2_ctx *c);
 
 int sw_validate(gb2_ctx *c, const gb2_sw_cfg *cfg, const int32_t *bands, int64_t n, int64_t qmax,
                 int64_t rmax, SwPlanInfo &pi);
+// Per band 0..kSplitMaxBand: the lane-split class shape * 6 + log2(lanes) that its
+// pairs take (kNoSplit: none), kSplitLong set where pairs of any score may run.
+struct BandLut {
+    uint8_t v[kSplitMaxBand + 1];
+};
+constexpr uint8_t kNoSplit = 0x80, kSplitLong = 0x40, kSplitClass = 0x3f;
+// Queues the pairs of (qv, rv) in x.queue by class, longest first, with each class's
+// [start, end) in x.seg (kSwClasses segments) and zeroed counters in x.counters.
+// fast / pack / narrow: the int32 register kernels, the packed kernels, the
+// one-thread-per-pair packed kernel may be used.
+int sw_plan(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, const int32_t *d_bands, int32_t band,
+            int64_t n, bool fast, bool pack, bool narrow, int32_t match_pos, const BandLut &lut);
 // Enqueues Smith-Waterman for n pairs of (qv, rv) on executor x; results to d_out.
 // profile: record the launches' duration when the context is profiling.
 int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,

@@ -169,7 +169,7 @@ int gcd_i(int a, int b)
 int64_t group_bytes(const Layout &l, const gb2_wfa_cfg &w, int sm_count)
 {
     int64_t b = align_up(l.in_bytes) + align_up(l.out_bytes);
-    b += l.n_sw * 8 + (int64_t)kSwClasses * kLenBuckets * 4 + 8192;  // keys, queue, counts
+    b += l.n_sw * 8 + (int64_t)kSwClasses * kSwBuckets * 4 + 12288;  // keys, queue, counts
     if (l.n_sw) {
         const int64_t lit_grid = std::min<int64_t>((l.n_sw + 127) / 128, (int64_t)sm_count * 2);
         b += lit_grid * 128 * 3 * (2 * (int64_t)l.max_band + 1) * 8;

@@ -292,10 +292,6 @@ struct Pack16Consts {
     uint32_t neg_g2; // minus -(go+ge) in both halves, mod 2^32
     uint32_t ge2;    // ge in both halves
     uint32_t ng2;    // -(go+ge) in both halves
-    // the wide-key multipliers stay last: with them placed before x128 the narrow
-    // band-32 kernel measured 9% slower (665 vs 610 us per 262,144-pair launch,
-    // same registers)
-    uint32_t x8, x32;
 };
 
 __device__ __forceinline__ uint32_t mad_hi_u32(uint32_t a, uint32_t b, uint32_t c)
@@ -328,42 +324,17 @@ __device__ __forceinline__ uint32_t seq_word16(const SeqView &s, int64_t off, in
 // the step lies inside the matrix (the common case); MASK = true zeroes the
 // first-maximum keys of cells past the query or reference end.  Returns the
 // packed row keys: low half row t, high half row t-1.
-//
-// WIDE keys (scores up to 4094, bands 16..128): the key H*128 + column of the
-// narrow form needs H <= 511 and 2B+1 <= 128 columns.  The wide form keys a
-// cell as H*8 + (7 - h%8) (no carry between halves while H <= 8191), takes
-// the maximum over each group of 8 registers, and turns each group's maximum
-// into relu(gk - 8*base) with one DPX instruction, base = the best score of
-// the rows already resolved: a cell can only become the new best when
-// H > base, and then H - base <= 2*match (a row's maximum exceeds the
-// previous row's by at most `match`).  The group key
-//   (H - base) * 256 + (31 - group) * 8 + (7 - h%8)
-// fits 16 bits for match <= 127, and its maximum over the groups is the
-// first maximum of the half; group keys below 256 mean "nothing above base".
-// Per register this costs what the narrow key costs (one multiply-add and
-// half a 3-way max); the DPX relu, two logic ops and a multiply-add run once
-// per group.
-template <int B, bool MASK, bool WIDE>
+template <int B, bool MASK>
 __device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const uint32_t *eq,
                                                  const uint32_t *bw, uint32_t &e_last, int limL,
-                                                 int limH, const Pack16Consts &c,
-                                                 uint32_t negbase8)
+                                                 int limH, const Pack16Consts &c)
 {
     constexpr int NL = B + 1, R = NL;
-    // Bands 64 and 128 are register-bound to 12 and 8 warps per SM, too few to
-    // hide the latency of the left-to-right chain through a row: there the
-    // H update is grouped so that only the 3-way max waits on the left
-    // neighbour (two dependent instructions per register instead of three).
-    // Measured on 1,000,000 reads: band 128 2,723 -> 2,901 GCUPS, band 64
-    // 3,613 -> 3,655; the narrow bands 16 and 32 (20 warps per SM) are 4%
-    // faster with the other grouping.
-    constexpr bool SHORT_CHAIN = B >= 64;
     const uint32_t SENT = 0x0000C000u;
     uint32_t hl = Hr[R - 1] << 16;                    // low: band edge 0; high: H(t-1, B)
     uint32_t el = __byte_perm(SENT, e_last, 0x5410);  // low: chain start; high: E'(t-1, B)
     uint32_t h0new = 0;
     uint32_t rk = 0, kpend = 0;
-    uint32_t gacc = 0, gpend = 0, g2pend = 0;  // WIDE: group maximum, pending keys
 #pragma unroll
     for (int h = 0; h < R; ++h) {
         const int k = h >> 4, j = h & 15, jj = h & 7;
@@ -376,14 +347,8 @@ __device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const ui
             mad_hi_u32(wv & ((1u << pos) | (1u << (pos + 16))), c.dm[jj & 3], c.mmg2);
         const uint32_t up = (h + 1 < R) ? Hr[h + 1 < R ? h + 1 : h] : (h0new >> 16);
         const uint32_t e = __viaddmax_s16x2(el, c.ge2, up);
-        uint32_t hn;
-        if (!SHORT_CHAIN) {
-            const uint32_t tt = __vimax3_s16x2(e, hl, c.ng2);
-            hn = __viaddmax_s16x2(Hr[h], sub, tt) * c.one + c.neg_g2;
-        } else {
-            const uint32_t a = __viaddmax_s16x2(Hr[h], sub, e);
-            hn = __vimax3_s16x2(a, hl, c.ng2) * c.one + c.neg_g2;
-        }
+        const uint32_t tt = __vimax3_s16x2(e, hl, c.ng2);
+        uint32_t hn = __viaddmax_s16x2(Hr[h], sub, tt) * c.one + c.neg_g2;
         hl = hn;
         if (h == R - 1)
             hn &= 0x0000FFFFu;  // padding column stays 0
@@ -391,58 +356,22 @@ __device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const ui
             h0new = hn;
         Hr[h] = hn;
         el = e;
-        if (!WIDE) {
-            uint32_t key =
-                hn * c.x128 + (((uint32_t)(127 - h)) | ((uint32_t)(127 - NL - h) << 16));
-            if (MASK)
-                key &= (h < limL ? 0x0000FFFFu : 0u) | (h < limH ? 0xFFFF0000u : 0u);
-            if (h & 1)
-                rk = __vimax3_u16x2(rk, kpend, key);
-            else
-                kpend = key;
-        } else {
-            const int i = h & 7, g = h >> 3;
-            const uint32_t t8 = 7u - (uint32_t)i;
-            uint32_t key = hn * c.x8 + (t8 | (t8 << 16));
-            if (MASK)
-                key &= (h < limL ? 0x0000FFFFu : 0u) | (h < limH ? 0xFFFF0000u : 0u);
-            if (i == 0)
-                gacc = key;
-            else if (i & 1)
-                gpend = key;
-            else
-                gacc = __vimax3_u16x2(gacc, gpend, key);
-            if (i == 7 || h == R - 1) {
-                if (i & 1)
-                    gacc = __vimax3_u16x2(gacc, gpend, gpend);
-                const uint32_t ck = __viaddmax_s16x2_relu(gacc, negbase8, 0u);
-                const uint32_t cg = (uint32_t)((31 - g) * 8) * 0x00010001u;
-                const uint32_t k2 = (ck & 0xFFF8FFF8u) * c.x32 + ((ck & 0x00070007u) | cg);
-                if (g & 1)
-                    rk = __vimax3_u16x2(rk, g2pend, k2);
-                else
-                    g2pend = k2;
-            }
-        }
+        uint32_t key = hn * c.x128 + (((uint32_t)(127 - h)) | ((uint32_t)(127 - NL - h) << 16));
+        if (MASK)
+            key &= (h < limL ? 0x0000FFFFu : 0u) | (h < limH ? 0xFFFF0000u : 0u);
+        if (h & 1)
+            rk = __vimax3_u16x2(rk, kpend, key);
+        else
+            kpend = key;
     }
-    if (!WIDE) {
-        if ((R - 1) % 2 == 0)
-            rk = __vimax3_u16x2(rk, kpend, kpend);
-    } else {
-        constexpr int NG = (R + 7) / 8;
-        if ((NG - 1) % 2 == 0)
-            rk = __vimax3_u16x2(rk, g2pend, g2pend);
-    }
+    if ((R - 1) % 2 == 0)
+        rk = __vimax3_u16x2(rk, kpend, kpend);
     e_last = el;
     return rk;
 }
 
-// Band 128 is register-bound to two blocks per SM either way; with the
-// minimum-blocks hint of 1 the compiler schedules it in 254 registers instead
-// of 251 and the kernel measured 6% faster (2,734 vs 2,583 GCUPS).  The other
-// widths keep the default schedule (hint 0).
-template <int B, bool WIDE>
-__global__ void __launch_bounds__(128, (B == 128) ? 1 : 0)
+template <int B>
+__global__ void __launch_bounds__(128)
 sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_result *__restrict__ out)
 {
     static_assert(B % 16 == 0, "band must be a multiple of 16");
@@ -453,8 +382,7 @@ sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_resul
     constexpr int BW0 = NL / 16;        // first word of columns B+1.. (offset one column)
     constexpr int NBW = B / 16;         // shifted words of the previous row
     constexpr int RW0 = NE - B / 16;    // 16-base word entering the window at t = 0
-    static_assert(WIDE || W <= 127, "column index must fit the narrow key");
-    static_assert(!WIDE || (R + 7) / 8 <= 32, "group index must fit the wide key");
+    static_assert(W <= 127, "column index must fit the key");
     static_assert(NL % 16 == 1 && BW0 + NBW < NE, "word layout");
 
     int64_t n;
@@ -502,8 +430,6 @@ sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_resul
             uint32_t e_last = SENT;
             uint32_t saved_lowkey = 0, bestkey = 0, thr = 127;
             int32_t bq = 0;
-            // WIDE: best score, its column, and the base the saved key was taken at
-            int32_t best = 0, bcol = 0, base_prev = 0;
             uint32_t qw = 0, rw = 0;
             uint32_t qn = seq_word16(q, qoff, 0), rn = seq_word16(r, roff, RW0);  // next words
             const int steps = qlen > 0 ? qlen + 1 : 0;
@@ -555,51 +481,24 @@ sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_resul
                     if (t >= 1 && t - 1 < qlen)
                         limH = max(0, min(R, rlen - (t - 1 - B + NL)));
                 }
-                // WIDE keys are relative to the best score of rows <= t-2
-                const uint32_t negbase8 = (uint32_t)(uint16_t)(-8 * best) * 0x00010001u;
                 const uint32_t rk =
-                    full ? pack16_cells<B, false, WIDE>(Hr, eq, bw, e_last, 0, 0, c, negbase8)
-                         : pack16_cells<B, true, WIDE>(Hr, eq, bw, e_last, limL, limH, c,
-                                                       negbase8);
-                if (!WIDE) {
-                    // row t-1 is complete: its first half came one step earlier; a key
-                    // above thr = bestkey | 127 has a larger H than the best so far
-                    const uint32_t rowkey = max(saved_lowkey, rk >> 16);
-                    if (rowkey > thr) {
-                        thr = rowkey | 127u;
-                        bestkey = rowkey;
-                        bq = t - 1;
-                    }
-                    saved_lowkey = rk & 0xFFFFu;
-                } else {
-                    // the saved low half of row t-1 was keyed against base_prev: rebase
-                    // it to this step's base; then the low half wins ties (its columns
-                    // come first)
-                    const uint32_t dsh = (uint32_t)(best - base_prev) << 8;
-                    const uint32_t sl = saved_lowkey >= dsh + 256u ? saved_lowkey - dsh : 0u;
-                    const uint32_t hi = rk >> 16;
-                    const int32_t dl = (int32_t)(sl >> 8), dh = (int32_t)(hi >> 8);
-                    base_prev = best;
-                    if (dl > 0 || dh > 0) {
-                        if (dl >= dh) {
-                            best += dl;
-                            bcol = 255 - (int32_t)(sl & 255u);
-                        } else {
-                            best += dh;
-                            bcol = NL + 255 - (int32_t)(hi & 255u);
-                        }
-                        bq = t - 1;
-                    }
-                    saved_lowkey = rk & 0xFFFFu;
+                    full ? pack16_cells<B, false>(Hr, eq, bw, e_last, 0, 0, c)
+                         : pack16_cells<B, true>(Hr, eq, bw, e_last, limL, limH, c);
+                // row t-1 is complete: its first half came one step earlier; a key
+                // above thr = bestkey | 127 has a larger H than the best so far
+                const uint32_t rowkey = max(saved_lowkey, rk >> 16);
+                if (rowkey > thr) {
+                    thr = rowkey | 127u;
+                    bestkey = rowkey;
+                    bq = t - 1;
                 }
+                saved_lowkey = rk & 0xFFFFu;
 #pragma unroll
                 for (int i = 0; i < NE; ++i)
                     ep[i] = eq[i];
             }
-            if (!WIDE) {
-                best = (int32_t)(bestkey >> 7);
-                bcol = 127 - (int32_t)(bestkey & 127u);
-            }
+            const int32_t best = (int32_t)(bestkey >> 7);
+            const int32_t bcol = 127 - (int32_t)(bestkey & 127u);
             gb2_sw_result res;
             res.score = best;
             res.query_end = best > 0 ? bq : 0;
@@ -799,23 +698,19 @@ static int occ_band()
     return nb > 0 ? nb : 1;
 }
 
-template <int B, bool WIDE>
+template <int B>
 static int occ_pack16()
 {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sw_pack16_kernel<B, WIDE>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sw_pack16_kernel<B>, 128, 0);
     return nb > 0 ? nb : 1;
 }
 
 int sw_blocks_per_sm(int band_class, int variant)
 {
     switch (band_class) {
-    case 16 | kPack16: return occ_pack16<16, false>();
-    case 32 | kPack16: return occ_pack16<32, false>();
-    case 16 | kPackWide: return occ_pack16<16, true>();
-    case 32 | kPackWide: return occ_pack16<32, true>();
-    case 64 | kPackWide: return occ_pack16<64, true>();
-    case 128 | kPackWide: return occ_pack16<128, true>();
+    case 16 | kPack16: return occ_pack16<16>();
+    case 32 | kPack16: return occ_pack16<32>();
     case 16: return variant == 1 ? occ_band<16, 2, 17>() : occ_band<16, 1, 33>();
     case 32:
         return variant == 1 ? occ_band<32, 2, 33>()
@@ -831,11 +726,7 @@ int sw_pairs_per_block(int band_class, int variant)
     int G = 1;
     switch (band_class) {
     case 16 | kPack16:
-    case 32 | kPack16:
-    case 16 | kPackWide:
-    case 32 | kPackWide:
-    case 64 | kPackWide:
-    case 128 | kPackWide: return 128;
+    case 32 | kPack16: return 128;
     case 16: G = variant == 1 ? 2 : 1; break;
     case 32: G = variant == 1 ? 2 : (variant == 2 ? 4 : 1); break;
     case 64: G = variant == 1 ? 4 : 2; break;
@@ -845,6 +736,13 @@ int sw_pairs_per_block(int band_class, int variant)
     return 4 * (32 / G);
 }
 
+double sw_pack16_cost(int band, const SplitLoad &l)
+{
+    // 573 cycles per warp and row at band 32 (1,000,000 reads)
+    return split_time(17.4 * (band + 1), 24.5 * (band + 1) + 190,
+                      (double)l.pairs / 32 / (4.0 * l.sm_count), l);
+}
+
 // variant selects (G, K) for a band class: 0 = default.
 cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParams p, int32_t band,
                       const int32_t *bands, PairList pl, gb2_sw_result *out, int64_t *scratch,
@@ -852,11 +750,7 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
 {
     switch (band_class) {
     case 16 | kPack16:
-    case 32 | kPack16:
-    case 16 | kPackWide:
-    case 32 | kPackWide:
-    case 64 | kPackWide:
-    case 128 | kPackWide: {
+    case 32 | kPack16: {
         int g = grid;
         if (g <= 0) {
             if (pl.seg || pl.n <= 0)
@@ -867,8 +761,6 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
         Pack16Consts c;
         c.one = 1;
         c.x4 = 4;
-        c.x8 = 8;
-        c.x32 = 32;
         c.x128 = 128;
         c.x256 = 256;
         c.half = 0x80000000u;
@@ -878,14 +770,10 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
         c.neg_g2 = 0u - gg * 0x00010001u;
         c.ge2 = (uint32_t)(uint16_t)p.ge * 0x00010001u;
         c.ng2 = (uint32_t)(uint16_t)gg * 0x00010001u;
-        switch (band_class) {
-        case 16 | kPack16: sw_pack16_kernel<16, false><<<g, 128, 0, st>>>(q, r, c, pl, out); break;
-        case 32 | kPack16: sw_pack16_kernel<32, false><<<g, 128, 0, st>>>(q, r, c, pl, out); break;
-        case 16 | kPackWide: sw_pack16_kernel<16, true><<<g, 128, 0, st>>>(q, r, c, pl, out); break;
-        case 32 | kPackWide: sw_pack16_kernel<32, true><<<g, 128, 0, st>>>(q, r, c, pl, out); break;
-        case 64 | kPackWide: sw_pack16_kernel<64, true><<<g, 128, 0, st>>>(q, r, c, pl, out); break;
-        default: sw_pack16_kernel<128, true><<<g, 128, 0, st>>>(q, r, c, pl, out); break;
-        }
+        if (band_class == (16 | kPack16))
+            sw_pack16_kernel<16><<<g, 128, 0, st>>>(q, r, c, pl, out);
+        else
+            sw_pack16_kernel<32><<<g, 128, 0, st>>>(q, r, c, pl, out);
         return cudaGetLastError();
     }
     case 16:

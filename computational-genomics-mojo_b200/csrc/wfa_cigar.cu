@@ -117,7 +117,7 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
         all_rec += rec[(size_t)i];
     const int64_t arena_bytes = std::max<int64_t>(16, std::min(budget, all_rec));
     if ((rc = ensure(c, x.scratch32, (size_t)(grid * 4 * warp_bytes), x.st)) ||
-        (rc = ensure(c, x.counters, 4096, x.st)) ||
+        (rc = ensure(c, x.counters, kCounterBytes, x.st)) ||
         (rc = ensure(c, cb.arena, (size_t)arena_bytes, x.st)) ||
         (rc = ensure(c, cb.pairs, (size_t)n * 4, x.st)) ||
         (rc = ensure(c, cb.arena_off, (size_t)n * 8, x.st)) ||
