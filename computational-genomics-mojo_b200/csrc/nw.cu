@@ -194,10 +194,37 @@ int nw_blocks_per_sm()
 
 using namespace gb2;
 
+// The shape and lane count of the lane-split kernel (sw_split.cu) for bands up to
+// maxb, or -1: its right padding needs mismatch >= 2 * (go + ge) and gap terms that
+// are not gains, its packed score steps match - mismatch <= 255, and every value
+// H + g * (qi + ri), re-centred by 2g per row every 16 rows, must lie between the
+// 16-bit limit and the floor that stands for cells outside the matrix.
+static int nw_split_shape(const SwParams &p, int64_t maxb, int64_t qmax, int64_t rmax,
+                          const SplitLoad &load, int &lg)
+{
+    const int64_t g = -((int64_t)p.go + p.ge), mm = p.mismatch, m = p.match;
+    if (maxb > kSplitMaxBand || g < 0 || g > 255 || p.ge > 0 || mm < -2 * g || mm > 255 || m < mm ||
+        m - mm > 255)
+        return -1;
+    const SplitChoice ch = split_choose(p, (int32_t)maxb, load, true, false);
+    if (ch.shape < 0)
+        return -1;
+    const int64_t G = 1 << ch.lg, cols = 2 * (int64_t)split_regs(ch.shape) * G;
+    const int64_t len = std::min(qmax, rmax) + 1, mp = std::max<int64_t>(m, 0);
+    const int64_t drift = g * (36 + 4 * G + 2 * maxb + cols);
+    const int64_t top = mp * len + drift;
+    const int64_t bottom = std::max<int64_t>(-mm, 0) * len + g * (maxb + 2) +
+                           std::abs((int64_t)p.go) - maxb * p.ge + drift + 18 * (mp + 2 * g);
+    if (top > 32000 || bottom > 30500)
+        return -1;
+    lg = ch.lg;
+    return ch.shape;
+}
+
 // Runs NW over n resident pairs into d_out (device); blocking.
 static int nw_core(gb2_ctx *c, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,
                    const gb2_sw_cfg *cfg, const int32_t *h_bands, int64_t n,
-                   gb2_sw_result *d_out, int flags)
+                   gb2_sw_result *d_out, int flags, bool narrow_lengths)
 {
     if (!cfg)
         return set_err(c, GB2_EINVAL, "cfg is NULL");
@@ -222,10 +249,50 @@ static int nw_core(gb2_ctx *c, SeqView qv, SeqView rv, int64_t qmax, int64_t rma
     Exec &x = c->x;
     const SwParams p{cfg->match_score, cfg->mismatch, cfg->gap_open, cfg->gap_extend};
     const int32_t band = cfg->band_width;
+    int lg = 0;
+    const int shape = (flags & GB2_FLAG_GENERIC) ? -1
+                                                 : nw_split_shape(p, maxb, qmax, rmax, split_load(qv, qmax, n, c->sm_count), lg);
+    if (shape >= 0) {
+        const int32_t *d_bands = nullptr;
+        int rc;
+        if (h_bands) {
+            if ((rc = ensure(c, c->bands, (size_t)n * 4, x.st)) ||
+                (rc = h2d(c, c->bands.p, h_bands, (size_t)n * 4, x.st)))
+                return rc;
+            d_bands = (const int32_t *)c->bands.p;
+        }
+        SplitWork w{};
+        w.count = 1;
+        w.lg[0] = lg;
+        w.high[0] = -1;
+        const int64_t per = 4 * (32 >> lg);
+        // Pairs of a warp run as many rows as the longest of them: queue ragged pairs
+        // by length, when there is more than one group of them per warp scheduler.
+        if (!narrow_lengths && n > (int64_t)c->sm_count * per) {
+            const int k = kSwSplit0 + shape * 6 + lg;
+            BandLut lut;
+            for (uint8_t &v : lut.v)
+                v = (uint8_t)(shape * 6 + lg);
+            if ((rc = sw_plan(c, x, qv, rv, nullptr, 0, n, false, true, false, 0, lut)))
+                return rc;
+            w.list[0] = PairList{(const int32_t *)x.queue.p, 0, (const int64_t *)x.seg.p + 2 * k,
+                                 (int *)x.counters.p + kCounterStride * k};
+        } else {
+            if ((rc = ensure(c, x.counters, kCounterBytes, x.st)))
+                return rc;
+            GB2_CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
+            w.list[0] = PairList{nullptr, n, nullptr, (int *)x.counters.p};
+        }
+        const int grid = (int)std::min<int64_t>(
+            (n + per - 1) / per, (int64_t)c->sm_count * split_blocks_per_sm(true, shape));
+        GB2_CU(c, launch_split(true, shape, qv, rv, p, band, d_bands, w, d_out, grid, x.st));
+        c->launches += 1;
+        return GB2_OK;
+    }
     const bool reg = !h_bands && (band == 16 || band == 32) && !(flags & GB2_FLAG_GENERIC);
     if (reg) {
         int rc;
-        if ((rc = ensure(c, x.counters, 4096, x.st)))
+        if ((rc = ensure(c, x.counters, kCounterBytes, x.st)))
             return rc;
         GB2_CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
         const int per = band == 16 ? nw_blocks_per_sm<16>() : nw_blocks_per_sm<32>();
@@ -278,7 +345,8 @@ static int gb2_nw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
     const SeqView qv{q->d_packed, q->d_offsets, q->d_lengths, 0, q->n_words};
     const SeqView rv{r->d_packed, r->d_offsets, r->d_lengths, 0, r->n_words};
     if ((rc = nw_core(c, qv, rv, q->max_len, r->max_len, cfg, bands, n,
-                      (gb2_sw_result *)c->out_sw.p, flags)))
+                      (gb2_sw_result *)c->out_sw.p, flags,
+                      narrow_range(q->min_len, q->max_len) && narrow_range(r->min_len, r->max_len))))
         return rc;
     GB2_CU(c, cudaMemcpyAsync(out, c->out_sw.p, (size_t)n * sizeof(gb2_sw_result),
                               cudaMemcpyDeviceToHost, c->x.st));
