@@ -6,6 +6,7 @@
 // bucketing of pair lists, the chunked host-to-device pipeline of the
 // end-to-end entry points, and the per-pair drop-in calls.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <functional>
@@ -747,15 +748,22 @@ static int wfa_block_warps(int64_t qmax, int64_t rmax, int64_t n, int variant)
     return n <= kWfaWideMaxPairs && std::max(qmax, rmax) >= kWfaWideTeamLen ? kWfaWideWarps : 4;
 }
 
-// Tiered WFA (wfa_tiers.cu): every pair starts on the smallest team whose
-// launch still fills the GPU -- one warp for large batches, four warps for up
-// to 16 pairs per SM, eight for up to two per SM, sixteen for one, so a single
-// long pair (the per-call drop-in) gets a whole SM -- and moves up a tier
-// (1, 2, 4, 8, 16 warps) when its wavefront outgrows the window; pairs that
-// outgrow the last or need int32 rows
-// finish in G.  One launch per tier from the first, in order on x.st; the
-// launches after the first take their pair count from the device.  With
-// GB2_FLAG_BATCHED the first tier's queue is ordered longest first.
+// Tiered WFA (wfa_tiers.cu): pairs start on a team of one, four or eight warps and move
+// up a tier (1, 2, 4, 8, 16 warps) when their wavefront outgrows the window; pairs that
+// outgrow the last or need int32 rows finish in G.  One launch per tier from the first,
+// in order on x.st; the launches after the first take their pair count from the device.
+// With GB2_FLAG_BATCHED the first tier's queue is ordered longest first.
+//
+// The first tier: one warp per pair costs the least work, more warps the least time for
+// the longest pair.  What decides is how many pairs as long as the longest the batch
+// amounts to, by the square of the length (the mean over the longest to the power 1.5
+// estimates that from the packed words).  Measured, 1 / 4 / 8 warps first (ms):
+//   100-10,000 bp, 300 pairs (30 such)  4.39 / 2.87 / 2.58;  4,000 (400) 6.26 / 4.56 / 4.48
+//   8,000 (800) 7.5 / 7.5 / 8.9;  12,000 (1,200) 8.9 / 10.4 / 13.2
+//   100-1,500 bp, 3,000 (610) 0.57 / 0.44 / 0.69;  8,000 (1,600) 0.73 / 0.95 / 1.62
+//   8,000-10,000 bp, 2,000 (1,700) 10.1 / 11.6 / 13.5
+// so one warp above 6 per SM, four above 2.7, else eight (a single pair, the per-call
+// drop-in: sixteen warps took 0.68 ms for 4,000 bp, eight 0.62).
 static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,
                      const WfaParams &p, int64_t n, int32_t *d_out, int flags, int32_t *d_ub)
 {
@@ -767,7 +775,10 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     if (n < kWfaTwoWarpMinPairsPerSm * sms)
         pl.usable[1] = false;
     constexpr int G = kWfaShared;  // the global-memory tier
-    int first = n <= sms ? 4 : (n <= 2 * sms ? 3 : (n <= 16 * sms ? 2 : 0));
+    const double longest = (double)std::max<int64_t>({qmax, rmax, 1});
+    const double mean = std::min(32.0 * (double)std::max(qv.n_words, rv.n_words) / (double)n, longest);
+    const double alike = (double)n * std::pow(mean / longest, 1.5) / (double)sms;
+    int first = alike > 6.0 ? 0 : (alike > 2.7 ? 2 : 3);
     while (first < G && !pl.usable[first])
         ++first;
     auto next_of = [&](int t) {
@@ -821,7 +832,6 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         list = (const int32_t *)x.queue.p;
         seg = (const int64_t *)x.seg.p;
     }
-    static const int teams_per_block[G + 1] = {16, 8, 4, 2, 1, 1};
     int prev = -1;  // the tier launched before t: its suspended pairs are t's entries
     for (int t = first; t <= G; ++t) {
         if (t < G && !pl.usable[t])
@@ -856,8 +866,9 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         io.gring = (int32_t *)x.scratch32.p;
         // the tiers after the first prune by the bound pass's costs
         io.ubound = (d_ub && t > 0) ? d_ub : nullptr;
-        const int64_t per = teams_per_block[t];
-        const int grid = (int)(t == first ? std::min<int64_t>(sms, (n + per - 1) / per) : sms);
+        // a team's first pair is the one of its place in the grid: as many blocks as there
+        // are pairs spread a small batch over the SMs
+        const int grid = (int)(t == first ? std::min<int64_t>(sms, n) : sms);
         cudaEvent_t e0 = prof_begin(c, x.st);
         CU(c, launch_wfa_tier(pl, t, grid, qv, rv, p, io, d_out, (int64_t *)x.work.p,
                               (int *)x.errflag.p, x.st));

@@ -163,7 +163,7 @@ constexpr int kWfaShared = 5;  // tiers with their rings in shared memory
 struct WfaTierPlan {
     int nslot;
     int32_t W[kWfaShared + 1], H[kWfaShared + 1];  // window per slot row; element of diagonal 0
-    int32_t seq_cap[kWfaShared + 1];     // 16-base window entries of a sequence copy
+    int32_t seq_cap[kWfaShared + 1];     // 16-base words of a sequence copy
     int64_t team_bytes[kWfaShared + 1];  // shared bytes per team
     int64_t ring_bytes[kWfaShared + 1];  // of them, the ring
     int64_t dump_stride[kWfaShared];     // bytes of a suspended pair's record, per source tier

@@ -12,20 +12,29 @@
 // reaches one diagonal further per step), so the window fills from its
 // centre outwards and every element is NEG-filled once when the pair starts;
 // afterwards each step only overwrites its own interval and turns what the
-// reused slot held outside it back into NEG.  Reads at k-1 and k+1 therefore
-// need no bounds tests, and the neighbours of a diagonal are fixed offsets.
+// reused slot held outside it back into NEG where a later step could read it.
+// Reads at k-1 and k+1 therefore need no bounds tests.
+//
+// A step.  A thread takes groups of four (or, for the last round, two)
+// neighbouring diagonals: rows come in as 8-byte loads, the recurrences are
+// 16-bit-pair DPX on two diagonals per register, and only the extension is per
+// diagonal (wf_group).  The intervals are packed (lo, -hi) pairs, so that unions,
+// widening and clipping are single DPX instructions too.  Before, every thread took
+// single diagonals TW apart: 20,000 pairs of 100-10,000 bp went from 16.5 to 11.9 ms,
+// of which the groups 16.5 -> 13.9 (with the packed intervals), the sequence copies
+// below 13.9 -> 12.4, one inlined extension loop for a lane's diagonals 12.4 -> 12.1.
 //
 // Tiers.  Work per pair grows with the square of its cost (most pairs are
-// cheap, most cells are in the few expensive ones), so a pair starts on the
-// smallest team and moves up when its interval outgrows the window:
-//   T1   one warp per pair,      sixteen per block, W = 616  (x4 o6 e2)
-//   T2   two warps per pair,     eight per block,   W = 1,240
-//   T4   four warps per pair,    four per block,    W = 2,488
-//   T8   eight warps per pair,   two per block,     W = 4,984
-//   T16  sixteen warps per pair, one per block,     W = 9,968
+// cheap, most cells are in the few expensive ones), so a pair starts on a
+// small team and moves up when its interval outgrows the window:
+//   T1   one warp per pair,      sixteen per block, W = 632  (x4 o6 e2)
+//   T2   two warps per pair,     eight per block,   W = 1,264
+//   T4   four warps per pair,    four per block,    W = 2,760
+//   T8   eight warps per pair,   two per block,     W = 5,536
+//   T16  sixteen warps per pair, one per block,     W = 11,976
 // each in its own launch, one after another on the executor's stream.  A
 // pair whose next step would read or write outside its window is suspended:
-// the team writes its state (slot intervals, step, ring contents over the
+// the team writes its state (step intervals, step, ring contents over the
 // live span) to a dump record in HBM and queues the pair for the next tier,
 // whose launch restores it into its larger window and continues from the
 // same step.  No cell is computed twice.  A pair that outgrows T16, or whose
@@ -35,10 +44,14 @@
 // When the dump space of a transition is used up, the pair starts over in
 // the next tier instead (same results, more work).
 //
-// Sequences are copied into shared memory as overlapping 64-bit windows
-// (entry j = 16-base halves j and j+1), so a 16-base window at any position
-// is one 64-bit load and one funnel shift; pairs longer than a tier's copy
-// capacity read their windows from the packed words in global memory.
+// Sequences are copied into shared memory as 16-base words, so a 16-base window at
+// any position is two neighbouring words and one funnel shift; pairs longer than a
+// tier's copy capacity read their windows from the packed words in global memory.
+//
+// Bound: instruction issue.  Per warp and step about 100 instructions of bookkeeping,
+// 139 per round of four diagonals a lane (82 of two) of which the extension's two window
+// loads, shifts, compare and clamps are 80, and about 100 for the lanes whose whole first
+// window matched.  At the sizes above T1 issues 69% of its slots, T4 62%.
 #include <type_traits>
 
 #include "gb2_internal.cuh"
@@ -77,14 +90,6 @@ __device__ __forceinline__ Shape make_shape(const WfaParams &p)
     w.nslot = w.hm + 2 * w.hie;
     return w;
 }
-
-template <typename RT> struct Neg;
-template <> struct Neg<int16_t> {
-    static constexpr int32_t value = -32768;
-};
-template <> struct Neg<int32_t> {
-    static constexpr int32_t value = -(1 << 30);
-};
 
 // ---- team synchronisation ----------------------------------------------------
 // TEAM warps align one pair; a block holds NTEAMS teams.  A whole block uses
@@ -125,11 +130,11 @@ struct Team {
 };
 
 // ---- sequences ---------------------------------------------------------------
-// 16-base windows of a sequence: from the shared copy (win[j] = {half j, half
-// j+1}, halves MSB-first) or from the packed little-endian words in global
-// memory (logical half j at 32-bit index j ^ 1, clamped to the array).
+// 16-base windows of a sequence: from the shared copy (16-base words in order, first
+// base on top) or from the packed little-endian words in global memory (logical word j
+// at 32-bit index j ^ 1, clamped to the array).
 struct SeqWin {
-    const uint2 *win;
+    const uint32_t *win;
     const uint32_t *w32;
     int32_t last;
 };
@@ -138,33 +143,31 @@ template <bool SMEM>
 __device__ __forceinline__ uint32_t win16(const SeqWin &s, int32_t pos)
 {
     const int32_t j = pos >> 4;
-    if (SMEM) {
-        const uint2 e = s.win[j];
-        return __funnelshift_l(e.y, e.x, (uint32_t)pos << 1);
-    }
+    if (SMEM)
+        return __funnelshift_l(s.win[j + 1], s.win[j], (uint32_t)pos << 1);
     const uint32_t hi = __ldg(s.w32 + ((uint32_t)j ^ 1u));
     const uint32_t lo = __ldg(s.w32 + ((uint32_t)min(j + 1, s.last) ^ 1u));
     return __funnelshift_l(lo, hi, (uint32_t)pos << 1);
 }
 
-// Copies nw packed words (2*nw halves) into win[0 .. 2*nw) when SMEM.
+// Copies nw packed words into win[0 .. 2*nw) when SMEM, and two guard words after them,
+// whose bases match nothing in the other sequence's guard.  (One word per 16 bases and
+// two loads per window, instead of overlapping 64-bit windows and one: the one-warp
+// tier's copy holds 6,144 bases in 3 KB, where it held 2,048 in 2 KB and longer pairs
+// read their windows from global memory.)
 template <bool SMEM>
-__device__ __forceinline__ SeqWin stage_seq(const SeqView &v, int64_t off, int32_t nw, uint2 *win,
-                                            int tt, int tw)
+__device__ __forceinline__ SeqWin stage_seq(const SeqView &v, int64_t off, int32_t nw,
+                                            uint32_t *win, int tt, int tw, uint32_t guard)
 {
     if (SMEM) {
-        const int32_t nh = 2 * nw;
         const uint64_t *src = v.packed + off;
-        for (int32_t i = tt; i < nh; i += tw) {
-            const uint64_t a = __ldg(src + (i >> 1));
-            const uint32_t hj = (i & 1) ? (uint32_t)a : (uint32_t)(a >> 32);
-            uint32_t hj1 = 0;
-            if (i + 1 < nh) {
-                const uint64_t b = __ldg(src + ((i + 1) >> 1));
-                hj1 = ((i + 1) & 1) ? (uint32_t)b : (uint32_t)(b >> 32);
-            }
-            win[i] = make_uint2(hj, hj1);
+        for (int32_t i = tt; i < nw; i += tw) {
+            const uint64_t a = __ldg(src + i);
+            *reinterpret_cast<uint2 *>(win + 2 * i) =
+                make_uint2((uint32_t)(a >> 32), (uint32_t)a);
         }
+        if (tt == 0)
+            *reinterpret_cast<uint2 *>(win + 2 * nw) = make_uint2(guard, guard);
         return SeqWin{win, nullptr, 0};
     }
     const int64_t last = 2 * (v.n_words - off) - 1;
@@ -176,22 +179,31 @@ __device__ __forceinline__ SeqWin stage_seq(const SeqView &v, int64_t off, int32
 // 16-base windows, leading zeros / 2 = matching bases, clamped by the
 // remaining lengths.  Requires row >= 0 and row - k >= 0.
 template <bool SMEM>
-__device__ __noinline__ int32_t ext_run(const SeqWin &qs, int32_t qlen, const SeqWin &rs,
+__device__ __forceinline__ int32_t ext_more(const SeqWin &qs, int32_t qlen, const SeqWin &rs,
                                            int32_t rlen, int32_t row, int32_t k)
 {
-    int32_t col = row - k;
-    while (row < qlen && col < rlen) {
-        const uint32_t x = win16<SMEM>(qs, row) ^ win16<SMEM>(rs, col);
-        const int ml = __clz((int)x) >> 1;
-        const int lim = min(qlen - row, rlen - col);
-        if (ml >= lim)
-            return row + lim;
-        row += ml;
-        col += ml;
-        if (ml < 16)
+    const int32_t end = min(qlen, rlen + k);
+    while (row < end) {
+        // four windows at once: their loads do not wait for one another
+        uint32_t x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int32_t at = min(row + 16 * i, end - 1);
+            x[i] = win16<SMEM>(qs, at) ^ win16<SMEM>(rs, at - k);
+        }
+        const uint32_t y = x[0] ? x[0] : x[1] ? x[1] : x[2] ? x[2] : x[3];
+        row += (x[0] ? 0 : x[1] ? 16 : x[2] ? 32 : 48) + (__clz((int)y) >> 1);
+        if (y)
             break;
     }
-    return row;
+    return min(row, end);
+}
+
+template <bool SMEM>
+__device__ __noinline__ int32_t ext_run(const SeqWin &qs, int32_t qlen, const SeqWin &rs,
+                                        int32_t rlen, int32_t row, int32_t k)
+{
+    return ext_more<SMEM>(qs, qlen, rs, rlen, row, k);
 }
 
 // First window of U diagonals at once; the ones whose whole window matched
@@ -233,9 +245,134 @@ __device__ __forceinline__ void ext_u(const SeqWin &qs, int32_t qlen, const SeqW
     }
 }
 
+// N = 4 or 2 neighbouring diagonals of one step in int16 rings: window positions p0 ..
+// p0 + N - 1 (p0 a multiple of N), diagonals k0 on; positions outside [pa, pb] are stored
+// as NEG.  Rows point at window position 0.  Two diagonals per register: the rows come in
+// by N-element loads and 4-byte ones for the neighbours left and right (N = 4: 8 loads and
+// 7 permutes for what were 20 two-byte loads), and the recurrences are 16-bit-pair DPX.
+// The extension is per diagonal: positions are kept doubled (bit offsets into the packed
+// bases), clamped unsigned so that a dead row -- negative, and so is its column -- reads
+// the two guard windows, which differ in their first base: it advances by 0 without a
+// test.
+template <int N, bool SMEM>
+__device__ __forceinline__ void wf_group(const int16_t *Mx, const int16_t *Moe, const int16_t *Ie,
+                                         const int16_t *De, int16_t *Mw, int16_t *Iw, int16_t *Dw,
+                                         int32_t p0, int32_t k0, int32_t pa, int32_t pb,
+                                         const SeqWin &qs, int32_t qlen, const SeqWin &rs,
+                                         int32_t rlen, uint32_t qguard2, uint32_t rguard2)
+{
+    constexpr int P = N / 2;  // registers of two diagonals
+    const uint32_t NEG2 = 0x80008000u, ONE2 = 0x00010001u;
+    auto load = [&](const int16_t *row, uint32_t (&v)[P]) {
+        if (N == 4) {
+            const uint2 t = *reinterpret_cast<const uint2 *>(row + p0);
+            v[0] = t.x;
+            v[P - 1] = t.y;
+        } else {
+            v[0] = *reinterpret_cast<const uint32_t *>(row + p0);
+        }
+    };
+    auto store = [&](int16_t *row, const uint32_t (&v)[P]) {
+        if (N == 4)
+            *reinterpret_cast<uint2 *>(row + p0) = make_uint2(v[0], v[P - 1]);
+        else
+            *reinterpret_cast<uint32_t *>(row + p0) = v[0];
+    };
+    auto pair_at = [&](const int16_t *row, int off) {
+        return *reinterpret_cast<const uint32_t *>(row + p0 + off);
+    };
+    uint32_t mx[P], mo[P], ie[P], de[P];
+    load(Mx, mx);
+    load(Moe, mo);
+    load(Ie, ie);
+    load(De, de);
+    const uint32_t mol = pair_at(Moe, -2), mor = pair_at(Moe, N), iel = pair_at(Ie, -2),
+                   der = pair_at(De, N);
+    uint32_t iv[P], dv[P], mv[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        // elements k - 1 of M and I, k + 1 of M and D, for the two diagonals k
+        const uint32_t ml = __byte_perm(j ? mo[j ? j - 1 : 0] : mol, mo[j], 0x5432);
+        const uint32_t il = __byte_perm(j ? ie[j ? j - 1 : 0] : iel, ie[j], 0x5432);
+        const uint32_t mr = __byte_perm(mo[j], j + 1 < P ? mo[j + 1 < P ? j + 1 : j] : mor, 0x5432);
+        const uint32_t dr = __byte_perm(de[j], j + 1 < P ? de[j + 1 < P ? j + 1 : j] : der, 0x5432);
+        const uint32_t i0 = __vmaxs2(ml, il);
+        dv[j] = __vmaxs2(mr, dr);
+        // max(mx + 1, i + 1, d)
+        mv[j] = __viaddmax_s16x2(mx[j], ONE2, __viaddmax_s16x2(i0, ONE2, dv[j]));
+        iv[j] = __viaddmax_s16x2(i0, ONE2, NEG2);
+    }
+    if (qlen > 0 && rlen > 0) {
+        int32_t row[N], end[N];
+        uint32_t x[N];
+        uint32_t least = 0xFFFFFFFFu;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            row[u] = (u & 1) ? (int32_t)mv[u / 2] >> 16 : (int32_t)(int16_t)mv[u / 2];
+            end[u] = __viaddmin_s32(k0 + u, rlen, qlen);  // last row of the diagonal
+            if (SMEM) {
+                const uint32_t q2 = __viaddmin_u32((uint32_t)row[u], (uint32_t)row[u], qguard2);
+                const uint32_t r2 = __viaddmin_u32(2u * (uint32_t)row[u],
+                                                   (uint32_t)(-2 * (k0 + u)), rguard2);
+                const uint32_t *const a = reinterpret_cast<const uint32_t *>(
+                    reinterpret_cast<const char *>(qs.win) + ((q2 >> 3) & ~3u));
+                const uint32_t *const b = reinterpret_cast<const uint32_t *>(
+                    reinterpret_cast<const char *>(rs.win) + ((r2 >> 3) & ~3u));
+                x[u] = __funnelshift_l(a[1], a[0], q2) ^ __funnelshift_l(b[1], b[0], r2);
+            } else {
+                const int32_t pq = (int32_t)min((uint32_t)row[u], (uint32_t)(qlen - 1));
+                const int32_t pr = (int32_t)min((uint32_t)(row[u] - k0 - u), (uint32_t)(rlen - 1));
+                x[u] = row[u] < 0 ? 0xFFFFFFFFu : win16<false>(qs, pq) ^ win16<false>(rs, pr);
+            }
+            least = min(least, x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int32_t adv = __clz((int)x[u]) >> 1;  // 16 for a whole matching window
+            row[u] = max(row[u], __viaddmin_s32(row[u], adv, end[u]));
+        }
+        // whole windows matched: those diagonals go on by themselves, the lanes' together
+        if (least == 0) {
+            uint32_t todo = 0;
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+                todo |= x[u] == 0 && row[u] < end[u] ? 1u << u : 0u;
+            while (todo) {
+                const int v = __ffs((int)todo) - 1;
+                todo &= todo - 1;
+                int32_t at = row[0];
+#pragma unroll
+                for (int u = 1; u < N; ++u)
+                    at = v == u ? row[u] : at;
+                at = ext_more<SMEM>(qs, qlen, rs, rlen, at, k0 + v);
+#pragma unroll
+                for (int u = 0; u < N; ++u)
+                    row[u] = v == u ? at : row[u];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < P; ++j)
+            mv[j] = __byte_perm((uint32_t)row[2 * j], (uint32_t)row[2 * j + 1], 0x5410);
+    }
+    if (p0 < pa || p0 + N - 1 > pb) {  // the interval's ends
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const int32_t e0 = p0 + 2 * j, e1 = e0 + 1;
+            const uint32_t keep = (e0 >= pa && e0 <= pb ? 0xFFFFu : 0u) |
+                                  (e1 >= pa && e1 <= pb ? 0xFFFF0000u : 0u);
+            mv[j] = (mv[j] & keep) | (NEG2 & ~keep);
+            iv[j] = (iv[j] & keep) | (NEG2 & ~keep);
+            dv[j] = (dv[j] & keep) | (NEG2 & ~keep);
+        }
+    }
+    store(Iw, iv);
+    store(Dw, dv);
+    store(Mw, mv);
+}
+
 // ---- dump records ---------------------------------------------------------------
 // A suspended pair: int32 header {next step, M slot, I/D slot, span lo, span
-// hi} at 0, lane j's {M slot j lo, hi, I/D slot j lo, hi} at int 32 + 4j, and
+// hi} at 0, {lo, hi} of the step in M slot j at int 32 + 2j, and
 // from byte kDumpHeader the nslot ring rows over [span lo, span hi], each
 // span elements of int16.
 //
@@ -265,25 +402,300 @@ struct DumpOut {
     int *ctr;           // records claimed
 };
 
-// ---- one pair ------------------------------------------------------------------
-// Aligns pair pi with this team.  ring: the team's window (nslot rows of W
-// elements, diagonal k of slot j at ring[j * W + H + k]).  resume: a dump
-// record to continue from, or nullptr.  Returns the cost (>= 0), -1 past
-// max_error, kPromote (state written to record *dump_idx, or *dump_idx = -1
-// when no record was free), or kRestart (int16 rows would overflow).  The
-// return value is uniform over the team.
-template <int TEAM, int NTEAMS, int U, bool SMEM_SEQ, typename RT>
-__device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r, const WfaParams &p,
-                                             const Shape &w, int64_t pi, RT *ring, int32_t W,
-                                             int32_t H, uint2 *sq, uint2 *sr,
-                                             const Team<TEAM, NTEAMS> &team,
-                                             volatile int64_t *bcast, const uint8_t *resume,
-                                             const DumpOut &dump, int64_t *dump_idx,
-                                             int64_t &cells, int32_t band_w, int32_t ub)
+// ---- one pair, int16 rings ------------------------------------------------------
+// Aligns pair pi with this team.  ring: the team's window (nslot rows of W elements,
+// diagonal k of slot j at ring[j * W + H + k]).  resume: a dump record to continue
+// from, or nullptr.  Returns the cost (>= 0), -1 past max_error, kPromote (state
+// written to record *dump_idx, or *dump_idx = -1 when no record was free), or kRestart
+// (int16 rows would overflow).  The return value is uniform over the team.
+//
+// Intervals.  A step's diagonals [lo, hi] are kept as (lo, -hi) in the halves of one
+// register, kNone when there are none, so that the union of sources is a 16-bit-pair
+// minimum, one diagonal further a -1 in both halves, and clipping a maximum.  Lane j
+// holds those of the step in M slot j: of its M (ivm) and of its I and D (ivi), which
+// start later (no step reached by mismatches alone has any).  Diagonals of a window
+// fit 14 bits; limits beyond it are cut to +-kFar.
+constexpr uint32_t kNone = 0x3FFF3FFFu;
+constexpr int32_t kFar = 16000;
+
+__device__ __forceinline__ uint32_t pack2(int32_t lo, int32_t nhi)
+{
+    return __byte_perm((uint32_t)lo, (uint32_t)nhi, 0x5410);
+}
+__device__ __forceinline__ int32_t cut(int32_t v) { return min(max(v, -kFar), kFar); }
+
+template <int TEAM, int NTEAMS, bool SMEM_SEQ>
+__device__ __forceinline__ int32_t tier_pair16(
+    const SeqView &q, const SeqView &r, const WfaParams &p, const Shape &w, int64_t pi,
+    int16_t *ring, int32_t W, int32_t H, uint32_t *sq, uint32_t *sr, const Team<TEAM, NTEAMS> &team,
+    volatile int64_t *bcast, const uint8_t *resume, const DumpOut &dump, int64_t *dump_idx,
+    int64_t &cells, int32_t band_w, int32_t ub)
 {
     constexpr int TW = TEAM * 32;
-    constexpr int32_t NEG = Neg<RT>::value;
-    constexpr bool R16 = std::is_same<RT, int16_t>::value;
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t ONES = 0xFFFFFFFFu;  // -1 in both halves
+    const int lane = threadIdx.x & 31;
+    const int tt = (int)(threadIdx.x % TW);
+    const int hm = w.hm, hie = w.hie, xs = w.xs, oes = w.oes, es = w.es, g = w.g;
+    const int32_t max_err = p.max_error;
+    const int64_t qoff = q.offsets[pi] - q.word_base;
+    const int64_t roff = r.offsets[pi] - r.word_base;
+    const int32_t qlen = (int32_t)q.lengths[pi], rlen = (int32_t)r.lengths[pi];
+    if (qlen == 0 && rlen == 0)
+        return 0;
+    const int32_t qnw = (qlen + 31) >> 5, rnw = (rlen + 31) >> 5;
+    team.sync();  // the previous pair's reads of the shared copies and the ring are done
+    const SeqWin qs = stage_seq<SMEM_SEQ>(q, qoff, qnw, sq, tt, TW, 0u);
+    const SeqWin rs = stage_seq<SMEM_SEQ>(r, roff, rnw, sr, tt, TW, 0xFFFFFFFFu);
+    {
+        // every ring element NEG (W is a multiple of 8 and the window 16-byte aligned)
+        uint4 *v = reinterpret_cast<uint4 *>(ring);
+        const uint4 n4 = make_uint4(0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u);
+        for (int32_t i = tt; i < w.nslot * W / 8; i += TW)
+            v[i] = n4;
+    }
+    const int32_t target = qlen - rlen;
+    // doubled positions of the guard windows
+    const uint32_t qguard2 = (uint32_t)qnw * 64u, rguard2 = (uint32_t)rnw * 64u;
+    uint32_t ivm = kNone, ivi = kNone;
+    int ms = 0, is = 0;
+    int32_t sp = 1;
+    team.sync();  // NEG fill done before the restored / initial values land
+    if (resume) {
+        const int32_t *hd = reinterpret_cast<const int32_t *>(resume);
+        sp = hd[0];
+        ms = hd[1];
+        is = hd[2];
+        const int32_t ulo = hd[3], uhi = hd[4];
+        ivm = (uint32_t)hd[32 + 2 * lane];
+        ivi = (uint32_t)hd[33 + 2 * lane];
+        const int32_t span = uhi - ulo + 1;
+        if (span > 0) {
+            const int16_t *src = reinterpret_cast<const int16_t *>(resume + kDumpHeader);
+            const int32_t total = w.nslot * span;
+            for (int32_t i = tt; i < total; i += TW) {
+                const int32_t j = i / span, kk = i - j * span;
+                ring[j * W + H + ulo + kk] = src[i];
+            }
+        }
+    } else {
+        // score 0: M[0,0] = 0 extended along diagonal 0 (:130-140)
+        const int32_t row0 = ext_run<SMEM_SEQ>(qs, qlen, rs, rlen, 0, 0);
+        if (lane == 0)
+            ivm = 0;
+        if (tt == 0)
+            ring[H] = (int16_t)row0;
+        cells += 1;
+        if (target == 0 && row0 >= qlen)
+            return 0;
+    }
+    team.sync();
+    // limits that do not change: the matrix, then [target] let in, then max_error and
+    // the bound pass's band (around the line from diagonal 0 to the target)
+    const int32_t tc = cut(target);
+    const uint32_t lim_matrix = pack2(-min(rlen, kFar), -min(qlen, kFar));
+    const uint32_t lim_target = pack2(tc, -tc);
+    int32_t flo = -min(max_err, kFar), fnhi = flo;
+    if (band_w > 0) {
+        flo = max(flo, cut(min(0, target) - band_w));
+        fnhi = max(fnhi, cut(-max(0, target) - band_w));
+    }
+    const uint32_t lim_fixed = pack2(flo, fnhi);
+    // a step reads whole groups of four and the pairs beside them
+    const uint32_t lim_window = pack2(4 - H, -(W - 6 - H));
+    // pruning by the upper bound ub: R = (ub - s) / e at the next step, kept as quotient
+    // and remainder; the diagonals [target - R, target + R]
+    int32_t plo = -(1 << 30), pnhi = -(1 << 30), rr = 0;
+    if (ub >= 0) {
+        const int32_t num = ub - sp * g, rq = num / p.e;
+        rr = num - rq * p.e;
+        plo = target - rq;
+        pnhi = -target - rq;
+    }
+    // row offsets, in elements: the step's own rows and its sources'.  A source before
+    // the first step falls on a slot not written yet, which is NEG with no interval.
+    const int32_t mrows = hm * W, irows = hie * W;
+    int32_t om = ms * W, oi = is * W;
+    // steps s = sp * g <= max_err; int16 rows are proven for sp <= 32767 - qlen, and a dead
+    // row (NEG plus at most one per step) has a negative column on every diagonal of the
+    // window while sp < 32768 - H
+    const int32_t sp_end = max_err / g;
+    const int32_t sp_lim = min(sp_end, 32767 - max(qlen, H + 8));
+    for (; sp <= sp_lim; ++sp) {
+        const int32_t s = sp * g;
+        const int nms = ms + 1 == hm ? 0 : ms + 1;
+        const int sx = nms >= xs ? nms - xs : nms - xs + hm;
+        const int soe = nms >= oes ? nms - oes : nms - oes + hm;
+        const int se = nms >= es ? nms - es : nms - es + hm;
+        const uint32_t vx = __shfl_sync(FULL, ivm, sx);
+        const uint32_t voe = __shfl_sync(FULL, ivm, soe);
+        const uint32_t ve = __shfl_sync(FULL, ivi, se);
+        // I and D: the sources one diagonal further out (kNone stays above every limit)
+        const uint32_t vid = __viaddmax_s16x2(__vmins2(voe, ve), ONES, 0x80008000u);
+        const uint32_t vall = __vmins2(vid, vx);
+        uint32_t lim = __vmaxs2(lim_matrix, pack2(-min(s, kFar), -min(s, kFar)));
+        lim = __vmaxs2(__vmins2(lim, lim_target), lim_fixed);
+        if (ub >= 0) {
+            // a diagonal k at score s costs at least s + e*|k - target| to finish (every
+            // diagonal change is a gap base): beyond the upper bound ub it cannot be on an
+            // alignment of cost <= ub, and dropping it only lowers values elsewhere, so the
+            // first hit stays at the same s
+            lim = __vmaxs2(lim, pack2(cut(plo), cut(pnhi)));
+            rr -= g;
+            if (rr < 0) {
+                rr += p.e;
+                ++plo;
+                ++pnhi;
+            }
+        }
+        const uint32_t ab = __vmaxs2(vall, lim);
+        const int32_t a = (int32_t)(int16_t)ab, b = -((int32_t)ab >> 16);
+        const bool empty = a > b;
+        if (!empty && __vmaxs2(ab, lim_window) != ab) {
+            // outside the window: the pair moves to the next tier, in the state after
+            // step sp - 1
+            int64_t di = -1;
+            if (dump.base) {
+                if (tt == 0) {
+                    const int64_t c = atomicAdd(dump.ctr, 1);
+                    *bcast = c < dump.cap ? c : -1;
+                }
+                team.sync();
+                di = *bcast;
+                team.sync();  // read by every thread before the slot is reused
+            }
+            if (di >= 0) {
+                uint8_t *rec = dump.base + di * dump.stride;
+                int32_t *hd = reinterpret_cast<int32_t *>(rec);
+                // the live span: the union of every step's interval, widened to 16-byte
+                // units of the window rows
+                const int32_t l = (int32_t)(int16_t)ivm, nh = (int32_t)ivm >> 16;
+                const bool some = lane < hm && l + nh <= 0;
+                int32_t l0 = __reduce_min_sync(FULL, some ? l : 0x7fffffff);
+                int32_t h0 = __reduce_max_sync(FULL, some ? -nh : -0x7fffffff);
+                if (l0 <= h0) {
+                    l0 -= (H + l0) & 7;
+                    h0 += 7 - ((H + h0) & 7);
+                }
+                if (tt == 0) {
+                    hd[0] = sp;
+                    hd[1] = ms;
+                    hd[2] = is;
+                    hd[3] = l0;
+                    hd[4] = h0;
+                }
+                if (tt < 32) {
+                    hd[32 + 2 * lane] = (int32_t)ivm;
+                    hd[33 + 2 * lane] = (int32_t)ivi;
+                }
+                const int32_t span = h0 - l0 + 1;
+                if (span > 0) {
+                    int16_t *dst = reinterpret_cast<int16_t *>(rec + kDumpHeader);
+                    // alignment as derived above, checked (the same on every thread of
+                    // the team): the element copy below otherwise
+                    const bool bulk = (((uintptr_t)dst & 15u) == 0) && ((W & 7) == 0) &&
+                                      ((__cvta_generic_to_shared(ring + H + l0) & 15u) == 0);
+                    if (bulk) {
+                        // every thread orders its ring writes before the async proxy's
+                        // reads, then one thread hands the rows to the copy engine and
+                        // waits for them before the team can reuse the window (the next
+                        // pair starts with a barrier)
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        team.sync();
+                        if (tt == 0) {
+                            for (int j = 0; j < w.nslot; ++j)
+                                bulk_row_to_global(dst + (int64_t)j * span, ring + j * W + H + l0,
+                                                   (uint32_t)span * 2u);
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                        }
+                    } else {
+                        const int32_t total = w.nslot * span;
+                        for (int32_t i = tt; i < total; i += TW) {
+                            const int32_t j = i / span, kk = i - j * span;
+                            dst[i] = ring[j * W + H + l0 + kk];
+                        }
+                    }
+                }
+            }
+            *dump_idx = di;
+            return kPromote;
+        }
+        ms = nms;
+        is = is + 1 == hie ? 0 : is + 1;
+        om = om + W == mrows ? 0 : om + W;
+        oi = oi + W == irows ? 0 : oi + W;
+        // What the reused slots held (the steps sp - hm for M, sp - hie for I and D) and
+        // this step does not overwrite becomes NEG.  Not on a side that the pruning bound
+        // cuts (ab above vall): the bound closes in by one diagonal per e of score, so a
+        // later step that reads this slot -- at e or o + e more, one diagonal further out,
+        // or at x more on the same diagonals -- stays inside [a, b] on that side.
+        const uint32_t old = __vmins2(__shfl_sync(FULL, ivm, ms),
+                                      __shfl_sync(FULL, ivi, ms >= hie ? ms - hie : ms - hie + hm));
+        int16_t *const Mw = ring + om, *const Iw = ring + mrows + oi, *const Dw = Iw + irows;
+        if (empty || __vmins2(old, ab) != ab) {
+            const int32_t olo = (int32_t)(int16_t)old, ohi = -((int32_t)old >> 16);
+            const uint32_t cutd = ab ^ vall;
+            // an unclipped side is cleaned up to the interval's end
+            const int32_t le = empty ? ohi : ((cutd & 0xFFFFu) ? olo - 1 : min(ohi, a - 1));
+            const int32_t rs0 = empty ? ohi + 1 : ((cutd >> 16) ? ohi + 1 : max(olo, b + 1));
+            if (olo <= ohi) {
+                for (int32_t k = olo + tt; k <= le; k += TW)
+                    Mw[H + k] = Iw[H + k] = Dw[H + k] = (int16_t)-32768;
+                for (int32_t k = rs0 + tt; k <= ohi; k += TW)
+                    Mw[H + k] = Iw[H + k] = Dw[H + k] = (int16_t)-32768;
+            }  // where the groups below reach over these, they write NEG too
+        }
+        if (!empty) {
+            cells += (int64_t)(b - a + 1);
+            const int16_t *const Mx = ring + sx * W, *const Moe = ring + soe * W;
+            const int16_t *const Ie = ring + mrows + (oi >= es * W ? oi - es * W
+                                                                   : oi - es * W + irows);
+            const int16_t *const De = Ie + irows;
+            const int32_t pa = H + a, pb = H + b;
+            // groups of neighbouring diagonals, one per thread and round: of four while
+            // more are left than a round of two covers, which wastes fewer threads on
+            // the last one
+            int32_t p0 = pa & ~3;
+            for (; pb - p0 >= 2 * TW; p0 += 4 * TW) {
+                const int32_t at = p0 + 4 * tt;
+                if (at <= pb)
+                    wf_group<4, SMEM_SEQ>(Mx, Moe, Ie, De, Mw, Iw, Dw, at, at - H, pa, pb, qs,
+                                          qlen, rs, rlen, qguard2, rguard2);
+            }
+            p0 += 2 * tt;
+            if (p0 <= pb)
+                wf_group<2, SMEM_SEQ>(Mx, Moe, Ie, De, Mw, Iw, Dw, p0, p0 - H, pa, pb, qs, qlen,
+                                      rs, rlen, qguard2, rguard2);
+        }
+        if (lane == ms) {
+            ivm = empty ? kNone : ab;
+            // I and D cover the step's diagonals, but no more than their own sources reach
+            const uint32_t own = __vmaxs2(vid, lim);
+            ivi = empty || (int32_t)(int16_t)own + ((int32_t)own >> 16) > 0 ? kNone : own;
+        }
+        team.sync();
+        // M[s, target] >= qlen ends the alignment (:221-224)
+        if (a <= target && target <= b && (int32_t)Mw[H + target] >= qlen)
+            return s;
+    }
+    return sp <= sp_end ? kRestart  // past the steps int16 values are proven for
+                        : -1;       // the loop ran out: cost above max_error (:226)
+}
+
+// ---- one pair, int32 rings (the G tier) ---------------------------------------------
+// As above over int32 rings in global memory that hold every diagonal: pairs start over
+// here, never move on, and write one diagonal per thread and round.
+template <int TEAM, int NTEAMS, int U, bool SMEM_SEQ>
+__device__ __forceinline__ int32_t tier_pair32(const SeqView &q, const SeqView &r,
+                                               const WfaParams &p, const Shape &w, int64_t pi,
+                                               int32_t *ring, int32_t W, int32_t H, uint32_t *sq,
+                                               uint32_t *sr, const Team<TEAM, NTEAMS> &team,
+                                               int64_t &cells, int32_t ub)
+{
+    constexpr int TW = TEAM * 32;
+    using RT = int32_t;
+    constexpr int32_t NEG = -(1 << 30);
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int tt = (int)(threadIdx.x % TW);
@@ -296,51 +708,20 @@ __device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r,
         return 0;
     const int32_t qnw = (qlen + 31) >> 5, rnw = (rlen + 31) >> 5;
     team.sync();  // the previous pair's reads of the shared copies and the ring are done
-    const SeqWin qs = stage_seq<SMEM_SEQ>(q, qoff, qnw, sq, tt, TW);
-    const SeqWin rs = stage_seq<SMEM_SEQ>(r, roff, rnw, sr, tt, TW);
-    // every ring element NEG
-    {
-        const int32_t total = (w.nslot + 1) * W;  // the slots and the NEG row
-        if (R16) {
-            // W is a multiple of 8 and the window 16-byte aligned
-            uint4 *v = reinterpret_cast<uint4 *>(ring);
-            const uint4 n4 = make_uint4(0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u);
-            for (int32_t i = tt; i < total / 8; i += TW)
-                v[i] = n4;
-        } else {
-            for (int32_t i = tt; i < total; i += TW)
-                ring[i] = (RT)NEG;
-        }
-    }
+    const SeqWin qs = stage_seq<SMEM_SEQ>(q, qoff, qnw, sq, tt, TW, 0u);
+    const SeqWin rs = stage_seq<SMEM_SEQ>(r, roff, rnw, sr, tt, TW, 0xFFFFFFFFu);
+    for (int32_t i = tt; i < (w.nslot + 1) * W; i += TW)  // the slots and the NEG row
+        ring[i] = NEG;
     const int32_t target = qlen - rlen;
     RT *const base = ring + H;
     auto slot = [&](int j) { return base + j * W; };
     // per-slot intervals: lane j holds M slot j's and I/D slot j's
     int32_t mlo = 1, mhi = 0, ilo = 1, ihi = 0;
     int ms = 0, is = 0;
-    int64_t sp0 = 1;
+    const int64_t sp0 = 1;
     int32_t result = kRunning;
     team.sync();  // NEG fill done before the restored / initial values land
-    if (resume) {
-        const int32_t *hd = reinterpret_cast<const int32_t *>(resume);
-        sp0 = hd[0];
-        ms = hd[1];
-        is = hd[2];
-        const int32_t ulo = hd[3], uhi = hd[4];
-        mlo = hd[32 + 4 * lane];
-        mhi = hd[33 + 4 * lane];
-        ilo = hd[34 + 4 * lane];
-        ihi = hd[35 + 4 * lane];
-        const int32_t span = uhi - ulo + 1;
-        if (span > 0) {
-            const RT *src = reinterpret_cast<const RT *>(resume + kDumpHeader);
-            const int32_t total = w.nslot * span;
-            for (int32_t i = tt; i < total; i += TW) {
-                const int32_t j = i / span, kk = i - j * span;
-                slot(j)[ulo + kk] = src[i];
-            }
-        }
-    } else {
+    {
         // score 0: M[0,0] = 0 extended along diagonal 0 (:130-140)
         const int32_t row0 = ext_run<SMEM_SEQ>(qs, qlen, rs, rlen, 0, 0);
         if (lane == 0) {
@@ -361,11 +742,9 @@ __device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r,
         rr = num - rq * p.e;
     }
     if (result == kRunning) {
-        // steps s = sp * g <= max_err; int16 rows are proven for sp <= 32767 - qlen
-        const int32_t sp_end = max_err / g;
-        const int32_t sp_lim = R16 ? min(sp_end, 32767 - qlen) : sp_end;
+        const int32_t sp_end = max_err / g;  // steps s = sp * g <= max_err
         int32_t sp = (int32_t)sp0;
-        for (; sp <= sp_lim; ++sp) {
+        for (; sp <= sp_end; ++sp) {
             const int32_t s = (int32_t)(sp * g);
             const int nms = ms + 1 == hm ? 0 : ms + 1;
             const int nis = is + 1 == hie ? 0 : is + 1;
@@ -376,13 +755,6 @@ __device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r,
             }
             lo = max(lo, -max_err);
             hi = min(hi, max_err);
-            if (band_w > 0) {
-                // the bound pass: only the band around the line from diagonal 0 to
-                // the target, which still holds real alignments (their costs bound
-                // the optimum from above)
-                lo = max(lo, min(0, target) - band_w);
-                hi = min(hi, max(0, target) + band_w);
-            }
             if (ub >= 0) {
                 // a diagonal k at score s costs at least s + e*|k - target| to finish
                 // (every diagonal change is a gap base): beyond the upper bound ub it
@@ -425,86 +797,6 @@ __device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r,
             }
             const int32_t a = max(ulo, lo);
             const int32_t b = min(uhi, hi);
-            // this step reads [a-1, b+1] and writes [a, b]: outside the window
-            // the pair moves to the next tier, in the state after step sp-1
-            if (a <= b && (a - 1 < -H || b + 1 > W - 1 - H)) {
-                int64_t di = -1;
-                if (dump.base) {
-                    if (tt == 0) {
-                        const int64_t c = atomicAdd(dump.ctr, 1);
-                        *bcast = c < dump.cap ? c : -1;
-                    }
-                    team.sync();
-                    di = *bcast;
-                    team.sync();  // read by every thread before the slot is reused
-                }
-                if (di >= 0) {
-                    uint8_t *rec = dump.base + di * dump.stride;
-                    int32_t *hd = reinterpret_cast<int32_t *>(rec);
-                    // the live span: the union of every slot's interval
-                    int32_t l0 = 0x7fffffff, h0 = -0x7fffffff;
-                    if (lane < hm && mlo <= mhi) {
-                        l0 = mlo;
-                        h0 = mhi;
-                    }
-                    if (lane < hie && ilo <= ihi) {
-                        l0 = min(l0, ilo);
-                        h0 = max(h0, ihi);
-                    }
-                    l0 = __reduce_min_sync(FULL, l0);
-                    h0 = __reduce_max_sync(FULL, h0);
-                    if (R16 && l0 <= h0) {  // widen to 16-byte units of the window rows
-                        l0 -= (H + l0) & 7;
-                        h0 += 7 - ((H + h0) & 7);
-                    }
-                    if (tt == 0) {
-                        hd[0] = (int32_t)sp;
-                        hd[1] = ms;
-                        hd[2] = is;
-                        hd[3] = l0;
-                        hd[4] = h0;
-                    }
-                    if (tt < 32) {
-                        hd[32 + 4 * lane] = mlo;
-                        hd[33 + 4 * lane] = mhi;
-                        hd[34 + 4 * lane] = ilo;
-                        hd[35 + 4 * lane] = ihi;
-                    }
-                    const int32_t span = h0 - l0 + 1;
-                    if (span > 0) {
-                        int16_t *dst = reinterpret_cast<int16_t *>(rec + kDumpHeader);
-                        // alignment as derived above, checked (the same on every thread
-                        // of the team): the element copy below otherwise
-                        const bool bulk =
-                            R16 && (((uintptr_t)dst & 15u) == 0) && ((W & 7) == 0) &&
-                            ((__cvta_generic_to_shared(slot(0) + l0) & 15u) == 0);
-                        if (bulk) {
-                            // every thread orders its ring writes before the async
-                            // proxy's reads, then one thread hands the rows to the
-                            // copy engine and waits for them before the team can
-                            // reuse the window (the next pair starts with a barrier)
-                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            team.sync();
-                            if (tt == 0) {
-                                for (int j = 0; j < w.nslot; ++j)
-                                    bulk_row_to_global(dst + (int64_t)j * span, slot(j) + l0,
-                                                       (uint32_t)span * 2u);
-                                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-                            }
-                        } else {
-                            const int32_t total = w.nslot * span;
-                            for (int32_t i = tt; i < total; i += TW) {
-                                const int32_t j = i / span, kk = i - j * span;
-                                dst[i] = (int16_t)slot(j)[l0 + kk];
-                            }
-                        }
-                    }
-                }
-                *dump_idx = di;
-                result = kPromote;
-                break;
-            }
             ms = nms;
             is = nis;
             const int32_t omlo = __shfl_sync(FULL, mlo, ms);
@@ -559,13 +851,8 @@ __device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r,
                         const int32_t i0 = max(io, ie), d0 = max(dop, dex);
                         // max(mx + 1, i0 + 1, d0) as two DPX add-max instructions
                         const int32_t m1 = __viaddmax_s32(mx, 1, __viaddmax_s32(i0, 1, d0));
-                        if (R16) {
-                            iv[u] = i0 + 1;
-                            mv[u] = m1;
-                        } else {
-                            iv[u] = i0 < 0 ? NEG : i0 + 1;
-                            mv[u] = m1 < 0 ? NEG : m1;
-                        }
+                        iv[u] = i0 < 0 ? NEG : i0 + 1;
+                        mv[u] = m1 < 0 ? NEG : m1;
                         dv[u] = d0;
                     }
                     ext_u<UU, SMEM_SEQ>(qs, qlen, rs, rlen, mv, ks, live);
@@ -602,8 +889,7 @@ __device__ __forceinline__ int32_t tier_pair(const SeqView &q, const SeqView &r,
             }
         }
         if (result == kRunning)
-            result = sp <= sp_end ? kRestart  // past the steps int16 values are proven for
-                                  : -1;       // the loop ran out: cost above max_error (:226)
+            result = -1;  // the loop ran out: cost above max_error (:226)
     }
     return result;
 }
@@ -637,7 +923,7 @@ struct TierGeom {
     int32_t W, H;           // window: elements per slot row, offset of diagonal 0
     int64_t team_bytes;     // shared bytes of one team (ring + sequence copies)
     int64_t ring_bytes;     // of them, the ring (shared) -- 0 for the G tier
-    int32_t seq_cap;        // 16-base window entries per sequence copy
+    int32_t seq_cap;        // 16-base words per sequence copy, the guard's two included
     int32_t *gring;         // G tier: per-block int32 regions of nslot * W
 };
 
@@ -659,8 +945,8 @@ wfa_tier_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, TierOut tout, Tier
                                       (int64_t)blockIdx.x * (w.nslot + 1) * (int64_t)geo.W);
     else
         ring = reinterpret_cast<RT *>(mine);
-    uint2 *const sq = reinterpret_cast<uint2 *>(mine + geo.ring_bytes);
-    uint2 *const sr = sq + geo.seq_cap;
+    uint32_t *const sq = reinterpret_cast<uint32_t *>(mine + geo.ring_bytes);
+    uint32_t *const sr = sq + geo.seq_cap;
     int64_t n = in.n;
     const int32_t *list = in.list;
     if (in.seg) {
@@ -671,12 +957,18 @@ wfa_tier_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, TierOut tout, Tier
         n = *in.n_dev;
     int64_t cells = 0;
     volatile int64_t *bc = &bcast[team_id];
-    for (;;) {
-        if (tt == 0)
-            *bc = atomicAdd(in.ctr, 1);
-        team.sync();
-        const int64_t it = *bc;
-        team.sync();  // every thread has read the slot before it is reused
+    // A team's first item is given by its place in the grid, one team of every block
+    // before the second of any: the longest pairs, first in the list, go to as many SMs
+    // as there are.  Later ones are asked for.
+    int64_t it = (int64_t)team_id * gridDim.x + blockIdx.x;
+    for (bool asked = false;; asked = true) {
+        if (asked) {
+            if (tt == 0)
+                *bc = atomicAdd(in.ctr, 1) + (int64_t)gridDim.x * NTEAMS;
+            team.sync();
+            it = *bc;
+            team.sync();  // every thread has read the slot before it is reused
+        }
         if (it >= n)
             break;
         int64_t pi;
@@ -690,8 +982,8 @@ wfa_tier_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, TierOut tout, Tier
             pi = list ? (int64_t)list[it] : it;
         }
         const int64_t ql = q.lengths[pi], rl = r.lengths[pi];
-        const bool smem_seq = 2 * ((ql + 31) >> 5) <= geo.seq_cap &&
-                              2 * ((rl + 31) >> 5) <= geo.seq_cap;
+        const bool smem_seq = 2 * ((ql + 31) >> 5) + 2 <= geo.seq_cap &&  // and the guard
+                              2 * ((rl + 31) >> 5) + 2 <= geo.seq_cap;
         int64_t di = -2;
         int32_t res;
         int32_t ub = -1;
@@ -700,14 +992,17 @@ wfa_tier_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, TierOut tout, Tier
             if (ub < 0)
                 ub = p.max_error;
         }
-        if (smem_seq)
-            res = tier_pair<TEAM, NTEAMS, 4, true, RT>(q, r, p, w, pi, ring, geo.W, geo.H, sq, sr,
+        auto align = [&](auto smem) -> int32_t {
+            constexpr bool SMEM = decltype(smem)::value;
+            if constexpr (GRING)
+                return tier_pair32<TEAM, NTEAMS, 4, SMEM>(q, r, p, w, pi, ring, geo.W, geo.H, sq,
+                                                          sr, team, cells, ub);
+            else
+                return tier_pair16<TEAM, NTEAMS, SMEM>(q, r, p, w, pi, ring, geo.W, geo.H, sq, sr,
                                                        team, bc, resume, tout.dump, &di, cells,
                                                        in.band_w, ub);
-        else
-            res = tier_pair<TEAM, NTEAMS, 4, false, RT>(q, r, p, w, pi, ring, geo.W, geo.H, sq, sr,
-                                                        team, bc, resume, tout.dump, &di, cells,
-                                                        in.band_w, ub);
+        };
+        res = smem_seq ? align(std::true_type{}) : align(std::false_type{});
         if (tt == 0) {
             if (res >= -1) {
                 out[pi] = res;
@@ -742,7 +1037,7 @@ struct TierSpec {
     int32_t seq_bases;  // longest sequence copied to shared memory
 };
 // S, M, L tiers
-static const TierSpec kTiers[kWfaShared] = {{1, 16, 2048}, {2, 8, 4096}, {4, 4, 8192}, {8, 2, 16384}, {16, 1, 32768}};
+static const TierSpec kTiers[kWfaShared] = {{1, 16, 6144}, {2, 8, 12288}, {4, 4, 16384}, {8, 2, 32768}, {16, 1, 32768}};
 
 WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax)
 {
@@ -762,15 +1057,15 @@ WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax)
     for (int t = 0; t < kWfaShared; ++t) {
         const TierSpec &s = kTiers[t];
         const int64_t team_bytes = kTierBlockSmem / s.nteams;
-        const int64_t seq_entries = 2 * ((s.seq_bases + 31) / 32);  // halves per sequence
-        const int64_t seq_bytes = 2 * seq_entries * 8;
-        int64_t W = (team_bytes - seq_bytes) / ((nslot + 1) * 2);
+        const int64_t seq_entries = 2 * ((s.seq_bases + 31) / 32) + 2;  // and the guard
+        const int64_t seq_bytes = 2 * seq_entries * 4;
+        int64_t W = (team_bytes - seq_bytes) / (nslot * 2);
         W = W / 8 * 8;  // 16-byte rows: the NEG fill uses 16-byte stores
         plan.W[t] = (int32_t)W;
         plan.H[t] = (int32_t)(W / 2 - 1);
         plan.seq_cap[t] = (int32_t)seq_entries;
         plan.team_bytes[t] = team_bytes & ~int64_t(15);
-        plan.ring_bytes[t] = (int64_t)(nslot + 1) * W * 2;
+        plan.ring_bytes[t] = (int64_t)nslot * W * 2;
         plan.usable[t] = W >= 64;
         plan.dump_stride[t] = (kDumpHeader + (int64_t)nslot * W * 2 + 255) & ~int64_t(255);
     }
@@ -779,8 +1074,8 @@ WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax)
     constexpr int G = kWfaShared;
     plan.W[G] = (int32_t)(((2 * lmax + 8) + 7) & ~int64_t(7));
     plan.H[G] = (int32_t)(lmax + 3);
-    plan.seq_cap[G] = (int32_t)(2 * ((kTiers[G - 1].seq_bases + 31) / 32));
-    plan.team_bytes[G] = 2 * (int64_t)plan.seq_cap[G] * 8;
+    plan.seq_cap[G] = (int32_t)(2 * ((kTiers[G - 1].seq_bases + 31) / 32) + 2);
+    plan.team_bytes[G] = 2 * (int64_t)plan.seq_cap[G] * 4;
     plan.ring_bytes[G] = 0;
     plan.usable[G] = true;
     plan.gring_block_bytes = (int64_t)(nslot + 1) * plan.W[G] * 4;
