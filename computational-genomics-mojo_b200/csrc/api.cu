@@ -787,9 +787,22 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
                 return u;
         return -1;
     };
-    // dump records of the transitions out of the first two tiers
+    // The last tier that can get pairs: a diagonal is at most as far out as the longer
+    // sequence is long and as there are steps, and a tier whose window holds that, for
+    // steps that int16 rows are proven for, passes nothing on.
+    const int64_t steps = p.max_error / gcd_h(p.x, gcd_h(p.o, p.e));
+    const int64_t reach = std::min(std::max(qmax, rmax), steps);
+    int last = G;
+    for (int t = G - 1; t >= first; --t)
+        if (pl.usable[t] && reach + 4 <= pl.H[t] && reach + 6 + pl.H[t] <= pl.W[t] &&
+            steps <= 32767 - std::max<int64_t>(qmax, pl.H[t] + 8))
+            last = t;
+    // short pairs start on eight lanes each, when there are enough to fill the warps
+    const bool shorts = first == 0 && std::max(qmax, rmax) <= kWfaShortLen &&
+                        wfa_short_usable(pl);
+    // dump records of the transitions out of each tier
     int64_t dcap[G] = {}, doff[G] = {}, dbytes = 0;
-    for (int t = first; t < G; ++t) {
+    for (int t = first; t < std::min(last, G); ++t) {
         if (!pl.usable[t] || next_of(t) < 0)
             continue;
         dcap[t] = std::min<int64_t>(n, kTierDumpCap / pl.dump_stride[t]);
@@ -797,9 +810,10 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         dbytes += dcap[t] * pl.dump_stride[t];
     }
     int rc;
-    if ((rc = ensure(c, x.tierq, (size_t)n * 8 * G, x.st)) ||
+    if ((rc = ensure(c, x.tierq, (size_t)n * 8 * (G + 1), x.st)) ||
         (rc = ensure(c, x.dumps, (size_t)std::max<int64_t>(dbytes, 256), x.st)) ||
-        (rc = ensure(c, x.scratch32, (size_t)(sms * pl.gring_block_bytes), x.st)) ||
+        (last == G &&
+         (rc = ensure(c, x.scratch32, (size_t)(sms * pl.gring_block_bytes), x.st))) ||
         (rc = ensure(c, x.counters, kCounterBytes, x.st)))
         return rc;
     CU(c, cudaMemsetAsync(x.counters.p, 0, kCounterBytes, x.st));
@@ -808,8 +822,9 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     int *const q_n = ctr + (G + 1) * kCounterStride;     // + 32 * (tier - 1): pairs queued for tiers 1..G
     int *const d_ctr = ctr + (2 * G + 1) * kCounterStride;  // + 32 * tier: records claimed
     int *const b_ctr = ctr + (3 * G + 1) * kCounterStride;  // the bound pass
-    static_assert((3 * G + 2) * kCounterStride * 4 <= (int)kCounterBytes, "counter space");
-    int2 *const tq = (int2 *)x.tierq.p;              // + n * (tier - 1)
+    int *const s_ctr = ctr + (3 * G + 2) * kCounterStride;  // the short pairs: in, queued for T1
+    static_assert((3 * G + 4) * kCounterStride * 4 <= (int)kCounterBytes, "counter space");
+    int2 *const tq = (int2 *)x.tierq.p;              // + n * (tier - 1); tier 0's at n * G
     uint8_t *const dumps = (uint8_t *)x.dumps.p;
     const int32_t *list = nullptr;
     const int64_t *seg = nullptr;
@@ -832,13 +847,29 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         list = (const int32_t *)x.queue.p;
         seg = (const int64_t *)x.seg.p;
     }
+    if (shorts) {
+        WfaTierIo io{};
+        io.list = list;
+        io.seg = seg;
+        io.n = n;
+        io.ctr = s_ctr;
+        io.next = tq + n * G;
+        io.next_n = s_ctr + kCounterStride;
+        cudaEvent_t e0 = prof_begin(c, x.st);
+        CU(c, launch_wfa_short(pl, (int)sms, qv, rv, p, io, d_out, (int64_t *)x.work.p, x.st));
+        prof_end(c, e0, x.st);
+        c->launches += 1;
+    }
     int prev = -1;  // the tier launched before t: its suspended pairs are t's entries
-    for (int t = first; t <= G; ++t) {
+    for (int t = first; t <= last; ++t) {
         if (t < G && !pl.usable[t])
             continue;
         WfaTierIo io{};
         io.ctr = in_ctr + kCounterStride * t;
-        if (t == first) {
+        if (t == first && shorts) {
+            io.ents = tq + n * G;
+            io.n_dev = s_ctr + kCounterStride;
+        } else if (t == first) {
             io.list = list;
             io.seg = seg;
             io.n = n;
@@ -850,7 +881,7 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
                 io.dump_in_stride = pl.dump_stride[prev];
             }
         }
-        const int nt = t < G ? next_of(t) : -1;
+        const int nt = t < last ? next_of(t) : -1;
         if (nt >= 0) {
             io.next = tq + n * (nt - 1);
             io.next_n = q_n + kCounterStride * (nt - 1);
@@ -1992,12 +2023,17 @@ static int gb2_wfa_affine_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *
     std::vector<int64_t> key{2};
     key_batches(key, q, r);
     key.insert(key.end(), {cfg->x, cfg->o, cfg->e, cfg->max_error, n, flags});
+    // The tiers sort a batched call's pairs by length; alike ones need no sorting (500,000
+    // reads: 37 us).
+    const bool tiers = !(flags & GB2_FLAG_NAIVE) && ((flags >> 8) & 0xff) == 0;
+    const bool alike = narrow_range(q->min_len, q->max_len) && narrow_range(r->min_len, r->max_len);
+    const int run_flags = tiers && alike ? flags & ~GB2_FLAG_BATCHED : flags;
     rc = run_graphed(c, c->g_wfa, key, flags, nullptr, [&](bool) -> int {
         int r2;
         if ((r2 = wfa_begin(c, c->x)))
             return r2;
         return wfa_core(c, c->x, view_of(q), view_of(r), q->max_len, r->max_len, cfg, n,
-                        (int32_t *)c->out_wfa.p, flags);
+                        (int32_t *)c->out_wfa.p, run_flags);
     });
     if (rc) {
         cudaStreamSynchronize(c->x.st);

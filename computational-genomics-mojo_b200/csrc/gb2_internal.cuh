@@ -201,6 +201,12 @@ struct WfaTierIo {
     const int32_t *ubound;
     int32_t band_w;
 };
+// Short pairs, eight lanes each (before tier 0): whether the penalties' rows leave a
+// window, and the launch (list or seg, n, ctr in; next out).
+constexpr int32_t kWfaShortLen = 512;
+bool wfa_short_usable(const WfaTierPlan &pl);
+cudaError_t launch_wfa_short(const WfaTierPlan &pl, int sm_count, SeqView q, SeqView r, WfaParams p,
+                             const WfaTierIo &io, int32_t *out, int64_t *work, cudaStream_t st);
 cudaError_t launch_wfa_tier(const WfaTierPlan &pl, int tier, int grid, SeqView q, SeqView r,
                             WfaParams p, const WfaTierIo &io, int32_t *out, int64_t *work,
                             int *err_flag, cudaStream_t st);

@@ -52,6 +52,7 @@
 // 139 per round of four diagonals a lane (82 of two) of which the extension's two window
 // loads, shifts, compare and clamps are 80, and about 100 for the lanes whose whole first
 // window matched.  At the sizes above T1 issues 69% of its slots, T4 62%.
+#include <algorithm>
 #include <type_traits>
 
 #include "gb2_internal.cuh"
@@ -150,6 +151,9 @@ __device__ __forceinline__ uint32_t win16(const SeqWin &s, int32_t pos)
     return __funnelshift_l(lo, hi, (uint32_t)pos << 1);
 }
 
+// Bytes that must be readable past the last copy of a block (ext_more).
+constexpr int32_t kSeqSlack = 16;
+
 // Copies nw packed words into win[0 .. 2*nw) when SMEM, and two guard words after them,
 // whose bases match nothing in the other sequence's guard.  (One word per 16 bases and
 // two loads per window, instead of overlapping 64-bit windows and one: the one-warp
@@ -186,10 +190,25 @@ __device__ __forceinline__ int32_t ext_more(const SeqWin &qs, int32_t qlen, cons
     while (row < end) {
         // four windows at once: their loads do not wait for one another
         uint32_t x[4];
+        if (SMEM) {
+            // five neighbouring words of each copy; those past its end (the four words
+            // kSeqSlack leaves readable) only match past `end`
+            const uint32_t *const a = qs.win + (row >> 4), *const b = rs.win + ((row - k) >> 4);
+            const uint32_t sa = (uint32_t)row << 1, sb = (uint32_t)(row - k) << 1;
+            uint32_t wa = a[0], wb = b[0];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int32_t at = min(row + 16 * i, end - 1);
-            x[i] = win16<SMEM>(qs, at) ^ win16<SMEM>(rs, at - k);
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t na = a[i + 1], nb = b[i + 1];
+                x[i] = __funnelshift_l(na, wa, sa) ^ __funnelshift_l(nb, wb, sb);
+                wa = na;
+                wb = nb;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int32_t at = min(row + 16 * i, end - 1);
+                x[i] = win16<false>(qs, at) ^ win16<false>(rs, at - k);
+            }
         }
         const uint32_t y = x[0] ? x[0] : x[1] ? x[1] : x[2] ? x[2] : x[3];
         row += (x[0] ? 0 : x[1] ? 16 : x[2] ? 32 : 48) + (__clz((int)y) >> 1);
@@ -1025,6 +1044,191 @@ wfa_tier_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, TierOut tout, Tier
         atomicAdd((unsigned long long *)work, (unsigned long long)cells);
 }
 
+// ---- short pairs -------------------------------------------------------------------
+// Batches whose longest sequence has at most kWfaShortLen bases start here: eight lanes
+// per pair, four pairs per warp.  A read's wavefront is a dozen diagonals wide for a dozen
+// steps, so a whole warp on it idles and repeats the per-step bookkeeping for one pair;
+// here four pairs share it.  The slots rotate for the whole warp: a pair enters with its
+// score 0 in the slot that is current, whatever step the others are at.  Nothing is pruned
+// and the limits of the matrix only cut, so the diagonals of a pair's step sp are
+// [max(-reach, -rlen), min(reach, qlen)] with a reach that depends on the penalties and sp
+// alone: a table.  New pairs are taken when two of the four are done, so that their setup
+// is shared.  A pair whose interval outgrows the window, or its steps the table, is queued
+// for T1, which starts it over.  Blocks of four warps, five per SM.
+// Bound: ALU issue (81% busy).  500,000 reads of 150 bp at up to 6% divergence: the call
+// 2.91 -> 1.46 ms, the kernel 1.20 (T1 took 2.62); 1,800 warp instructions a pair against
+// 3,600.  With the four pairs in step from their first to the last of them to end, 1.35.
+struct ShortGeom {
+    int32_t W, H, seq_cap;
+    int32_t pair_bytes;
+};
+constexpr int kShortSteps = 512;
+
+// reach[sp] = {of M; what the reused slots held}: the furthest diagonals of the pairs'
+// step sp (-1: none) and of the steps whose slots it takes over.  By one thread.
+__device__ void short_reach(const Shape &w, uchar2 *reach)
+{
+    int8_t rm[32], ri[32];  // per M slot: M, and I and D
+    for (int j = 0; j < w.hm; ++j)
+        rm[j] = ri[j] = -1;
+    rm[0] = 0;
+    int ms = 0;
+    for (int sp = 1; sp < kShortSteps; ++sp) {
+        ms = ms + 1 == w.hm ? 0 : ms + 1;
+        auto back = [&](int d) { return ms >= d ? ms - d : ms - d + w.hm; };
+        int vid = max(rm[back(w.oes)], ri[back(w.es)]);
+        vid += vid >= 0;
+        const int va = max(vid, (int)rm[back(w.xs)]);
+        const int old = max((int)rm[ms], (int)ri[back(w.hie)]);
+        reach[sp] = make_uchar2((unsigned char)(va + 1), (unsigned char)(old + 1));
+        rm[ms] = (int8_t)min(va, 126);  // past every window
+        ri[ms] = (int8_t)min(vid, 126);
+    }
+}
+
+__global__ void __launch_bounds__(128, 5)
+wfa_short_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, int2 *next, int *next_n,
+                 ShortGeom geo, int32_t *__restrict__ out, int64_t *work)
+{
+    extern __shared__ __align__(16) uint8_t tsm[];
+    __shared__ uchar2 reach[kShortSteps];
+    const unsigned FULL = 0xffffffffu;
+    const Shape w = make_shape(p);
+    const int lane = threadIdx.x & 31, sub = lane >> 3, l8 = lane & 7, warp = threadIdx.x >> 5;
+    const int32_t W = geo.W, H = geo.H;
+    const int hm = w.hm, hie = w.hie, xs = w.xs, oes = w.oes, es = w.es;
+    uint8_t *const mine = tsm + (warp * 4 + sub) * geo.pair_bytes;
+    int16_t *const ring = reinterpret_cast<int16_t *>(mine);
+    uint32_t *const sq = reinterpret_cast<uint32_t *>(mine + w.nslot * W * 2);
+    uint32_t *const sr = sq + geo.seq_cap;
+    if (threadIdx.x == 0)
+        short_reach(w, reach);
+    __syncthreads();
+    int64_t n = in.n;
+    const int32_t *list = in.list;
+    if (in.seg) {
+        list = in.list + in.seg[0];
+        n = in.seg[1] - in.seg[0];
+    }
+    const int32_t sp_end = p.max_error / w.g;
+    const int32_t mrows = hm * W, irows = hie * W;
+    int64_t cells = 0;
+    // the warp's slots
+    int ms = 0, is = 0;
+    int32_t om = 0, oi = 0;
+    // this lane's pair
+    bool active = false;
+    int32_t pi = 0, qlen = 0, rlen = 0, target = 0, sp = 0;
+    uint32_t qguard2 = 0, rguard2 = 0;
+    const SeqWin qs{sq, nullptr, 0}, rs{sr, nullptr, 0};
+    // pairs come four (then as many as are done) at a time: the first by the warp's place
+    int64_t given = ((int64_t)warp * gridDim.x + blockIdx.x) * 4;
+    bool more = true, asked = false;
+    for (;;) {
+        const unsigned act = __ballot_sync(FULL, active) & 0x01010101u;
+        const int idle = 4 - __popc(act);
+        if (more && idle >= 2) {
+            if (asked) {
+                int64_t b0 = 0;
+                if (lane == 0)
+                    b0 = atomicAdd(in.ctr, idle) + (int64_t)gridDim.x * 16;
+                given = __shfl_sync(FULL, b0, 0);
+            }
+            asked = true;
+            const int64_t it =
+                given + __popc(~act & 0x01010101u & ((1u << (8 * sub)) - 1u));
+            more = given + idle < n;
+            const bool fresh = !active && it < n;
+            if (fresh) {
+                pi = list ? list[it] : (int32_t)it;
+                qlen = (int32_t)q.lengths[pi];
+                rlen = (int32_t)r.lengths[pi];
+                const int32_t qnw = (qlen + 31) >> 5, rnw = (rlen + 31) >> 5;
+                stage_seq<true>(q, q.offsets[pi] - q.word_base, qnw, sq, l8, 8, 0u);
+                stage_seq<true>(r, r.offsets[pi] - r.word_base, rnw, sr, l8, 8, 0xFFFFFFFFu);
+                uint4 *v = reinterpret_cast<uint4 *>(ring);
+                const uint4 n4 = make_uint4(0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u);
+                for (int32_t i = l8; i < w.nslot * W / 8; i += 8)
+                    v[i] = n4;
+                target = qlen - rlen;
+                qguard2 = (uint32_t)qnw * 64u;
+                rguard2 = (uint32_t)rnw * 64u;
+            }
+            __syncwarp();
+            if (fresh) {
+                // score 0: M[0,0] = 0 extended along diagonal 0 (:130-140)
+                const int32_t row0 = ext_more<true>(qs, qlen, rs, rlen, 0, 0);
+                sp = 0;
+                active = !(target == 0 && row0 >= qlen) && sp_end > 0;
+                if (l8 == 0) {
+                    ring[om + H] = (int16_t)row0;
+                    cells += 1;
+                    if (!active)
+                        out[pi] = target == 0 && row0 >= qlen ? 0 : -1;
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        if (!act)
+            break;
+        // one step of every pair
+        ++sp;
+        ms = ms + 1 == hm ? 0 : ms + 1;
+        is = is + 1 == hie ? 0 : is + 1;
+        om = om + W == mrows ? 0 : om + W;
+        oi = oi + W == irows ? 0 : oi + W;
+        const int32_t ox = om >= xs * W ? om - xs * W : om - xs * W + mrows;
+        const int32_t ooe = om >= oes * W ? om - oes * W : om - oes * W + mrows;
+        const int32_t oe = oi >= es * W ? oi - es * W : oi - es * W + irows;
+        int16_t *const Mw = ring + om, *const Iw = ring + mrows + oi, *const Dw = Iw + irows;
+        int32_t va = -1;
+        if (active) {
+            const uchar2 re = reach[min(sp, kShortSteps - 1)];
+            va = (int32_t)re.x - 1;
+            // what the reused slots held further out, inside the window, becomes NEG
+            for (int k = va + 1 + l8; k <= min((int)re.y - 1, H); k += 8) {
+                Mw[H + k] = Iw[H + k] = Dw[H + k] = (int16_t)-32768;
+                Mw[H - k] = Iw[H - k] = Dw[H - k] = (int16_t)-32768;
+            }
+        }
+        const int32_t a = max(-va, -rlen), b = min(va, qlen);
+        if (active && (a - 4 < -H || b + 5 > W - 1 - H || sp >= kShortSteps - 1)) {
+            active = false;
+            if (l8 == 0)
+                next[atomicAdd(next_n, 1)] = make_int2(pi, -1);
+        }
+        const int32_t pa = H + a, pb = active && va >= 0 ? H + b : -1;
+        if (l8 == 0)
+            cells += max(pb - pa + 1, 0);
+        const int16_t *const Mx = ring + ox, *const Moe = ring + ooe, *const Ie = ring + mrows + oe;
+        const int16_t *const De = Ie + irows;
+        // one round of two diagonals a lane covers 16 positions from an even one; wider
+        // intervals take rounds of four
+        if (__any_sync(FULL, pb - (pa & ~1) >= 16)) {
+            for (int32_t at = (pa & ~3) + 4 * l8; __any_sync(FULL, at <= pb); at += 32)
+                if (at <= pb)
+                    wf_group<4, true>(Mx, Moe, Ie, De, Mw, Iw, Dw, at, at - H, pa, pb, qs, qlen,
+                                      rs, rlen, qguard2, rguard2);
+        } else {
+            const int32_t at = (pa & ~1) + 2 * l8;
+            if (at <= pb)
+                wf_group<2, true>(Mx, Moe, Ie, De, Mw, Iw, Dw, at, at - H, pa, pb, qs, qlen, rs,
+                                  rlen, qguard2, rguard2);
+        }
+        __syncwarp();
+        // M[s, target] >= qlen ends the alignment (:221-224)
+        const bool hit = pb >= 0 && a <= target && target <= b && (int32_t)Mw[H + target] >= qlen;
+        if (active && (hit || sp >= sp_end)) {
+            active = false;
+            if (l8 == 0)
+                out[pi] = hit ? sp * w.g : -1;
+        }
+    }
+    if (l8 == 0 && work && cells)
+        atomicAdd((unsigned long long *)work, (unsigned long long)cells);
+}
+
 }  // namespace
 
 // ---- host side --------------------------------------------------------------------
@@ -1082,16 +1286,56 @@ WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax)
     return plan;
 }
 
+// Shared memory of a pair of the short kernel: five blocks of sixteen pairs per SM, and
+// the pairs' rows half a set of banks apart, so that four pairs' 8-byte loads of the same
+// row fall on both halves.
+constexpr int32_t kShortPairBytes = 2752;
+static_assert(kShortPairBytes % 128 == 64 &&
+                  5 * (16 * kShortPairBytes + kSeqSlack + 2 * kShortSteps + 1024) <= 228 * 1024,
+              "five blocks per SM");
+
+static ShortGeom short_geom(int nslot)
+{
+    ShortGeom g;
+    g.seq_cap = 2 * ((kWfaShortLen + 31) / 32) + 2;
+    g.W = (kShortPairBytes - 8 * g.seq_cap) / (nslot * 2) / 8 * 8;
+    g.W = std::min(g.W, 248);  // the reach table's bytes
+    g.H = g.W / 2 - 1;
+    g.pair_bytes = kShortPairBytes;
+    return g;
+}
+
+bool wfa_short_usable(const WfaTierPlan &pl) { return short_geom(pl.nslot).W >= 64; }
+
+cudaError_t launch_wfa_short(const WfaTierPlan &pl, int sm_count, SeqView q, SeqView r, WfaParams p,
+                             const WfaTierIo &io, int32_t *out, int64_t *work, cudaStream_t st)
+{
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        wfa_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        16 * kShortPairBytes + kSeqSlack);
+    if (attr != cudaSuccess)
+        return attr;
+    TierIn in{};
+    in.list = io.list;
+    in.n = io.n;
+    in.seg = io.seg;
+    in.ctr = io.ctr;
+    const int grid = (int)std::min<int64_t>(5 * (int64_t)sm_count, (io.n + 15) / 16);
+    wfa_short_kernel<<<grid, 128, 16 * kShortPairBytes + kSeqSlack, st>>>(q, r, p, in, io.next, io.next_n,
+                                                               short_geom(pl.nslot), out, work);
+    return cudaGetLastError();
+}
+
 template <int TEAM, int NTEAMS, typename RT, bool GRING>
 static cudaError_t tier_launch(const WfaTierPlan &pl, int t, int grid, SeqView q, SeqView r,
                                WfaParams p, const TierIn &in, const TierOut &o, int32_t *gring,
                                int32_t *out, int64_t *work, int *err_flag, cudaStream_t st)
 {
-    const size_t smem = (size_t)pl.team_bytes[t] * NTEAMS;
+    const size_t smem = (size_t)pl.team_bytes[t] * NTEAMS + kSeqSlack;
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(wfa_tier_kernel<TEAM, NTEAMS, RT, GRING>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTierBlockSmem);
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTierBlockSmem + kSeqSlack);
         attr = true;
     }
     TierGeom geo{pl.W[t], pl.H[t], pl.team_bytes[t], pl.ring_bytes[t], pl.seq_cap[t], gring};

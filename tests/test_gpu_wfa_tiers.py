@@ -125,3 +125,29 @@ def test_empty_and_tiny_pairs(device, oracle):
     q, r = _pack(qs), _pack(rs)
     for me in (0, 3, 8, 400, 1200):
         _check(device, oracle, q, r, WFAConfig(4, 6, 2, me), (1, 30, 400))
+
+
+@pytest.mark.parametrize("pen", [(4, 6, 2), (3, 5, 2), (7, 1, 3), (5, 0, 5), (1, 0, 1), (9, 4, 6),
+                                 (10, 20, 9), (2, 28, 3)])
+def test_short_pairs(device, oracle, pen):
+    """Batches of at most 512 bases: eight lanes per pair.  Reads, unrelated pairs whose
+    intervals outgrow the window (the one-warp tier starts them over), one-sided length
+    differences, and the longest that qualify beside one base more (which do not)."""
+    rng = np.random.default_rng(pen[0] * 100 + pen[2])
+    qs, rs = [], []
+    for k in range(150):
+        t = _rnd(rng, int(rng.integers(0, 160)) if k % 5 else int(rng.integers(300, 513)))
+        q = _mutate(rng, t, float(rng.choice([0.0, 0.02, 0.06, 0.3])))[:512]
+        if k % 7 == 3:
+            q = _rnd(rng, len(t))
+        elif k % 7 == 5:
+            q = q[len(q) // 2:]
+        elif k % 7 == 6:
+            t = t[:len(t) // 3]
+        qs.append(q)
+        rs.append(t)
+    q, r = _pack(qs), _pack(rs)
+    for me in (2 * max(pen[0] * 512, pen[1] + 512 * pen[2]), 200, 17, 0):
+        _check(device, oracle, q, r, WFAConfig(*pen, me), (100,))
+    q, r = _pack(qs + [_rnd(rng, 513)]), _pack(rs + [_rnd(rng, 500)])
+    _check(device, oracle, q, r, WFAConfig(*pen, 300), (100,))
