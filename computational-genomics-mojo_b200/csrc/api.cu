@@ -932,16 +932,16 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
 }
 
 int wfa_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,
-             const gb2_wfa_cfg *cfg, int64_t n, int32_t *d_out, int flags, int64_t *d_hist)
+             const gb2_wfa_cfg *cfg, int64_t n, int32_t *d_out, int flags)
 {
     if (n <= 0)
         return GB2_OK;
     if (qmax >= (1ll << 30) || rmax >= (1ll << 30))
         return set_err(c, GB2_ERANGE, "sequence longer than 2^30");
     const WfaParams p{cfg->x, cfg->o, cfg->e, cfg->max_error};
-    // the tiered kernels, unless the call asks for the naive baseline, a tuning
-    // variant of the single-kernel design below, or the CIGAR pass's history sizes
-    if (!(flags & GB2_FLAG_NAIVE) && ((flags >> 8) & 0xff) == 0 && !d_hist) {
+    // the tiered kernels, unless the call asks for the naive baseline or a tuning
+    // variant of the single-kernel design below
+    if (!(flags & GB2_FLAG_NAIVE) && ((flags >> 8) & 0xff) == 0) {
         // Batches with long pairs: for every pair the one-warp tier suspends (the
         // expensive ones), a bound pass finds the cost of its best alignment
         // inside a band of +-kWfaBoundBand diagonals around the line from
@@ -1025,8 +1025,7 @@ int wfa_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t 
     }
     cudaEvent_t e0 = prof_begin(c, x.st);
     CU(c, launch_wfa(variant, bw, qv, rv, p, longs, shorts, d_out, (int32_t *)x.scratch32.p,
-                     slot_width, (int)grid, (int *)x.errflag.p, (int64_t *)x.work.p, d_hist,
-                     x.st));
+                     slot_width, (int)grid, (int *)x.errflag.p, (int64_t *)x.work.p, x.st));
     prof_end(c, e0, x.st);
     c->launches += 1;
     return GB2_OK;

@@ -148,12 +148,9 @@ struct WfaParams {
 constexpr int kWfaWideWarps = 16;
 // Resident blocks per SM of the WFA kernel variant.
 int wfa_blocks_per_sm(int variant, int block_warps);
-// hist (optional): per pair, the bytes of the cell part of its WFA history
-// record (wfa_hist_cell_bytes summed over the visited scores), 0 when the
-// cost is -1.
 cudaError_t launch_wfa(int variant, int block_warps, SeqView q, SeqView r, WfaParams p,
                        PairList longs, PairList shorts, int32_t *out, int32_t *scratch,
-                       int64_t slot_width, int grid, int *err_flag, int64_t *work, int64_t *hist,
+                       int64_t slot_width, int grid, int *err_flag, int64_t *work,
                        cudaStream_t st);
 
 // Tiered WFA (wfa_tiers.cu): tiers 0..4 align a pair with 1, 2, 4, 8 and 16
@@ -224,8 +221,8 @@ __host__ __device__ inline int64_t wfa_hist_record_bytes(int64_t cell_bytes, int
     return (12 * steps + cell_bytes + 15) & ~int64_t(15);
 }
 
-// CIGAR pass over pairs pairs[0..n) (cost and history cell bytes from the
-// cost pass, history record at arena + arena_off[pair]; the first n_team
+// CIGAR pass over pairs pairs[0..n) (cost from the cost pass, and a bound on the
+// history cell bytes; history record at arena + arena_off[pair]; the first n_team
 // pairs one per 128-thread block, the rest one per warp; counters[0] and
 // counters[32] zeroed); run-length CIGAR ops of pair i go to
 // runs[run_off[i] ..], their count to run_count[i].  A run is len << 2 | op

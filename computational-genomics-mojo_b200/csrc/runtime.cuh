@@ -276,10 +276,8 @@ int wfa_validate(gb2_ctx *c, const gb2_wfa_cfg *cfg, int64_t n);
 // Clears the WFA error flag and work counter of x (once per call, before the
 // first wfa_core of that call).
 int wfa_begin(gb2_ctx *c, Exec &x);
-// d_hist (optional): per pair, the history cell bytes the CIGAR pass needs.
 int wfa_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,
-             const gb2_wfa_cfg *cfg, int64_t n, int32_t *d_out, int flags,
-             int64_t *d_hist = nullptr);
+             const gb2_wfa_cfg *cfg, int64_t n, int32_t *d_out, int flags);
 // Reads back x's WFA error flag and work counter (synchronises x's stream),
 // folds the work into the context's statistics and turns the flag into a status.
 int wfa_end(gb2_ctx *c, Exec &x);

@@ -3,12 +3,11 @@
 // wfa_affine_cigar_cpu (genomics/cpu/align_cpu.mojo:380-623) keeps M before
 // and after extension, I and D for every score up to the optimum and every
 // diagonal in [-max_err, max_err], then walks back from (opt, qlen - rlen).
-// Here a first pass is the cost kernel, which also reports how many bytes
-// each pair's history record will take; a second pass (wfa_cigar_kernel in
-// wfa_kernels.cu) re-runs each pair's forward recurrences with the cost
-// kernel's own code in history mode, appending per visited score the
-// M-after-extension values and one decision byte per diagonal to the pair's
-// record in an arena sized from the first pass, and walks the record back
+// Here a first pass finds the costs (the tiered kernels); a second one
+// (wfa_cigar_kernel in wfa_kernels.cu) re-runs each pair's forward recurrences in
+// history mode, over the diagonals that can finish within the known cost, appending
+// per visited score the M-after-extension values and one decision byte per diagonal
+// to the pair's record in an arena sized from the costs, and walks the record back
 // into CIGAR runs (wfa_trace.cuh).  The host groups pairs, largest records
 // first, so the records of a group fit the arena, then gathers every pair's
 // runs into the caller's array.
@@ -63,17 +62,34 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
     const int arena_mib = (int)(((unsigned)flags >> 24) & 0xff);
     flags &= 0x00ffffff;
     if ((rc = wfa_core(c, x, qv, rv, qmax, rmax, cfg, n, (int32_t *)cb.cost.p,
-                       flags | GB2_FLAG_BATCHED, (int64_t *)cb.hist.p)))
+                       flags | GB2_FLAG_BATCHED)))
         return rc;
     if ((rc = wfa_end(c, x)))
         return rc;
-    std::vector<int64_t> hist((size_t)n);
     GB2_CU(c, cudaMemcpyAsync(cost, cb.cost.p, (size_t)n * 4, cudaMemcpyDeviceToHost, x.st));
-    GB2_CU(c, cudaMemcpyAsync(hist.data(), cb.hist.p, (size_t)n * 8, cudaMemcpyDeviceToHost,
-                              x.st));
     GB2_CU(c, cudaStreamSynchronize(x.st));
 
     const int g = std::gcd(cfg->x, std::gcd(cfg->o, cfg->e));
+    // History cell bytes of a pair of cost c, at most: step sp of S = c / g visits diagonals
+    // within sp / es + 1 of diagonal 0 (a source is one diagonal further per es steps at
+    // most) and within (S - sp) / es of the target, so each half of the steps 2j / es + 3
+    // for j = 0 .. S / 2 + 1, and never more than the matrix has.  A step of w cells takes
+    // at most 5w + 3 bytes.
+    const int es = cfg->e / g;
+    std::vector<int64_t> hist((size_t)n);
+    for (int64_t i = 0; i < n; ++i) {
+        if (cost[i] < 0) {
+            hist[(size_t)i] = 0;
+            continue;
+        }
+        const int64_t S = cost[i] / g, half = S / 2 + 1;
+        const int64_t visited =
+            std::min(2 * (half * (half + 1) / es + 3 * (half + 1)),
+                     (S + 1) * (h_qlen[i] + h_rlen[i] + 1));
+        hist[(size_t)i] = (5 * visited + 3 * (S + 2) + 3) & ~int64_t(3);
+    }
+    GB2_CU(c, cudaMemcpyAsync(cb.hist.p, hist.data(), (size_t)n * 8, cudaMemcpyHostToDevice,
+                              x.st));
     // per pair: record bytes, run capacity and its offset
     std::vector<int64_t> rec((size_t)n), run_off((size_t)n);
     int64_t run_total = 0, rec_max = 0;

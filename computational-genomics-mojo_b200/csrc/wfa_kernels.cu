@@ -228,7 +228,7 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
                                                   int64_t pi, int32_t *region, int64_t slot_width,
                                                   uint32_t *sq, uint32_t *sr,
                                                   int32_t *__restrict__ out, int *err_flag,
-                                                  int64_t *work, int64_t *hist, uint8_t *hrec,
+                                                  int64_t *work, uint8_t *hrec,
                                                   int64_t hlimit, int hsteps)
 {
     constexpr int TW = TEAM * 32;
@@ -238,12 +238,19 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
     const int tt = TEAM == 1 ? lane : (int)threadIdx.x;
     const int hm = w.hm, hie = w.hie, xs = w.xs, oes = w.oes, es = w.es, g = w.g;
     const int32_t max_err = p.max_error;
+    // HREC: the cost is known, and a diagonal k at score s that cannot finish within it
+    // (s + e*|k - target| > cost) is not visited.  The walk back visits only cells of
+    // optimal alignments, whose prefixes all stay inside, so their values, and the values
+    // of every source that ties with the one taken, are those of the whole wavefront.
+    const int32_t known = HREC ? (hsteps - 1) * w.g : 0;
+    // through a shuffle: the assembler of CUDA 12.9 otherwise merges
+    // max(max(lo, -max_err), target - R) below into a 3-way maximum of +max_err
+    const int32_t neg_err = __shfl_sync(FULL, -max_err, 0);
     const int64_t qoff = q.offsets[pi] - q.word_base;
     const int64_t roff = r.offsets[pi] - r.word_base;
     const int32_t qlen = (int32_t)q.lengths[pi], rlen = (int32_t)r.lengths[pi];
     int32_t result = -1;
     int64_t cells = 0;
-    int64_t hbytes = 8;  // history bytes of the visited cells (score 0: one cell)
     int32_t *const hdr = reinterpret_cast<int32_t *>(hrec);
     int64_t hcur = 3 * (int64_t)hsteps;  // next free 4-byte word of the record
     bool overrun = false, need32 = false;
@@ -305,6 +312,9 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
             result = 0;
         } else {
             int ms = 0, is = 0;  // ring slots of the current score
+            // (known - s) / e at the next score, as quotient and remainder
+            int32_t prune_q = HREC ? (known - g) / p.e : 0;
+            int32_t prune_r = HREC ? known - g - prune_q * p.e : 0;
             for (int64_t sp = 1; HREC ? sp < hsteps : sp * g <= max_err; ++sp) {
                 if (std::is_same<RT, int16_t>::value && sp > 32767 - (int64_t)qlen) {
                     need32 = true;  // past the steps int16 values are proven for
@@ -318,8 +328,18 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
                     lo = min(lo, target);
                     hi = max(hi, target);
                 }
-                lo = max(lo, -max_err);
+                lo = max(lo, neg_err);
                 hi = min(hi, max_err);
+                if (HREC) {
+                    const int32_t R = prune_q;
+                    prune_r -= g;
+                    if (prune_r < 0) {
+                        prune_r += p.e;
+                        --prune_q;
+                    }
+                    lo = max(lo, target - R);
+                    hi = min(hi, target + R);
+                }
                 const int sx = sp >= xs ? (ms >= xs ? ms - xs : ms - xs + hm) : -1;
                 const int soe = sp >= oes ? (ms >= oes ? ms - oes : ms - oes + hm) : -1;
                 const int se = sp >= es ? (is >= es ? is - es : is - es + hie) : -1;
@@ -387,7 +407,6 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
                 bool hit = false;
                 if (a <= b) {
                     cells += (int64_t)(b - a + 1);
-                    hbytes += wfa_hist_cell_bytes(b - a + 1);
                     const RT *Mx = sx >= 0 ? M(sx) : nullptr;
                     const RT *Moe = soe >= 0 ? M(soe) : nullptr;
                     const RT *Ie = se >= 0 ? I(se) : nullptr;
@@ -510,8 +529,6 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
             out[pi] = result;
         if (work)
             atomicAdd((unsigned long long *)work, (unsigned long long)cells);
-        if (hist)
-            hist[pi] = result >= 0 ? hbytes : 0;
     }
     return overrun ? -3 : result;
 }
@@ -524,7 +541,7 @@ __device__ __forceinline__ int32_t wfa_pair_dispatch(const SeqView &q, const Seq
                                                      int64_t pi, int32_t *region,
                                                      int64_t slot_width, uint32_t *sq,
                                                      uint32_t *sr, int seqw, int32_t *out,
-                                                     int *err_flag, int64_t *work, int64_t *hist,
+                                                     int *err_flag, int64_t *work,
                                                      uint8_t *hrec = nullptr, int64_t hlimit = 0,
                                                      int hsteps = 0)
 {
@@ -535,21 +552,21 @@ __device__ __forceinline__ int32_t wfa_pair_dispatch(const SeqView &q, const Seq
     if (smem) {
         if (r16)
             res = wfa_align_pair<U, TEAM, true, int16_t, HREC>(q, r, p, w, pi, region, slot_width,
-                                                               sq, sr, out, err_flag, work, hist,
+                                                               sq, sr, out, err_flag, work,
                                                                hrec, hlimit, hsteps);
         if (res == -4)
             res = wfa_align_pair<U, TEAM, true, int32_t, HREC>(q, r, p, w, pi, region, slot_width,
-                                                               sq, sr, out, err_flag, work, hist,
+                                                               sq, sr, out, err_flag, work,
                                                                hrec, hlimit, hsteps);
         return res;
     }
     if (r16)
         res = wfa_align_pair<U, TEAM, false, int16_t, HREC>(q, r, p, w, pi, region, slot_width,
-                                                            sq, sr, out, err_flag, work, hist,
+                                                            sq, sr, out, err_flag, work,
                                                             hrec, hlimit, hsteps);
     if (res == -4)
         res = wfa_align_pair<U, TEAM, false, int32_t, HREC>(q, r, p, w, pi, region, slot_width,
-                                                            sq, sr, out, err_flag, work, hist,
+                                                            sq, sr, out, err_flag, work,
                                                             hrec, hlimit, hsteps);
     return res;
 }
@@ -568,7 +585,7 @@ template <int U, int BW>
 __global__ void __launch_bounds__(32 * BW, BW == 4 ? 5 : 1)
 wfa_kernel(SeqView q, SeqView r, WfaParams p, PairList longs, PairList shorts,
            int32_t *__restrict__ out, int32_t *__restrict__ scratch, int64_t slot_width,
-           int *err_flag, int64_t *work, int64_t *hist)
+           int *err_flag, int64_t *work)
 {
     static_assert(BW >= 4, "team copies need 4 warps' share of shared memory");
     extern __shared__ __align__(16) uint32_t seqs[];
@@ -599,7 +616,7 @@ wfa_kernel(SeqView q, SeqView r, WfaParams p, PairList longs, PairList shorts,
             const int64_t pi = lq ? (int64_t)lq[si] : si;
             wfa_pair_dispatch<U, BW>(q, r, p, w, pi, region, slot_width, seqs,
                                     seqs + 2 * kWfaTeamSeqWords, kWfaTeamSeqWords, out, err_flag,
-                                    work, hist);
+                                    work);
         }
         __syncthreads();  // shared copies of the last long pair are no longer read
     }
@@ -617,7 +634,7 @@ wfa_kernel(SeqView q, SeqView r, WfaParams p, PairList longs, PairList shorts,
             break;
         const int64_t pi = sq ? (int64_t)sq[si] : si;
         wfa_pair_dispatch<U, 1>(q, r, p, w, pi, region, slot_width, my, my + 2 * kWfaSeqWords,
-                                kWfaSeqWords, out, err_flag, work, hist);
+                                kWfaSeqWords, out, err_flag, work);
     }
 }
 
@@ -656,8 +673,17 @@ __device__ __forceinline__ void cigar_pair(const SeqView &q, const SeqView &r, c
     const int64_t limit = 3 * (int64_t)S + hist_cells[pi] / 4;
     const int32_t res = wfa_pair_dispatch<4, TEAM, true>(q, r, p, w, pi, region, slot_width, sq,
                                                          sr, seqw, nullptr, err_flag, nullptr,
-                                                         nullptr, rec, limit, S);
+                                                         rec, limit, S);
     team_sync<TEAM>();  // the record is complete and visible to thread 0
+    // its header beside the walk, where it fits the sequence copies
+    const int32_t *hdr = reinterpret_cast<const int32_t *>(rec);
+    if (3 * (int64_t)S <= 4 * (int64_t)seqw && res == c) {
+        int32_t *const copy = reinterpret_cast<int32_t *>(sq);
+        for (int i = tt; i < 3 * S; i += 32 * TEAM)
+            copy[i] = hdr[i];
+        team_sync<TEAM>();
+        hdr = copy;
+    }
     if (tt != 0)
         return;
     if (res != c) {  // the cost pass and this pass disagree
@@ -665,7 +691,7 @@ __device__ __forceinline__ void cigar_pair(const SeqView &q, const SeqView &r, c
         run_count[pi] = -1;
         return;
     }
-    const int64_t nrun = wfa_traceback(rec, c, w.g, w.xs, w.oes, w.es, (int32_t)qlen,
+    const int64_t nrun = wfa_traceback(rec, hdr, c, w.g, w.xs, w.oes, w.es, (int32_t)qlen,
                                        (int32_t)rlen, runs + run_off[pi], qlen + rlen + 1);
     if (nrun < 0) {
         atomicOr(err_flag, 4);
@@ -789,7 +815,7 @@ int wfa_blocks_per_sm(int variant, int block_warps)
 
 cudaError_t launch_wfa(int variant, int block_warps, SeqView q, SeqView r, WfaParams p,
                        PairList longs, PairList shorts, int32_t *out, int32_t *scratch,
-                       int64_t slot_width, int grid, int *err_flag, int64_t *work, int64_t *hist,
+                       int64_t slot_width, int grid, int *err_flag, int64_t *work,
                        cudaStream_t st)
 {
     // block_warps kWfaWideWarps: the wide kernel (4 diagonals per thread per
@@ -799,19 +825,19 @@ cudaError_t launch_wfa(int variant, int block_warps, SeqView q, SeqView r, WfaPa
         wfa_prepare<4, kWfaWideWarps>();
         wfa_kernel<4, kWfaWideWarps><<<grid, 32 * kWfaWideWarps, wfa_smem_bytes(kWfaWideWarps),
                                        st>>>(q, r, p, longs, shorts, out, scratch, slot_width,
-                                             err_flag, work, hist);
+                                             err_flag, work);
     } else if (variant & 0x20) {
         wfa_prepare<1, 4>();
         wfa_kernel<1, 4><<<grid, 128, wfa_smem_bytes(4), st>>>(
-            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work, hist);
+            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work);
     } else if (variant & 0x10) {
         wfa_prepare<2, 4>();
         wfa_kernel<2, 4><<<grid, 128, wfa_smem_bytes(4), st>>>(
-            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work, hist);
+            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work);
     } else {
         wfa_prepare<4, 4>();
         wfa_kernel<4, 4><<<grid, 128, wfa_smem_bytes(4), st>>>(
-            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work, hist);
+            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work);
     }
     return cudaGetLastError();
 }

@@ -514,7 +514,9 @@ __device__ __forceinline__ int32_t tier_pair16(
     const int32_t tc = cut(target);
     const uint32_t lim_matrix = pack2(-min(rlen, kFar), -min(qlen, kFar));
     const uint32_t lim_target = pack2(tc, -tc);
-    int32_t flo = -min(max_err, kFar), fnhi = flo;
+    // (through a shuffle: the assembler of CUDA 12.9 can lose the sign of a negated kernel
+    // argument when it merges maxima into a 3-way one)
+    int32_t flo = __shfl_sync(FULL, -min(max_err, kFar), 0), fnhi = flo;
     if (band_w > 0) {
         flo = max(flo, cut(min(0, target) - band_w));
         fnhi = max(fnhi, cut(-max(0, target) - band_w));
@@ -720,6 +722,7 @@ __device__ __forceinline__ int32_t tier_pair32(const SeqView &q, const SeqView &
     const int tt = (int)(threadIdx.x % TW);
     const int hm = w.hm, hie = w.hie, xs = w.xs, oes = w.oes, es = w.es, g = w.g;
     const int32_t max_err = p.max_error;
+    const int32_t neg_err = __shfl_sync(FULL, -max_err, 0);  // see flo above
     const int64_t qoff = q.offsets[pi] - q.word_base;
     const int64_t roff = r.offsets[pi] - r.word_base;
     const int32_t qlen = (int32_t)q.lengths[pi], rlen = (int32_t)r.lengths[pi];
@@ -772,7 +775,7 @@ __device__ __forceinline__ int32_t tier_pair32(const SeqView &q, const SeqView &
                 lo = min(lo, target);
                 hi = max(hi, target);
             }
-            lo = max(lo, -max_err);
+            lo = max(lo, neg_err);
             hi = min(hi, max_err);
             if (ub >= 0) {
                 // a diagonal k at score s costs at least s + e*|k - target| to finish

@@ -21,15 +21,20 @@ namespace gb2 {
 
 struct WfaHist {
     const uint8_t *rec;
-    const int32_t *hdr;
-    __device__ __forceinline__ int32_t mafter(int sp, int32_t k) const
+    const int32_t *hdr;  // the record's header, or a copy of it
+    // M after extension and the decision of one cell
+    __device__ __forceinline__ void cell(int sp, int32_t k, int32_t &m, uint32_t &d) const
     {
+        m = -(1 << 30);
+        d = 0;
         if (sp < 0)
-            return -(1 << 30);
+            return;
         const int32_t a = hdr[3 * sp], b = hdr[3 * sp + 1];
         if (k < a || k > b)
-            return -(1 << 30);
-        return reinterpret_cast<const int32_t *>(rec)[hdr[3 * sp + 2] + (k - a)];
+            return;
+        const int64_t off = hdr[3 * sp + 2];
+        m = reinterpret_cast<const int32_t *>(rec)[off + (k - a)];
+        d = rec[(off + (b - a + 1)) * 4 + (k - a)];
     }
     __device__ __forceinline__ uint32_t dec(int sp, int32_t k) const
     {
@@ -46,11 +51,12 @@ struct WfaHist {
 // Runs of the optimal alignment of cost c (score index c/g, diagonal
 // qlen - rlen) into dst[0 .. cap); returns their count, or -1 when the record
 // is inconsistent or the runs do not fit.  Sequential (one thread).
-__device__ __forceinline__ int64_t wfa_traceback(const uint8_t *rec, int32_t c, int g, int xs,
+__device__ __forceinline__ int64_t wfa_traceback(const uint8_t *rec, const int32_t *hdr, int32_t c,
+                                                 int g, int xs,
                                                  int oes, int es, int32_t qlen, int32_t rlen,
                                                  uint32_t *dst, int64_t cap)
 {
-    const WfaHist h{rec, reinterpret_cast<const int32_t *>(rec)};
+    const WfaHist h{rec, hdr};
     int64_t nrun = 0;
     uint32_t cur_op = 4, cur_len = 0;
     bool bad = false;
@@ -71,78 +77,48 @@ __device__ __forceinline__ int64_t wfa_traceback(const uint8_t *rec, int32_t c, 
         cur_op = op;
         cur_len = (uint32_t)cnt;
     };
-    int sp = c / g, mode = 0;
-    int32_t k = qlen - rlen, crow = h.mafter(sp, k);
+    // the M value and the decision of the cell the walk is at: both depend only on where
+    // it is, so they are loaded together, one memory latency per step
+    int sp = c / g;
+    int32_t k = qlen - rlen, crow = 0;
+    uint32_t d = 0;
+    h.cell(sp, k, crow, d);
     for (int64_t guard = 4 * ((int64_t)qlen + rlen) + 16; !bad; --guard) {
         if (guard <= 0 || sp < 0) {
             bad = true;
             break;
         }
-        if (mode == 0) {
-            const uint32_t src = h.dec(sp, k) & 3u;
-            int32_t before;
-            if (sp == 0) {
-                before = 0;  // M[0, 0] = 0 before extension
-            } else if (src == 1) {
-                before = h.mafter(sp - xs, k) + 1;
-            } else if (src == 2) {
-                int ssp = sp, j = 0;
-                int32_t kk = k;
-                while (ssp >= 0 && (h.dec(ssp, kk) & 4u)) {
-                    ssp -= es;
-                    kk -= 1;
-                    ++j;
-                }
-                before = h.mafter(ssp - oes, kk - 1) + 1 + j;
-            } else if (src == 3) {
-                int ssp = sp;
-                int32_t kk = k;
-                while (ssp >= 0 && (h.dec(ssp, kk) & 8u)) {
-                    ssp -= es;
-                    kk += 1;
-                }
-                before = h.mafter(ssp - oes, kk + 1);
-            } else {
+        const uint32_t src = d & 3u;
+        if (sp == 0) {
+            emit(0, crow);  // M[0, 0] = 0 before extension
+            if (k != 0)
                 bad = true;
-                break;
-            }
-            emit(0, crow - before);
-            crow = before;
-            if (sp == 0) {
-                if (k != 0)
-                    bad = true;
-                break;
-            }
-            if (src == 1) {
-                emit(1, 1);
-                sp -= xs;
-                crow = h.mafter(sp, k);
-            } else {
-                mode = (int)src - 1;  // 1: I, 2: D
-            }
-        } else if (mode == 1) {
-            emit(2, 1);
-            if (h.dec(sp, k) & 4u) {
+            break;
+        }
+        const int32_t after = crow;
+        if (src == 1) {
+            sp -= xs;
+            h.cell(sp, k, crow, d);
+            emit(0, after - (crow + 1));
+            emit(1, 1);
+        } else if (src == 2 || src == 3) {
+            // back over the gap's extensions to its open: I takes a row per base, D none
+            const uint32_t bit = src == 2 ? 4u : 8u;
+            const int32_t dk = src == 2 ? -1 : 1;
+            int32_t j = 1;
+            while (sp >= 0 && (d & bit)) {
                 sp -= es;
-                k -= 1;
-                crow -= 1;
-            } else {
-                sp -= oes;
-                k -= 1;
-                crow = h.mafter(sp, k);
-                mode = 0;
+                k += dk;
+                ++j;
+                d = h.dec(sp, k);
             }
+            sp -= oes;
+            k += dk;
+            h.cell(sp, k, crow, d);
+            emit(0, after - (crow + (src == 2 ? j : 0)));
+            emit(src, j);
         } else {
-            emit(3, 1);
-            if (h.dec(sp, k) & 8u) {
-                sp -= es;
-                k += 1;
-            } else {
-                sp -= oes;
-                k += 1;
-                crow = h.mafter(sp, k);
-                mode = 0;
-            }
+            bad = true;
         }
     }
     if (!bad && cur_len) {

@@ -151,3 +151,37 @@ def test_short_pairs(device, oracle, pen):
         _check(device, oracle, q, r, WFAConfig(*pen, me), (100,))
     q, r = _pack(qs + [_rnd(rng, 513)]), _pack(rs + [_rnd(rng, 500)])
     _check(device, oracle, q, r, WFAConfig(*pen, 300), (100,))
+
+
+@pytest.mark.parametrize("pen", [(4, 6, 2), (3, 5, 2), (7, 1, 3), (5, 0, 5), (1, 0, 1), (9, 4, 6)])
+def test_cigars_of_the_pruned_history(device, oracle, pen):
+    """The CIGAR pass visits only diagonals that can finish within the known cost, in a
+    record sized from the cost: the strings, ties included, are the reference's, over
+    repeats (many equal alignments), one-sided length differences, unrelated pairs and
+    costs many times the lengths."""
+    rng = np.random.default_rng(pen[0] + 10 * pen[2])
+    unit = _rnd(rng, 7)
+    qs, rs = [], []
+    for k in range(60):
+        t = _rnd(rng, int(rng.integers(0, 90)))
+        if k % 4 == 1:
+            t = np.tile(unit, int(rng.integers(1, 13)))
+        q = _mutate(rng, t, float(rng.choice([0.02, 0.1, 0.3])))
+        if k % 6 == 2:
+            q = q[len(q) // 2:]
+        elif k % 6 == 3:
+            t = t[:len(t) // 3]
+        elif k % 6 == 4:
+            q = _rnd(rng, int(rng.integers(0, 60)))
+        qs.append(q)
+        rs.append(t)
+    letters = ["".join("ACGT"[c] for c in s) for s in qs], ["".join("ACGT"[c] for c in s) for s in rs]
+    q, r = _pack(qs), _pack(rs)
+    for me in (900, 60):
+        expect = [oracle.wfa_cigar(a, b, *pen, me) for a, b in zip(*letters)]
+        for copies in (1, 40):
+            cost, cig = device.wfa_cigar(_copies(q, copies), _copies(r, copies),
+                                         WFAConfig(*pen, me))
+            for i, want in enumerate(expect):
+                for j in (i, i + (copies - 1) * len(qs)):
+                    assert (int(cost[j]), cig[j]) == want, (pen, me, letters[0][i], letters[1][i])
