@@ -725,10 +725,10 @@ int wfa_validate(gb2_ctx *c, const gb2_wfa_cfg *cfg, int64_t n)
 int wfa_begin(gb2_ctx *c, Exec &x)
 {
     int rc;
-    if ((rc = ensure(c, x.errflag, 64, x.st)) || (rc = ensure(c, x.work, 64, x.st)))
+    // the error flag at 0, the work counter at kWorkOffset: one memset, one copy back
+    if ((rc = ensure(c, x.errflag, 2 * kWorkOffset, x.st)))
         return rc;
-    CU(c, cudaMemsetAsync(x.errflag.p, 0, 64, x.st));
-    CU(c, cudaMemsetAsync(x.work.p, 0, 64, x.st));
+    CU(c, cudaMemsetAsync(x.errflag.p, 0, 2 * kWorkOffset, x.st));
     return GB2_OK;
 }
 
@@ -856,7 +856,7 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         io.next = tq + n * G;
         io.next_n = s_ctr + kCounterStride;
         cudaEvent_t e0 = prof_begin(c, x.st);
-        CU(c, launch_wfa_short(pl, (int)sms, qv, rv, p, io, d_out, (int64_t *)x.work.p, x.st));
+        CU(c, launch_wfa_short(pl, (int)sms, qv, rv, p, io, d_out, wfa_work(x), x.st));
         prof_end(c, e0, x.st);
         c->launches += 1;
     }
@@ -901,7 +901,7 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         // are pairs spread a small batch over the SMs
         const int grid = (int)(t == first ? std::min<int64_t>(sms, n) : sms);
         cudaEvent_t e0 = prof_begin(c, x.st);
-        CU(c, launch_wfa_tier(pl, t, grid, qv, rv, p, io, d_out, (int64_t *)x.work.p,
+        CU(c, launch_wfa_tier(pl, t, grid, qv, rv, p, io, d_out, wfa_work(x),
                               (int *)x.errflag.p, x.st));
         prof_end(c, e0, x.st);
         c->launches += 1;
@@ -921,7 +921,7 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
             bp.band_w = kWfaBoundBand;
             bp.gring = io.gring;
             cudaEvent_t e1 = prof_begin(c, x.st);
-            CU(c, launch_wfa_tier(pl, 0, (int)sms, qv, rv, p, bp, d_ub, (int64_t *)x.work.p,
+            CU(c, launch_wfa_tier(pl, 0, (int)sms, qv, rv, p, bp, d_ub, wfa_work(x),
                                   (int *)x.errflag.p, x.st));
             prof_end(c, e1, x.st);
             c->launches += 1;
@@ -1025,7 +1025,7 @@ int wfa_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t 
     }
     cudaEvent_t e0 = prof_begin(c, x.st);
     CU(c, launch_wfa(variant, bw, qv, rv, p, longs, shorts, d_out, (int32_t *)x.scratch32.p,
-                     slot_width, (int)grid, (int *)x.errflag.p, (int64_t *)x.work.p, x.st));
+                     slot_width, (int)grid, (int *)x.errflag.p, wfa_work(x), x.st));
     prof_end(c, e0, x.st);
     c->launches += 1;
     return GB2_OK;
@@ -1033,11 +1033,14 @@ int wfa_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t 
 
 int wfa_end(gb2_ctx *c, Exec &x)
 {
-    int flag = 0;
-    int64_t work = 0;
-    CU(c, cudaMemcpyAsync(&flag, x.errflag.p, 4, cudaMemcpyDeviceToHost, x.st));
-    CU(c, cudaMemcpyAsync(&work, x.work.p, 8, cudaMemcpyDeviceToHost, x.st));
+    static_assert(kWorkOffset + 8 <= kPinSmall, "pinned words");
+    char *const pin = (char *)c->pin_small + (&x == &c->x2 ? kPinSmall : 0);
+    CU(c, cudaMemcpyAsync(pin, x.errflag.p, kWorkOffset + 8, cudaMemcpyDeviceToHost, x.st));
     CU(c, cudaStreamSynchronize(x.st));
+    int flag;
+    int64_t work;
+    memcpy(&flag, pin, sizeof flag);
+    memcpy(&work, pin + kWorkOffset, sizeof work);
     c->work_units += work;
     if (flag)
         return set_err(c, GB2_EKERNEL, "WFA kernel reported a pair longer than its scratch");
@@ -1169,7 +1172,8 @@ static void key_batches(std::vector<int64_t> &k, const gb2_batch *q, const gb2_b
 }
 
 // Pinned host staging for results.
-static int pin_out(gb2_ctx *c, size_t bytes)
+namespace gb2 {
+int pin_out(gb2_ctx *c, size_t bytes)
 {
     if (bytes <= c->pin_out_cap)
         return GB2_OK;
@@ -1182,22 +1186,45 @@ static int pin_out(gb2_ctx *c, size_t bytes)
     return GB2_OK;
 }
 
-static int d2h_results(gb2_ctx *c, void *host, const void *dev, size_t bytes)
+void touch_pages(void *p, size_t bytes)
 {
-    if (bytes == 0)
-        return GB2_OK;
-    if (is_pinned(host)) {
-        CU(c, cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->x.st));
-        return sync_and_check(c);
+    // a new array's pages are faulted in one by one (6 MB of results: 0.4-0.7 ms)
+    volatile char *const b = (volatile char *)p;
+    for (size_t i = 0; i < bytes; i += 4096)
+        b[i] = b[i];
+}
+
+int parts_to_host(gb2_ctx *c, gb2_sw_result *out, int64_t n, int64_t per, int parts)
+{
+    touch_pages(out, (size_t)n * sizeof(gb2_sw_result));
+    for (int k = 0; k < parts; ++k) {
+        const int64_t p0 = k * per, m = std::min(per, n - p0);
+        CU(c, cudaEventSynchronize(c->kback[k]));
+        memcpy(out + p0, (gb2_sw_result *)c->pin_out + p0, (size_t)m * sizeof(gb2_sw_result));
     }
-    int rc = pin_out(c, bytes);
-    if (rc)
-        return rc;
-    CU(c, cudaMemcpyAsync(c->pin_out, dev, bytes, cudaMemcpyDeviceToHost, c->x.st));
-    if ((rc = sync_and_check(c)))
-        return rc;
-    memcpy(host, c->pin_out, bytes);
     return GB2_OK;
+}
+}  // namespace gb2
+
+// Results of the work queued on c->x.st into the caller's array.  d2h_begin queues the
+// copy; d2h_end, after c->x.st is idle, finishes it.  A pageable array goes through the
+// context's pinned staging, and while the GPU works its pages are brought in.
+static int d2h_begin(gb2_ctx *c, void *host, const void *dev, size_t bytes, bool &staged)
+{
+    staged = !is_pinned(host);
+    int rc;
+    if (staged && (rc = pin_out(c, bytes)))
+        return rc;
+    CU(c, cudaMemcpyAsync(staged ? c->pin_out : host, dev, bytes, cudaMemcpyDeviceToHost, c->x.st));
+    if (staged)
+        touch_pages(host, bytes);
+    return GB2_OK;
+}
+
+static void d2h_end(gb2_ctx *c, void *host, size_t bytes, bool staged)
+{
+    if (staged)
+        memcpy(host, c->pin_out, bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -1631,7 +1658,9 @@ int gb2_create(int device, gb2_ctx **out)
             cudaEventRecord(c->pin_ev[i], c->x.st);
     }
     for (int i = 0; ok && i < kResidentParts; ++i)
-        ok = cudaEventCreateWithFlags(&c->kdone[i], cudaEventDisableTiming) == cudaSuccess;
+        ok = cudaEventCreateWithFlags(&c->kdone[i], cudaEventDisableTiming) == cudaSuccess &&
+             cudaEventCreateWithFlags(&c->kback[i], cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && pinned_alloc(&c->pin_small, 2 * kPinSmall) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; ok && i < kPipeSets; ++i) {
         PipeSet &ps = c->pipe[i];
@@ -1664,7 +1693,7 @@ int gb2_destroy(gb2_ctx *c)
     exec_free(c->x);
     exec_free(c->x2);
     CigarBufs &cb = c->cig;
-    DevBuf *bufs[] = {&c->out_sw,     &c->out_wfa,  &c->bands,     &c->flush,
+    DevBuf *bufs[] = {&c->out_sw,     &c->out_wfa,  &c->bands,     &c->flush,   &c->pair_in,
                       &cb.cost,       &cb.hist,     &cb.pairs,     &cb.arena_off,
                       &cb.arena,      &cb.runs,     &cb.run_off,   &cb.run_count,
                       &cb.out_off,    &cb.out};
@@ -1683,8 +1712,13 @@ int gb2_destroy(gb2_ctx *c)
                 cudaEventDestroy(e);
     }
     for (int i = 0; i < kResidentParts; ++i)
-        if (c->kdone[i])
-            cudaEventDestroy(c->kdone[i]);
+        for (cudaEvent_t e : {c->kdone[i], c->kback[i]})
+            if (e)
+                cudaEventDestroy(e);
+    if (c->pin_small)
+        cudaFreeHost(c->pin_small);
+    if (c->pin_pair)
+        cudaFreeHost(c->pin_pair);
     if (c->ev_join2)
         cudaEventDestroy(c->ev_join2);
     for (int i = 0; i < 2; ++i) {
@@ -1875,21 +1909,28 @@ static int gb2_sw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
             cudaStreamSynchronize(c->x.st);
             return rc;
         }
-        return d2h_results(c, out, c->out_sw.p, (size_t)n * sizeof(gb2_sw_result));
+        bool staged;
+        if ((rc = d2h_begin(c, out, c->out_sw.p, (size_t)n * sizeof(gb2_sw_result), staged)) ||
+            (rc = sync_and_check(c)))
+            return rc;
+        d2h_end(c, out, (size_t)n * sizeof(gb2_sw_result), staged);
+        return GB2_OK;
     }
     const bool out_pinned = is_pinned(out);
     if (!out_pinned && (rc = pin_out(c, (size_t)n * sizeof(gb2_sw_result))))
         return rc;
     gb2_sw_result *const host = out_pinned ? out : (gb2_sw_result *)c->pin_out;
     gb2_sw_result *const dres = (gb2_sw_result *)c->out_sw.p;
+    const int64_t per = (n + parts - 1) / parts;
+    bool eager = false;  // the parts' copies have their events
     auto issue = [&](bool capturing) -> int {
+        eager = !capturing;
         CU(c, cudaEventRecord(c->x.ev_fork, c->x.st));  // bands copied before either runs
         CU(c, cudaStreamWaitEvent(c->x2.st, c->x.ev_fork, 0));
         // profiling: one span per call, from the first part's start to the later
         // of the two executors' last kernels (the parts overlap, so their own
         // durations would double-count)
         cudaEvent_t span0 = capturing ? nullptr : prof_begin(c, c->x.st);
-        const int64_t per = (n + parts - 1) / parts;
         int r2 = GB2_OK;
         for (int k = 0; k < parts && r2 == GB2_OK; ++k) {
             const int64_t p0 = k * per, m = std::min(per, n - p0);
@@ -1906,6 +1947,8 @@ static int gb2_sw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
             if (!r2 && cudaMemcpyAsync(host + p0, dres + p0, (size_t)m * sizeof(gb2_sw_result),
                                        cudaMemcpyDeviceToHost, ex.st) != cudaSuccess)
                 r2 = set_err(c, GB2_ECUDA, "result copy failed");
+            if (!r2 && !capturing && cudaEventRecord(c->kback[k], ex.st) != cudaSuccess)
+                r2 = set_err(c, GB2_ECUDA, "event record failed");
         }
         // the second executor joins the first (a captured graph must end there)
         if (!r2 && (cudaEventRecord(c->ev_join2, c->x2.st) != cudaSuccess ||
@@ -1921,6 +1964,9 @@ static int gb2_sw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
         return r2;
     };
     rc = run_graphed(c, c->g_sw, key, flags, (char *)host, issue);
+    const bool by_part = !rc && eager && !out_pinned;
+    if (by_part && (rc = parts_to_host(c, out, n, per, parts)))
+        return rc;
     const cudaError_t e2 = cudaStreamSynchronize(c->x2.st);
     const int rc2 = sync_and_check(c);
     if (rc)
@@ -1929,7 +1975,7 @@ static int gb2_sw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
         return set_err(c, GB2_ECUDA, "second executor: %s", cudaGetErrorString(e2));
     if (rc2)
         return rc2;
-    if (!out_pinned)
+    if (!out_pinned && !by_part)
         memcpy(out, c->pin_out, (size_t)n * sizeof(gb2_sw_result));
     return GB2_OK;
 }
@@ -1982,6 +2028,44 @@ int gb2_sw_banded_host(gb2_ctx *c, const uint64_t *q_packed, const int64_t *q_of
     return drain_on_error(c, gb2_sw_banded_host_impl(c, q_packed, q_offsets, q_lengths, r_packed, r_offsets, r_lengths, cfg, bands, n, out, flags));
 }
 
+// One pair: lengths, offsets and words in one pinned staging array and one copy to the
+// device (the host pipeline would make three copies and rebuild the offsets there).  Pairs
+// of longer sequences take the pipeline.  Context lock held.
+constexpr int64_t kPairBases = 1 << 21;  // 512 KiB of words
+
+static int pair_upload(gb2_ctx *c, const uint64_t *q_words, int64_t qlen, const uint64_t *r_words,
+                       int64_t rlen, SeqView &qv, SeqView &rv)
+{
+    const int64_t qn = std::max<int64_t>(words_for(qlen), 1);
+    const int64_t rn = std::max<int64_t>(words_for(rlen), 1);
+    const size_t bytes = (size_t)(4 + qn + rn) * 8;
+    int rc;
+    if ((rc = ensure(c, c->pair_in, bytes, c->x.st)))
+        return rc;
+    if (bytes > c->pin_pair_cap) {
+        if (c->pin_pair)
+            cudaFreeHost(c->pin_pair);
+        c->pin_pair = nullptr;
+        c->pin_pair_cap = 0;
+        const size_t cap = std::max<size_t>(2 * bytes, 16384);
+        CU(c, pinned_alloc(&c->pin_pair, cap));
+        c->pin_pair_cap = cap;
+    }
+    int64_t *const h = (int64_t *)c->pin_pair;  // free: the last call waited for its copy
+    h[0] = 0;
+    h[1] = qlen;
+    h[2] = 0;
+    h[3] = rlen;
+    h[4] = h[4 + qn] = 0;
+    memcpy(h + 4, q_words, (size_t)words_for(qlen) * 8);
+    memcpy(h + 4 + qn, r_words, (size_t)words_for(rlen) * 8);
+    CU(c, cudaMemcpyAsync(c->pair_in.p, h, bytes, cudaMemcpyHostToDevice, c->x.st));
+    const int64_t *const d = (const int64_t *)c->pair_in.p;
+    qv = SeqView{(const uint64_t *)d + 4, d, d + 1, 0, qn};
+    rv = SeqView{(const uint64_t *)d + 4 + qn, d + 2, d + 3, 0, rn};
+    return GB2_OK;
+}
+
 static int gb2_sw_pair_impl(gb2_ctx *c, const uint64_t *q_words, int64_t qlen, const uint64_t *r_words,
                 int64_t rlen, const gb2_sw_cfg *cfg, gb2_sw_result *out)
 {
@@ -1989,6 +2073,27 @@ static int gb2_sw_pair_impl(gb2_ctx *c, const uint64_t *q_words, int64_t qlen, c
         return GB2_EINVAL;
     if (!out || qlen < 0 || rlen < 0 || (qlen > 0 && !q_words) || (rlen > 0 && !r_words))
         return set_err(c, GB2_EINVAL, "bad pair arguments");
+    if (qlen <= kPairBases && rlen <= kPairBases) {
+        std::lock_guard<std::mutex> lk(c->mu);
+        cudaSetDevice(c->device);
+        SwPlanInfo pi;
+        SeqView qv, rv;
+        int rc;
+        if ((rc = sw_validate(c, cfg, nullptr, 1, qlen, rlen, pi)))
+            return rc;
+        pi.narrow_lengths = narrow_range(qlen, qlen) && narrow_range(rlen, rlen);
+        if ((rc = ensure(c, c->out_sw, sizeof(gb2_sw_result), c->x.st)) ||
+            (rc = pair_upload(c, q_words, qlen, r_words, rlen, qv, rv)) ||
+            (rc = sw_core(c, c->x, qv, rv, qlen, rlen, cfg, nullptr, pi, 1,
+                          (gb2_sw_result *)c->out_sw.p, GB2_FLAG_PLAIN)))
+            return rc;
+        CU(c, cudaMemcpyAsync(c->pin_small, c->out_sw.p, sizeof(gb2_sw_result),
+                              cudaMemcpyDeviceToHost, c->x.st));
+        if ((rc = sync_and_check(c)))
+            return rc;
+        memcpy(out, c->pin_small, sizeof(gb2_sw_result));
+        return GB2_OK;
+    }
     const int64_t qo = 0, ro = 0;
     static const uint64_t zero = 0;
     return gb2_sw_banded_host(c, qlen ? q_words : &zero, &qo, &qlen, rlen ? r_words : &zero, &ro,
@@ -2038,9 +2143,12 @@ static int gb2_wfa_affine_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *
         cudaStreamSynchronize(c->x.st);
         return rc;
     }
-    if ((rc = wfa_end(c, c->x)))
+    bool staged;
+    if ((rc = d2h_begin(c, out, c->out_wfa.p, (size_t)n * 4, staged)) || (rc = wfa_end(c, c->x)))
         return rc;
-    return d2h_results(c, out, c->out_wfa.p, (size_t)n * 4);
+    harvest_profile(c);
+    d2h_end(c, out, (size_t)n * 4, staged);
+    return GB2_OK;
 }
 
 int gb2_wfa_affine(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r, const gb2_wfa_cfg *cfg,
@@ -2096,6 +2204,22 @@ static int gb2_wfa_pair_impl(gb2_ctx *c, const uint64_t *q_words, int64_t qlen, 
         return GB2_EINVAL;
     if (!out || qlen < 0 || rlen < 0 || (qlen > 0 && !q_words) || (rlen > 0 && !r_words))
         return set_err(c, GB2_EINVAL, "bad pair arguments");
+    if (qlen <= kPairBases && rlen <= kPairBases) {
+        std::lock_guard<std::mutex> lk(c->mu);
+        cudaSetDevice(c->device);
+        SeqView qv, rv;
+        int rc;
+        // the cost beside the error flag and the work counter: one copy back
+        if ((rc = wfa_validate(c, cfg, 1)) || (rc = wfa_begin(c, c->x)) ||
+            (rc = pair_upload(c, q_words, qlen, r_words, rlen, qv, rv)) ||
+            (rc = wfa_core(c, c->x, qv, rv, qlen, rlen, cfg, 1,
+                           (int32_t *)c->x.errflag.p + 1, GB2_FLAG_PLAIN)) ||
+            (rc = wfa_end(c, c->x)))
+            return rc;
+        harvest_profile(c);
+        memcpy(out, (const int32_t *)c->pin_small + 1, sizeof *out);
+        return GB2_OK;
+    }
     const int64_t qo = 0, ro = 0;
     static const uint64_t zero = 0;
     return gb2_wfa_affine_host(c, qlen ? q_words : &zero, &qo, &qlen, rlen ? r_words : &zero, &ro,

@@ -62,6 +62,11 @@ struct Exec {
     DevBuf ubound;        // WFA: per pair, the bound pass's cost (an upper bound of the optimum)
 };
 
+// WFA status buffer of an executor (Exec::errflag): the error flag, then the work counter
+constexpr size_t kWorkOffset = 64;
+constexpr size_t kPinSmall = 128;
+inline int64_t *wfa_work(Exec &x) { return (int64_t *)((char *)x.errflag.p + kWorkOffset); }
+
 // Device buffers of the WFA CIGAR entry point (grow-only, per context).
 struct CigarBufs {
     DevBuf cost, hist, pairs, arena_off, arena, runs, run_off, run_count, out_off, out;
@@ -172,6 +177,11 @@ struct gb2_ctx {
     gb2::PipeSet pipe[gb2::kPipeSets];
     gb2::CigarBufs cig;
     cudaEvent_t kdone[gb2::kResidentParts] = {};  // last kernel of each resident part
+    cudaEvent_t kback[gb2::kResidentParts] = {};  // its results are on the host
+    void *pin_small = nullptr;   // two times kPinSmall bytes: the executors' status words
+    void *pin_pair = nullptr;    // staging of the per-pair calls
+    size_t pin_pair_cap = 0;
+    gb2::DevBuf pair_in;
     cudaEvent_t ev_join2 = nullptr;  // second executor joined back into the first
     uint64_t buf_gen = 0;            // bumped whenever a context buffer is reallocated
     gb2::GraphCache g_sw, g_wfa;     // replay caches of gb2_sw_banded / gb2_wfa_affine
@@ -251,6 +261,12 @@ bool is_pinned(const void *p);
 // context's two pinned staging halves.
 int h2d(gb2_ctx *c, void *dst, const void *src, size_t bytes, cudaStream_t st);
 int64_t words_for(int64_t len);
+// Grows the context's pinned result staging (c->pin_out).
+int pin_out(gb2_ctx *c, size_t bytes);
+// Brings the pages of a result array in (its contents stay), for use while the GPU works.
+void touch_pages(void *p, size_t bytes);
+// Copies the parts of n results from c->pin_out to out as their c->kback events pass.
+int parts_to_host(gb2_ctx *c, gb2_sw_result *out, int64_t n, int64_t per, int parts);
 void harvest_profile(gb2_ctx *c);
 
 int sw_validate(gb2_ctx *c, const gb2_sw_cfg *cfg, const int32_t *bands, int64_t n, int64_t qmax,

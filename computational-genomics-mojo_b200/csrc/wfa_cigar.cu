@@ -46,6 +46,9 @@ __global__ void k_compact_runs(int64_t n, const uint32_t *__restrict__ runs,
 
 using namespace gb2;
 
+// Runs of up to this many bytes come back through pinned staging.
+constexpr int64_t kRunsStaged = 16 << 20;
+
 // Host side of gb2_wfa_cigar: the cost pass, then the CIGAR pass in groups of
 // pairs whose history records fit the arena budget, then the runs gathered.
 static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_qlen,
@@ -92,9 +95,8 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
                               x.st));
     // per pair: record bytes, run capacity and its offset
     std::vector<int64_t> rec((size_t)n), run_off((size_t)n);
-    int64_t run_total = 0, rec_max = 0;
+    int64_t run_total = 0, rec_max = 0, edits = 0;
     std::vector<int32_t> order;
-    order.reserve((size_t)n);
     for (int64_t i = 0; i < n; ++i) {
         run_off[(size_t)i] = run_total;
         run_total += h_qlen[i] + h_rlen[i] + 1;
@@ -102,16 +104,38 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
         if (cost[i] > 0 || (cost[i] == 0 && (h_qlen[i] | h_rlen[i]))) {
             rec[(size_t)i] = wfa_hist_record_bytes(hist[(size_t)i], cost[i] / g + 1);
             rec_max = std::max(rec_max, rec[(size_t)i]);
+            edits += 2 * (int64_t)(cost[i] / std::max(1, std::min(cfg->x, cfg->o + cfg->e))) + 1;
         }
-        order.push_back((int32_t)i);
     }
-    // largest records first: they carry the longest dependency chains
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t a, int32_t b) { return rec[(size_t)a] > rec[(size_t)b]; });
-    size_t free_b = 0, total_b = 0;
-    GB2_CU(c, cudaMemGetInfo(&free_b, &total_b));
-    int64_t budget = std::min<int64_t>((int64_t)free_b / 2,
-                                       arena_mib ? (int64_t)arena_mib << 20 : kCigarArenaCap);
+    // largest records first: they carry the longest dependency chains (by 4,096 classes of
+    // size: the order within one does not matter)
+    {
+        constexpr int64_t kClasses = 4096;
+        const int64_t width = rec_max / kClasses + 1;
+        std::vector<int32_t> at((size_t)kClasses + 1, 0);
+        const auto cls = [&](int64_t i) {
+            return (size_t)(kClasses - rec[(size_t)i] / width);
+        };
+        for (int64_t i = 0; i < n; ++i)
+            at[cls(i)] += rec[(size_t)i] > 0;
+        for (int64_t k = 1; k <= kClasses; ++k)
+            at[(size_t)k] += at[(size_t)k - 1];
+        order.resize((size_t)at[(size_t)kClasses]);
+        for (int64_t i = n - 1; i >= 0; --i)
+            if (rec[(size_t)i] > 0)
+                order[(size_t)--at[cls(i)]] = (int32_t)i;
+    }
+    int64_t all_rec = 0;
+    for (int64_t i = 0; i < n; ++i)
+        all_rec += rec[(size_t)i];
+    // The arena: all records when they fit what is there already (asking for the free
+    // memory takes about a millisecond), else at most half the free memory.
+    int64_t budget = arena_mib ? (int64_t)arena_mib << 20 : kCigarArenaCap;
+    if (std::min(budget, all_rec) > (int64_t)cb.arena.cap) {
+        size_t free_b = 0, total_b = 0;
+        GB2_CU(c, cudaMemGetInfo(&free_b, &total_b));
+        budget = std::min<int64_t>((int64_t)free_b / 2, budget);
+    }
     if (rec_max >= (1ll << 33))  // header offsets are int32 counts of 4-byte words
         return set_err(c, GB2_ERANGE, "one pair's WFA history needs %lld bytes (limit 8 GiB)",
                        (long long)rec_max);
@@ -127,10 +151,6 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
     int64_t grid = (int64_t)c->sm_count * wfa_cigar_blocks_per_sm();
     grid = std::min(grid, std::max<int64_t>(c->sm_count, kWfaScratchCap / (4 * warp_bytes)));
     grid = std::min(grid, std::max<int64_t>(1, (n + 3) / 4));
-    // the arena: the budget, or all records when they fit in less
-    int64_t all_rec = 0;
-    for (int64_t i = 0; i < n; ++i)
-        all_rec += rec[(size_t)i];
     const int64_t arena_bytes = std::max<int64_t>(16, std::min(budget, all_rec));
     if ((rc = ensure(c, x.scratch32, (size_t)(grid * 4 * warp_bytes), x.st)) ||
         (rc = ensure(c, x.counters, kCounterBytes, x.st)) ||
@@ -175,6 +195,8 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
                                    (uint32_t *)cb.runs.p, (const int64_t *)cb.run_off.p,
                                    (int32_t *)cb.run_count.p, (int *)x.errflag.p, x.st));
         c->launches += 1;
+        if (g0 == 0)  // while the GPU works: the runs' pages (two per edit at most)
+            touch_pages(runs, (size_t)std::min(runs_cap, edits) * 4);
         // the host arrays of this group stay untouched until its copies are done
         GB2_CU(c, cudaStreamSynchronize(x.st));
         g0 = g1;
@@ -207,8 +229,16 @@ static int wfa_cigar_run(gb2_ctx *c, SeqView qv, SeqView rv, const int64_t *h_ql
                                              (const int64_t *)cb.out_off.p, (uint32_t *)cb.out.p);
     GB2_CU(c, cudaGetLastError());
     c->launches += 1;
-    GB2_CU(c, cudaMemcpyAsync(runs, cb.out.p, (size_t)total * 4, cudaMemcpyDeviceToHost, x.st));
+    // through pinned staging, whose first use costs about as much as it saves on a few
+    // MiB: long outputs go directly
+    const bool staged = total * 4 <= kRunsStaged && !is_pinned(runs);
+    if (staged && (rc = pin_out(c, (size_t)total * 4)))
+        return rc;
+    GB2_CU(c, cudaMemcpyAsync(staged ? c->pin_out : runs, cb.out.p, (size_t)total * 4,
+                              cudaMemcpyDeviceToHost, x.st));
     GB2_CU(c, cudaStreamSynchronize(x.st));
+    if (staged)
+        memcpy(runs, c->pin_out, (size_t)total * 4);
     return GB2_OK;
 }
 
