@@ -1,5 +1,6 @@
 // gb2_internal.cuh -- shared declarations of libgenomics_b200 (not installed).
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -66,6 +67,22 @@ namespace gb2 {
 struct SwParams {
     int32_t match, mismatch, go, ge;
 };
+
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device (the setting
+// is the device's, so it is made once on each).
+template <typename K>
+cudaError_t allow_smem(K *kernel, int bytes, std::atomic<uint64_t> &done)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (e != cudaSuccess || (done.load(std::memory_order_relaxed) & bit))
+        return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64)
+        done.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
 
 // band_class flag selecting the packed int16x2 kernel of one thread per pair (bands 16
 // and 32, scores up to kPackHmax).

@@ -258,53 +258,67 @@ sw_band_kernel(SeqView q, SeqView r, SwParams p, PairList pl, gb2_sw_result *__r
 // Without the max(E, 0) clamp E differs from the reference's E only in
 // non-positive values, which never reach H (H takes max(.., 0)); the
 // -1000000 start of the chain at column 0 becomes a large negative value.
-// Bits: H <= 511 in every cell (the host checks match*min(qlen, rlen)), all
-// terms stay inside int16, the first-maximum key H*128 + (127-column) fits
-// an unsigned 16-bit half, and the per-half subtract of |go+ge| cannot
-// borrow because H' >= |go+ge|.
+// Bits: H <= 511 in every cell (the host checks match*(min(qlen, rlen) + 1)), all
+// terms stay inside int16, and the first-maximum key H*128 + (127-column) fits
+// an unsigned 16-bit half.
 //
-// Pipe balance.  The three DPX max instructions per register run on the
-// integer ALU pipe, which this recurrence saturates; the FMA pipe (integer
-// multiply-add) is a separate pipe of the same width.  So every step that a
-// multiply-add can do runs there, with multipliers passed as kernel
-// arguments (Pack16Consts) so the compiler cannot turn them back into
-// shifts:
-//  - the substitution score of both cells of a register is one mad.hi: the
-//    equality bits of the two cells sit at bits p and p+16 of a word, and
-//    hi32(bits * ((match-mismatch) << (32-p))) + (mismatch-(go+ge)) in both
-//    halves is exact while (match-mismatch) << (32-p) fits 32 bits (p >= 8
-//    here; the host requires match-mismatch <= 255);
-//  - the -(go+ge) subtract, the key H*128 + tag, the two-bit shifts that
-//    slide the reference window and the previous row's equality bits, and
-//    the one-bit shift of the equality test are multiply-adds or mad.hi.
-// Sequences are read as 16-base (32-bit) words, reloaded every 16 rows; the
-// reference word entering the window and the query word are consumed two
-// bits per row by multiplication.
+// What bounds it: instructions.  Issue saturates near 0.65 per cycle and scheduler,
+// however the work is split between the integer ALU pipe (the DPX maxima, logic) and the
+// FMA pipe (multiply-adds, fp16), each two cycles per instruction; so the step is built
+// for few of them, 5.5 per register and 0.5 for its substitution term, and both pipes
+// are kept near 65%:
+//  - the substitution terms of four registers (eight cells) are one 16-byte load from a
+//    table in shared memory, its row picked by one byte permutation from the word that
+//    interleaves the equality bits of both rows (a logic op and a 32-bit high product per
+//    register before);
+//  - all values lie in [0, 1021], where the bits of the fp16 number n * 2^-24 are the
+//    integer n: additions may run as fp16 on the FMA pipe, and one fp16 multiply-add with
+//    relu subtracts |go+ge| and takes max(.., 0).  Even registers use it and leave two
+//    DPX maxima; odd ones use three DPX maxima, the floor among them, and one addition.
+//    (All registers the one way 2.04 ms, the other 2.05, in turn 1.95.)
+//  - cells outside the matrix need no masks of their own: their equality bits are off, and
+//    then they change nothing (see sw_split.cu; the host's conditions are the same).
+// Multipliers are kernel arguments so that the compiler cannot turn the multiply-adds
+// into shifts.  256 threads per block, two blocks per SM: the table takes 64 KB a block
+// (192 x 3 and 320 x 2 threads: 2.12, 2.11 ms).
+// 1,000,000 reads of 150 bp, band 32: 2.51 -> 1.79 ms (band 16 with results to pageable
+// memory: 1.61 -> 1.28); instructions per row of band 32: 361 -> 275.
+// Sequences are read as 16-base (32-bit) words, reloaded every 16 rows; the query word is
+// consumed two bits per row by multiplication.
 // ---------------------------------------------------------------------------
-// Constants of sw_pack16_kernel, built by the host from SwParams.  The
-// multipliers (1, 4, 128, 256, 2^31 and the shifted score difference) are
-// kernel arguments rather than literals so that the multiply-adds using them
-// stay multiply-adds.
+// Constants of sw_pack16_kernel, built by the host from SwParams.
 struct Pack16Consts {
-    uint32_t one, x4, x128, x256, half;
-    uint32_t dm[4];  // (match - mismatch) << 18, 20, 22, 24
-    uint32_t mmg2;   // mismatch - (go+ge) in both halves
-    uint32_t neg_g2; // minus -(go+ge) in both halves, mod 2^32
-    uint32_t ge2;    // ge in both halves
-    uint32_t ng2;    // -(go+ge) in both halves
+    uint32_t x4, x8, x128, half;
+    uint32_t dm_pad;   // (match - mismatch) * 4
+    uint32_t dm;       // match - mismatch
+    uint32_t mmg2;     // mismatch - (go+ge) in both halves
+    uint32_t ge2;      // ge in both halves
+    uint32_t ng2;      // -(go+ge) in both halves
+    uint32_t one_f;    // 1.0 in both halves
+    uint32_t neg_g_f;  // -|go+ge| * 2^-24 in both halves
 };
+
+// Halves as fp16 numbers n * 2^-24, whose bits are the integer n for 0 <= n <= 2047.
+__device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// max(a * b + c, 0)
+__device__ __forceinline__ uint32_t fma_relu_f16x2(uint32_t a, uint32_t b, uint32_t c)
+{
+    uint32_t d;
+    asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
 
 __device__ __forceinline__ uint32_t mad_hi_u32(uint32_t a, uint32_t b, uint32_t c)
 {
     uint32_t d;
     asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
-}
-
-// (a << 2) | (b >> 30) as two multiply-adds (x4 == 4).
-__device__ __forceinline__ uint32_t shl2_in(uint32_t a, uint32_t b, uint32_t x4)
-{
-    return a * x4 + mad_hi_u32(b, x4, 0u);
 }
 
 // 16-base word k (bases 16k..16k+15, first base in the top two bits) of the
@@ -318,16 +332,15 @@ __device__ __forceinline__ uint32_t seq_word16(const SeqView &s, int64_t off, in
     return __ldg(reinterpret_cast<const uint32_t *>(s.packed) + i);
 }
 
-// One step of sw_pack16_kernel over all R registers.  eq[k] / bw[k]: the
-// equality bits (bit 30-2c for column 16k+c) of row t and of row t-1 shifted
-// so column B+1+h sits where column h does.  MASK = false when every cell of
-// the step lies inside the matrix (the common case); MASK = true zeroes the
-// first-maximum keys of cells past the query or reference end.  Returns the
-// packed row keys: low half row t, high half row t-1.
-template <int B, bool MASK>
-__device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const uint32_t *eq,
-                                                 const uint32_t *bw, uint32_t &e_last, int limL,
-                                                 int limH, const Pack16Consts &c)
+// One step of sw_pack16_kernel over all R registers.  cw[k]: the equality bits of
+// columns 16k .. 16k+15 of row t (column 16k+c at bit 30-2c) with those of row t-1,
+// columns B+1+16k .., one bit above them; e_pad: row t's word that starts at column B.
+// tab, l16: the score table and the lane's place in its rows.  Returns the packed row
+// keys: low half row t, high half row t-1.
+template <int B>
+__device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const uint32_t *cw,
+                                                 uint32_t e_pad, const char *tab, uint32_t l16,
+                                                 uint32_t &e_last, const Pack16Consts &c)
 {
     constexpr int NL = B + 1, R = NL;
     const uint32_t SENT = 0x0000C000u;
@@ -335,20 +348,29 @@ __device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const ui
     uint32_t el = __byte_perm(SENT, e_last, 0x5410);  // low: chain start; high: E'(t-1, B)
     uint32_t h0new = 0;
     uint32_t rk = 0, kpend = 0;
+    uint32_t sub[4];
 #pragma unroll
     for (int h = 0; h < R; ++h) {
-        const int k = h >> 4, j = h & 15, jj = h & 7;
-        // cells 8*(h>>3) .. +7 of both halves at bits 14-2*jj and 30-2*jj
-        const uint32_t wsel = (j < 8) ? __byte_perm(eq[k], bw[k], 0x7632)
-                                      : __byte_perm(eq[k], bw[k], 0x5410);
-        const uint32_t wv = (jj < 4) ? wsel : wsel * c.x256;  // cells 4..7 up to bits 14..8
-        const int pos = 14 - 2 * (jj & 3);
-        const uint32_t sub =
-            mad_hi_u32(wv & ((1u << pos) | (1u << (pos + 16))), c.dm[jj & 3], c.mmg2);
+        if (h == R - 1) {
+            sub[0] = mad_hi_u32(e_pad & 0x40000000u, c.dm_pad, c.mmg2);
+        } else if ((h & 3) == 0) {  // row of the table: the byte of these four columns
+            const uint32_t at = __byte_perm(cw[h >> 4], l16, 0x7704 | ((3 - ((h >> 2) & 3)) << 4));
+            const uint4 v = *reinterpret_cast<const uint4 *>(tab + at);
+            sub[0] = v.x;
+            sub[1] = v.y;
+            sub[2] = v.z;
+            sub[3] = v.w;
+        }
         const uint32_t up = (h + 1 < R) ? Hr[h + 1 < R ? h + 1 : h] : (h0new >> 16);
         const uint32_t e = __viaddmax_s16x2(el, c.ge2, up);
-        const uint32_t tt = __vimax3_s16x2(e, hl, c.ng2);
-        uint32_t hn = __viaddmax_s16x2(Hr[h], sub, tt) * c.one + c.neg_g2;
+        uint32_t hn;
+        if (h & 1) {
+            const uint32_t tt = __vimax3_s16x2(e, hl, c.ng2);
+            hn = add_f16x2(__viaddmax_s16x2(Hr[h], sub[h & 3], tt), c.neg_g_f);
+        } else {
+            const uint32_t tt = __vimax3_s16x2(add_f16x2(Hr[h], sub[h & 3]), e, hl);
+            hn = fma_relu_f16x2(tt, c.one_f, c.neg_g_f);
+        }
         hl = hn;
         if (h == R - 1)
             hn &= 0x0000FFFFu;  // padding column stays 0
@@ -356,9 +378,8 @@ __device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const ui
             h0new = hn;
         Hr[h] = hn;
         el = e;
-        uint32_t key = hn * c.x128 + (((uint32_t)(127 - h)) | ((uint32_t)(127 - NL - h) << 16));
-        if (MASK)
-            key &= (h < limL ? 0x0000FFFFu : 0u) | (h < limH ? 0xFFFF0000u : 0u);
+        const uint32_t key =
+            hn * c.x128 + (((uint32_t)(127 - h)) | ((uint32_t)(127 - NL - h) << 16));
         if (h & 1)
             rk = __vimax3_u16x2(rk, kpend, key);
         else
@@ -370,8 +391,19 @@ __device__ __forceinline__ uint32_t pack16_cells(uint32_t (&Hr)[B + 1], const ui
     return rk;
 }
 
+// Fields [lo, hi) of 16-column equality word i (column 16i + f at bit 30-2f).
+__device__ __forceinline__ uint32_t eq_fields(int32_t lo, int32_t hi, int i)
+{
+    const uint32_t a = (uint32_t)min(max(lo - 16 * i, 0), 16) * 2;
+    const uint32_t b = (uint32_t)min(max(hi - 16 * i, 0), 16) * 2;
+    return __funnelshift_rc(0x55555555u, 0u, a) & ~__funnelshift_rc(0xFFFFFFFFu, 0u, b);
+}
+
+constexpr int kPackThreads = 256;
+constexpr int kPackTableBytes = 256 * 256;
+
 template <int B>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kPackThreads, 2)
 sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_result *__restrict__ out)
 {
     static_assert(B % 16 == 0, "band must be a multiple of 16");
@@ -394,6 +426,20 @@ sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_resul
     const int64_t warps_total = (int64_t)gridDim.x * warps_per_block;
     const uint32_t SENT = 0x0000C000u;  // -16384 in the low half
 
+    // Score table: row i, 256 bytes, holds the substitution terms of four registers whose
+    // equality bits are the bit pairs of i (first register on top; even bit low half, odd
+    // bit high half), sixteen times over: the lanes of a 16-byte access phase share no bank.
+    extern __shared__ uint4 tab[];
+    for (int i = threadIdx.x; i < kPackTableBytes / 16; i += kPackThreads) {
+        const uint32_t x = (uint32_t)i >> 4;
+        auto term = [&](int s) {
+            return c.mmg2 + ((x >> s) & 1) * c.dm + (((x >> s) & 2) << 15) * c.dm;
+        };
+        tab[i] = make_uint4(term(6), term(4), term(2), term(0));
+    }
+    __syncthreads();
+    const uint32_t l16 = (uint32_t)(lane & 15) * 16;
+
     int64_t base = warp_global * 32;
     for (;;) {
         if (queue_counter) {
@@ -404,101 +450,98 @@ sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_resul
         }
         if (base >= n)
             break;
-        const int64_t slot = base + lane;
-        if (slot < n) {
-            const int64_t pi = queue ? (int64_t)queue[slot] : slot;
-            const int64_t qoff = q.offsets[pi] - q.word_base;
-            const int64_t roff = r.offsets[pi] - r.word_base;
-            const int32_t qlen = (int32_t)q.lengths[pi], rlen = (int32_t)r.lengths[pi];
-            uint32_t Hr[R];
+        const bool valid = base + lane < n;
+        const int64_t slot = valid ? base + lane : base;
+        const int64_t pi = queue ? (int64_t)queue[slot] : slot;
+        const int64_t qoff = q.offsets[pi] - q.word_base;
+        const int64_t roff = r.offsets[pi] - r.word_base;
+        const int32_t qlen = (int32_t)q.lengths[pi], rlen = (int32_t)r.lengths[pi];
+        uint32_t Hr[R];
 #pragma unroll
-            for (int h = 0; h < R; ++h)
-                Hr[h] = 0;
-            uint32_t ep[NE];  // equality bits of the previous row
+        for (int h = 0; h < R; ++h)
+            Hr[h] = 0;
+        // The reference window of row t, r[t-B .. t-B+16*NE), one 16-base word
+        // per entry, slid by one base per row; the base entering at the bottom
+        // is the top of `rw`, the word of positions t-B+16*NE.., reloaded every
+        // 16 rows (t-B+16*NE is a multiple of 16 exactly when t is).  Words
+        // before the reference start are zero and masked below.
+        // em: the columns of row t inside the matrix; ep, eo: equality bits of two rows.
+        uint32_t win[NE], em[NE], ep[NE], eo[NE];
 #pragma unroll
-            for (int i = 0; i < NE; ++i)
-                ep[i] = 0;
-            // The reference window of row t, r[t-B .. t-B+16*NE), one 16-base word
-            // per entry, slid by one base per row; the base entering at the bottom
-            // is the top of `rw`, the word of positions t-B+16*NE.., reloaded every
-            // 16 rows (t-B+16*NE is a multiple of 16 exactly when t is).  Words
-            // before the reference start are zero and masked below.
-            uint32_t win[NE];
+        for (int i = 0; i < NE; ++i) {
+            win[i] = (i < B / 16) ? 0u : seq_word16(r, roff, i - B / 16);
+            em[i] = eq_fields(B + 1, max(B + 1, rlen + B + 1), i);
+            ep[i] = 0;
+        }
+        uint32_t e_last = SENT;
+        uint32_t saved_lowkey = 0, bestkey = 0, thr = 127;
+        int32_t bq = 0;
+        uint32_t qw = 0, rw = 0;
+        uint32_t qn = seq_word16(q, qoff, 0), rn = seq_word16(r, roff, RW0);  // next words
+        // rows [B+1, B+1+inner) have all their columns inside, and rows [0, tail) none
+        // past the reference end
+        const int32_t tail = min(qlen, rlen - B);
+        const uint32_t inner = (uint32_t)max(tail - (B + 1), 0);
+        const int32_t steps = __reduce_max_sync(0xffffffffu, qlen > 0 ? qlen + 1 : 0);
+        auto one_row = [&](int32_t t, uint32_t(&eq)[NE], const uint32_t(&ep)[NE]) {
+            if ((uint32_t)(t - (B + 1)) >= inner) {
+                if (t < tail) {  // the start of the reference: a column more than at t-1
 #pragma unroll
-            for (int i = 0; i < NE; ++i)
-                win[i] = (i < B / 16) ? 0u : seq_word16(r, roff, i - B / 16);
-            uint32_t e_last = SENT;
-            uint32_t saved_lowkey = 0, bestkey = 0, thr = 127;
-            int32_t bq = 0;
-            uint32_t qw = 0, rw = 0;
-            uint32_t qn = seq_word16(q, qoff, 0), rn = seq_word16(r, roff, RW0);  // next words
-            const int steps = qlen > 0 ? qlen + 1 : 0;
-            const int full_end = min(qlen, rlen - B + 1);  // rows t < full_end lie inside
-            for (int t = 0; t < steps; ++t) {
-                if ((t & 15) == 0) {  // words of rows t..t+15; fetch the following ones
-                    qw = qn;
-                    rw = rn;
-                    qn = seq_word16(q, qoff, (t >> 4) + 1);
-                    rn = seq_word16(r, roff, (t >> 4) + RW0 + 1);
+                    for (int i = 0; i < NE; ++i)
+                        em[i] = __funnelshift_l(i + 1 < NE ? em[i + 1 < NE ? i + 1 : i] : 0x55555555u,
+                                                em[i], 2);
+                } else {
+                    const int32_t lo = max(B - t, 0), hi = t < qlen ? rlen - t + B : 0;
+#pragma unroll
+                    for (int i = 0; i < NE; ++i)
+                        em[i] = eq_fields(lo, max(hi, lo), i);
                 }
-                // equality bits of row t against its window r[t-B .. t+B]
-                const uint32_t qrep = mad_hi_u32(qw, c.x4, 0u) * 0x55555555u;
-                qw *= c.x4;
-                uint32_t eq[NE];
-#pragma unroll
-                for (int i = 0; i < NE; ++i) {
-                    const uint32_t x = win[i] ^ qrep;
-                    eq[i] = ~(x | mad_hi_u32(x, c.half, 0u)) & 0x55555555u;
-                }
-                if (t < B) {  // columns before the reference start never match
-#pragma unroll
-                    for (int i = 0; i < NE; ++i) {
-                        const int cnt = B - t - 16 * i;
-                        if (cnt >= 16)
-                            eq[i] = 0;
-                        else if (cnt > 0)
-                            eq[i] &= 0xFFFFFFFFu >> (2 * cnt);
-                    }
-                }
-                // slide the window one base for row t+1
-#pragma unroll
-                for (int i = 0; i + 1 < NE; ++i)
-                    win[i] = shl2_in(win[i], win[i + 1], c.x4);
-                win[NE - 1] = shl2_in(win[NE - 1], rw, c.x4);
-                rw *= c.x4;
-                // previous row's bits, shifted so column NL+h sits where column h does;
-                // the last word holds only the padding column
-                uint32_t bw[NBW + 1];
-#pragma unroll
-                for (int i = 0; i < NBW; ++i)
-                    bw[i] = shl2_in(ep[BW0 + i], ep[BW0 + i + 1], c.x4);
-                bw[NBW] = 0;
-                const bool full = t >= 1 && t < full_end;
-                int limL = 0, limH = 0;
-                if (!full) {
-                    if (t < qlen)
-                        limL = max(0, min(NL, rlen - (t - B)));
-                    if (t >= 1 && t - 1 < qlen)
-                        limH = max(0, min(R, rlen - (t - 1 - B + NL)));
-                }
-                const uint32_t rk =
-                    full ? pack16_cells<B, false>(Hr, eq, bw, e_last, 0, 0, c)
-                         : pack16_cells<B, true>(Hr, eq, bw, e_last, limL, limH, c);
-                // row t-1 is complete: its first half came one step earlier; a key
-                // above thr = bestkey | 127 has a larger H than the best so far
-                const uint32_t rowkey = max(saved_lowkey, rk >> 16);
-                if (rowkey > thr) {
-                    thr = rowkey | 127u;
-                    bestkey = rowkey;
-                    bq = t - 1;
-                }
-                saved_lowkey = rk & 0xFFFFu;
-#pragma unroll
-                for (int i = 0; i < NE; ++i)
-                    ep[i] = eq[i];
             }
-            const int32_t best = (int32_t)(bestkey >> 7);
-            const int32_t bcol = 127 - (int32_t)(bestkey & 127u);
+            // equality bits of row t against its window r[t-B .. t+B]
+            const uint32_t qrep = mad_hi_u32(qw, c.x4, 0u) * 0x55555555u;
+            qw *= c.x4;
+#pragma unroll
+            for (int i = 0; i < NE; ++i) {
+                const uint32_t x = win[i] ^ qrep;
+                eq[i] = ~(x | mad_hi_u32(x, c.half, 0u)) & em[i];
+            }
+            // slide the window one base for row t+1
+#pragma unroll
+            for (int i = 0; i < NE; ++i)
+                win[i] = __funnelshift_l(i + 1 < NE ? win[i + 1 < NE ? i + 1 : i] : rw, win[i], 2);
+            rw *= c.x4;
+            // both rows' bits: the previous row's shifted so column NL+h sits one
+            // bit above column h
+            uint32_t cw[NBW];
+#pragma unroll
+            for (int i = 0; i < NBW; ++i)
+                cw[i] = ep[BW0 + i] * c.x8 + mad_hi_u32(ep[BW0 + i + 1], c.x8, eq[i]);
+            const uint32_t rk =
+                pack16_cells<B>(Hr, cw, eq[NBW], (const char *)tab, l16, e_last, c);
+            // row t-1 is complete: its first half came one step earlier; a key
+            // above thr = bestkey | 127 has a larger H than the best so far
+            const uint32_t rowkey = max(saved_lowkey, rk >> 16);
+            if (rowkey > thr) {
+                bestkey = rowkey;
+                bq = t - 1;
+            }
+            thr = max(thr, rowkey | 127u);
+            saved_lowkey = rk & 0xFFFFu;
+        };
+        for (int32_t t0 = 0; t0 < steps; t0 += 16) {
+            qw = qn;  // words of rows t0 .. t0+15; fetch the following ones
+            rw = rn;
+            qn = seq_word16(q, qoff, (t0 >> 4) + 1);
+            rn = seq_word16(r, roff, (t0 >> 4) + RW0 + 1);
+            const int32_t t1 = min(t0 + 16, steps);
+            for (int32_t t = t0; t < t1; t += 2) {  // an odd count runs one empty row more
+                one_row(t, eo, ep);
+                one_row(t + 1, ep, eo);
+            }
+        }
+        const int32_t best = (int32_t)(bestkey >> 7);
+        const int32_t bcol = 127 - (int32_t)(bestkey & 127u);
+        if (valid) {
             gb2_sw_result res;
             res.score = best;
             res.query_end = best > 0 ? bq : 0;
@@ -699,10 +742,20 @@ static int occ_band()
 }
 
 template <int B>
+static cudaError_t pack16_smem()
+{
+    static std::atomic<uint64_t> done{0};
+    return allow_smem(sw_pack16_kernel<B>, kPackTableBytes, done);
+}
+
+template <int B>
 static int occ_pack16()
 {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sw_pack16_kernel<B>, 128, 0);
+    if (pack16_smem<B>() != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sw_pack16_kernel<B>, kPackThreads,
+                                                      kPackTableBytes) != cudaSuccess)
+        cudaGetLastError();
     return nb > 0 ? nb : 1;
 }
 
@@ -726,7 +779,7 @@ int sw_pairs_per_block(int band_class, int variant)
     int G = 1;
     switch (band_class) {
     case 16 | kPack16:
-    case 32 | kPack16: return 128;
+    case 32 | kPack16: return kPackThreads;
     case 16: G = variant == 1 ? 2 : 1; break;
     case 32: G = variant == 1 ? 2 : (variant == 2 ? 4 : 1); break;
     case 64: G = variant == 1 ? 4 : 2; break;
@@ -738,8 +791,8 @@ int sw_pairs_per_block(int band_class, int variant)
 
 double sw_pack16_cost(int band, const SplitLoad &l)
 {
-    // 573 cycles per warp and row at band 32 (1,000,000 reads)
-    return split_time(17.4 * (band + 1), 24.5 * (band + 1) + 190,
+    // 425 cycles per warp and row at band 32 (1,000,000 reads)
+    return split_time(12.9 * (band + 1), 24.5 * (band + 1) + 190,
                       (double)l.pairs / 32 / (4.0 * l.sm_count), l);
 }
 
@@ -755,25 +808,32 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
         if (g <= 0) {
             if (pl.seg || pl.n <= 0)
                 return pl.n <= 0 && !pl.seg ? cudaSuccess : cudaErrorInvalidValue;
-            g = (int)((pl.n + 127) / 128);
+            g = (int)((pl.n + kPackThreads - 1) / kPackThreads);
         }
         const uint32_t gg = (uint32_t)(-(p.go + p.ge)), dm = (uint32_t)(p.match - p.mismatch);
         Pack16Consts c;
-        c.one = 1;
         c.x4 = 4;
+        c.x8 = 8;
         c.x128 = 128;
-        c.x256 = 256;
         c.half = 0x80000000u;
-        for (int i = 0; i < 4; ++i)
-            c.dm[i] = dm << (18 + 2 * i);
+        c.dm_pad = dm * 4;
+        c.dm = dm;
         c.mmg2 = ((uint32_t)p.mismatch + gg) * 0x00010001u;
-        c.neg_g2 = 0u - gg * 0x00010001u;
         c.ge2 = (uint32_t)(uint16_t)p.ge * 0x00010001u;
-        c.ng2 = (uint32_t)(uint16_t)gg * 0x00010001u;
-        if (band_class == (16 | kPack16))
-            sw_pack16_kernel<16><<<g, 128, 0, st>>>(q, r, c, pl, out);
+        c.ng2 = gg * 0x00010001u;
+        c.one_f = 0x3C003C00u;
+        c.neg_g_f = (0x8000u | gg) * 0x00010001u;
+        const auto go = [&](auto kern) {
+            kern<<<g, kPackThreads, kPackTableBytes, st>>>(q, r, c, pl, out);
+        };
+        const bool b16 = band_class == (16 | kPack16);
+        const cudaError_t e = b16 ? pack16_smem<16>() : pack16_smem<32>();
+        if (e != cudaSuccess)
+            return e;
+        if (b16)
+            go(sw_pack16_kernel<16>);
         else
-            sw_pack16_kernel<32><<<g, 128, 0, st>>>(q, r, c, pl, out);
+            go(sw_pack16_kernel<32>);
         return cudaGetLastError();
     }
     case 16:
