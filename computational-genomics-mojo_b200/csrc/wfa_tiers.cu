@@ -1313,9 +1313,9 @@ bool wfa_short_usable(const WfaTierPlan &pl) { return short_geom(pl.nslot).W >= 
 cudaError_t launch_wfa_short(const WfaTierPlan &pl, int sm_count, SeqView q, SeqView r, WfaParams p,
                              const WfaTierIo &io, int32_t *out, int64_t *work, cudaStream_t st)
 {
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        wfa_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        16 * kShortPairBytes + kSeqSlack);
+    static std::atomic<uint64_t> smem_set{0};
+    const cudaError_t attr =
+        allow_smem(wfa_short_kernel, 16 * kShortPairBytes + kSeqSlack, smem_set);
     if (attr != cudaSuccess)
         return attr;
     TierIn in{};
@@ -1335,12 +1335,11 @@ static cudaError_t tier_launch(const WfaTierPlan &pl, int t, int grid, SeqView q
                                int32_t *out, int64_t *work, int *err_flag, cudaStream_t st)
 {
     const size_t smem = (size_t)pl.team_bytes[t] * NTEAMS + kSeqSlack;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(wfa_tier_kernel<TEAM, NTEAMS, RT, GRING>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTierBlockSmem + kSeqSlack);
-        attr = true;
-    }
+    static std::atomic<uint64_t> smem_set{0};
+    const cudaError_t attr = allow_smem(wfa_tier_kernel<TEAM, NTEAMS, RT, GRING>,
+                                        (int)kTierBlockSmem + kSeqSlack, smem_set);
+    if (attr != cudaSuccess)
+        return attr;
     TierGeom geo{pl.W[t], pl.H[t], pl.team_bytes[t], pl.ring_bytes[t], pl.seq_cap[t], gring};
     wfa_tier_kernel<TEAM, NTEAMS, RT, GRING><<<grid, TEAM * NTEAMS * 32, smem, st>>>(
         q, r, p, in, o, geo, out, work, err_flag);
