@@ -464,10 +464,7 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
             w.low[0] = low;
             w.high[0] = long_scores ? high : -1;
             w.list[0] = PairList{nullptr, n, nullptr, (int *)x.counters.p};
-            const int64_t per = 4 * (32 >> ch.lg);
-            const int grid = (int)std::min<int64_t>(
-                (n + per - 1) / per,
-                (int64_t)c->sm_count * split_blocks_per_sm(false, ch.shape));
+            const int grid = split_grid(false, ch.shape, ch.lg, n, c->sm_count);
             cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
             CU(c, launch_split(false, ch.shape, qv, rv, p, cfg->band_width, nullptr, w, d_out,
                                grid, x.st));
@@ -487,10 +484,15 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
             pl.counter = (int *)x.counters.p;
             // no more blocks than pairs need: in a batch smaller than one wave the warps of
             // the SMs that start first would otherwise take every pair (50,000 reads,
-            // band 32: 281 -> 193 us)
+            // band 32: 281 -> 193 us).  The packed kernel's warps then go by
+            // their place in the grid (40,000 reads, band 32: 134 -> 111 us).
             const int64_t per = sw_pairs_per_block(cls, var_of(cls));
-            grid = (int)std::min<int64_t>((int64_t)c->sm_count * sw_blocks_per_sm(cls, var_of(cls)),
-                                          (n + per - 1) / per);
+            const int64_t blocks = (int64_t)c->sm_count * sw_blocks_per_sm(cls, var_of(cls));
+            grid = (int)std::min(blocks, (n + per - 1) / per);
+            if ((cls & kPack16) && n <= blocks * per) {
+                pl.counter = nullptr;
+                grid = (int)std::min(blocks, (n + 31) / 32);
+            }
         }
         cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
         if (cls > 0) {
@@ -618,9 +620,8 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
             continue;
         if ((rc = next_stream(s)))
             return rc;
-        const int64_t per = 4 * (32 >> w.lg[0]);  // pairs of a block with the most lanes
-        const int grid = (int)std::min<int64_t>(
-            (n + per - 1) / per, (int64_t)c->sm_count * split_blocks_per_sm(false, shape));
+        // for the segment with the most lanes per pair
+        const int grid = split_grid(false, shape, w.lg[0], n, c->sm_count);
         CU(c, launch_split(false, shape, qv, rv, p, cfg->band_width, d_bands, w, d_out, grid, s));
         if ((rc = launched(s)))
             return rc;

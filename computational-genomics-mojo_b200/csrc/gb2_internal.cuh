@@ -84,6 +84,32 @@ cudaError_t allow_smem(K *kernel, int bytes, std::atomic<uint64_t> &done)
     return e;
 }
 
+// A warp's place in the grid, blocks in turn: fewer warps than the GPU holds spread over
+// all SMs.
+__device__ __forceinline__ int64_t warp_rank()
+{
+    return (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+}
+
+// Score table of the packed band kernels, in shared memory: row i, 256 bytes, holds the
+// substitution terms of four registers whose equality bits are the bit pairs of i (first
+// register on top; even bit low half, odd bit high half), sixteen times over, so that the
+// lanes of a 16-byte access phase share no bank.  base2: the terms of two unequal cells;
+// dm: what an equal one adds.
+constexpr int kScoreTableBytes = 256 * 256;
+
+__device__ __forceinline__ void score_table_fill(uint4 *tab, uint32_t base2, uint32_t dm,
+                                                 int threads)
+{
+    for (int i = threadIdx.x; i < kScoreTableBytes / 16; i += threads) {
+        const uint32_t x = (uint32_t)i >> 4;
+        auto term = [&](int s) {
+            return base2 + ((x >> s) & 1) * dm + (((x >> s) & 2) << 15) * dm;
+        };
+        tab[i] = make_uint4(term(6), term(4), term(2), term(0));
+    }
+}
+
 // band_class flag selecting the packed int16x2 kernel of one thread per pair (bands 16
 // and 32, scores up to kPackHmax).
 constexpr int kPack16 = 0x100;
@@ -127,13 +153,15 @@ inline SplitLoad split_load(const SeqView &q, int64_t qmax, int64_t n, int sm_co
 }
 // Estimated cycles of a batch whose warps issue for `issue` cycles per row, or whose
 // longest pair takes `chain` cycles per row; warps per scheduler.
-double split_time(double issue, double chain, double warps, const SplitLoad &l);
+double split_time(double issue, double chain, double warps, double rows, const SplitLoad &l);
 // The shape and lane count for pairs of one band; long_scores: Smith-Waterman scores may
 // pass kSplitHmax.  only_shape >= 0: that shape's lane count, or none.
 SplitChoice split_choose(const SwParams &p, int32_t band, const SplitLoad &l, bool nw,
                          bool long_scores, int only_shape = -1);
 int split_regs(int shape);
 int split_blocks_per_sm(bool nw, int shape);
+// Blocks for n pairs of 2^lg lanes each.
+int split_grid(bool nw, int shape, int lg, int64_t n, int sm_count);
 // Whether pairs whose scores pass kSplitHmax may run: the range [low, high] the
 // pair's largest value is kept in (see the file's header) is wide enough.
 bool split_rebase(const SwParams &p, int shape, int lg, int32_t *low, int32_t *high);

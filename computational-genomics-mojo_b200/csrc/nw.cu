@@ -278,8 +278,7 @@ static int nw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, const SwParams &
             GB2_CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
             w.list[0] = PairList{nullptr, n, nullptr, (int *)x.counters.p};
         }
-        const int grid = (int)std::min<int64_t>(
-            (n + per - 1) / per, (int64_t)c->sm_count * split_blocks_per_sm(true, shape));
+        const int grid = split_grid(true, shape, lg, n, c->sm_count);
         GB2_CU(c, launch_split(true, shape, qv, rv, p, band, d_bands, w, d_out, grid, x.st));
         c->launches += 1;
         return GB2_OK;

@@ -400,7 +400,6 @@ __device__ __forceinline__ uint32_t eq_fields(int32_t lo, int32_t hi, int i)
 }
 
 constexpr int kPackThreads = 256;
-constexpr int kPackTableBytes = 256 * 256;
 
 template <int B>
 __global__ void __launch_bounds__(kPackThreads, 2)
@@ -421,22 +420,12 @@ sw_pack16_kernel(SeqView q, SeqView r, Pack16Consts c, PairList pl, gb2_sw_resul
     const int32_t *__restrict__ queue = pairs_resolve(pl, n);
     int *const queue_counter = pl.counter;
     const int lane = threadIdx.x & 31;
-    const int warps_per_block = blockDim.x >> 5;
-    const int64_t warp_global = (int64_t)blockIdx.x * warps_per_block + (threadIdx.x >> 5);
-    const int64_t warps_total = (int64_t)gridDim.x * warps_per_block;
+    const int64_t warp_global = warp_rank();
+    const int64_t warps_total = (int64_t)gridDim.x * (kPackThreads / 32);
     const uint32_t SENT = 0x0000C000u;  // -16384 in the low half
 
-    // Score table: row i, 256 bytes, holds the substitution terms of four registers whose
-    // equality bits are the bit pairs of i (first register on top; even bit low half, odd
-    // bit high half), sixteen times over: the lanes of a 16-byte access phase share no bank.
     extern __shared__ uint4 tab[];
-    for (int i = threadIdx.x; i < kPackTableBytes / 16; i += kPackThreads) {
-        const uint32_t x = (uint32_t)i >> 4;
-        auto term = [&](int s) {
-            return c.mmg2 + ((x >> s) & 1) * c.dm + (((x >> s) & 2) << 15) * c.dm;
-        };
-        tab[i] = make_uint4(term(6), term(4), term(2), term(0));
-    }
+    score_table_fill(tab, c.mmg2, c.dm, kPackThreads);
     __syncthreads();
     const uint32_t l16 = (uint32_t)(lane & 15) * 16;
 
@@ -745,7 +734,7 @@ template <int B>
 static cudaError_t pack16_smem()
 {
     static std::atomic<uint64_t> done{0};
-    return allow_smem(sw_pack16_kernel<B>, kPackTableBytes, done);
+    return allow_smem(sw_pack16_kernel<B>, kScoreTableBytes, done);
 }
 
 template <int B>
@@ -754,7 +743,7 @@ static int occ_pack16()
     int nb = 0;
     if (pack16_smem<B>() != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sw_pack16_kernel<B>, kPackThreads,
-                                                      kPackTableBytes) != cudaSuccess)
+                                                      kScoreTableBytes) != cudaSuccess)
         cudaGetLastError();
     return nb > 0 ? nb : 1;
 }
@@ -792,8 +781,8 @@ int sw_pairs_per_block(int band_class, int variant)
 double sw_pack16_cost(int band, const SplitLoad &l)
 {
     // 425 cycles per warp and row at band 32 (1,000,000 reads)
-    return split_time(12.9 * (band + 1), 24.5 * (band + 1) + 190,
-                      (double)l.pairs / 32 / (4.0 * l.sm_count), l);
+    return split_time(12.9 * (band + 1), 24.5 * (band + 1) + 200,
+                      (double)l.pairs / 32 / (4.0 * l.sm_count), 1, l);
 }
 
 // variant selects (G, K) for a band class: 0 = default.
@@ -824,7 +813,7 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
         c.one_f = 0x3C003C00u;
         c.neg_g_f = (0x8000u | gg) * 0x00010001u;
         const auto go = [&](auto kern) {
-            kern<<<g, kPackThreads, kPackTableBytes, st>>>(q, r, c, pl, out);
+            kern<<<g, kPackThreads, kScoreTableBytes, st>>>(q, r, c, pl, out);
         };
         const bool b16 = band_class == (16 | kPack16);
         const cudaError_t e = b16 ? pack16_smem<16>() : pack16_smem<32>();

@@ -51,23 +51,27 @@
 // left moves then add nothing: two DPX instructions per two cells), re-centred
 // every 16 steps; the host checks that the values fit.
 //
-// Bound: the ALU and the FMA-heavy pipe, two cycles per warp instruction each: per
-// register of two cells 4.5 ALU instructions (three DPX, a logic op, half a 3-way
-// maximum) and three multiply-adds, of which the mad.hi takes two slots; at R = 33
-// about 400 instructions per row of 66 columns issue in 652 cycles.  Short chains
-// (one warp per scheduler) take 24.5 R + 190 cycles per row.
+// What bounds it: instructions, which issue at about 0.65 per cycle and scheduler (see
+// sw_kernels.cu), 5.5 per register of two cells and 0.5 for its substitution term, one
+// 16-byte load of the score table per four registers (NW: 2 and 0.5); at R = 33 a row of
+// 66 columns takes 500 cycles.  Short batches are bound by the chain from register to
+// register: one warp per scheduler takes 19 R + 150 cycles per row.  256 threads a block,
+// two blocks per SM: each block's table takes 64 KB.  (With 16-bit sums kept off the chain,
+// max(H_diag + sub, E', H_left) - g, the chain is 15 R + 207 but full batches take 5-9%
+// longer: the mixed bands below 1.50 against 1.38 ms.)
 // Measured (ms, before: the register kernels of one thread per pair or 2-8 lanes in
-// int32, and for other bands the literal kernel with int64 rows in memory):
-//   Smith-Waterman, 100,000 pairs of 100-300 bp, band 40       57.9 -> 0.68
-//   50,000 pairs of 100-2,000 bp, bands 16/32/64/128 per pair  5.66 -> 1.73
-//   4,000 pairs of 2-10 kbp, band 128                          13.5 -> 2.84
-//   500,000 reads of 150 bp, band 128 / 64                     7.25 -> 5.91 / 2.80 -> 2.82
-//   Needleman-Wunsch, 20,000 pairs of 100-1,000 bp, band 64    46.7 -> 0.50
-//   500,000 reads, band 32                                     2.44 -> 1.89
+// int32, and for other bands the literal kernel with int64 rows in memory; then this
+// kernel with a logic op and a high product per register in place of the table):
+//   Smith-Waterman, 100,000 pairs of 100-300 bp, band 40       57.9 -> 0.67 -> 0.57
+//   50,000 pairs of 100-2,000 bp, bands 16/32/64/128 per pair  5.66 -> 1.73 -> 1.22
+//   4,000 pairs of 2-10 kbp, band 128                          13.5 -> 2.84 -> 2.56
+//   Needleman-Wunsch, 20,000 pairs of 100-1,000 bp, band 64    46.7 -> 0.46 -> 0.36
+//   500,000 reads, band 32                                     2.44 -> 1.38 -> 1.19
 // The one-thread kernel stays for short reads of bands 16 and 32 in large batches: its
-// row of 33 registers takes 573 cycles against 652 (1,000,000 reads, band 32: 2.51
-// against 2.89 ms); split_choose compares both.
+// row of 33 registers takes 425 cycles against 500 and its pairs need no start
+// (400,000 reads, band 32: 0.72 against 0.89 ms); split_choose compares both.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "gb2_internal.cuh"
@@ -80,8 +84,8 @@ constexpr int32_t kNwFloor = -31000;         // Needleman-Wunsch: cells outside 
 constexpr int32_t kNwNeg = -1000000;
 
 struct SplitConsts {
-    uint32_t x4, x8, x256, x64k, half, one;
-    uint32_t dm[4];   // (match - mismatch) << 18, 20, 22, 24
+    uint32_t x4, x8, x64k, half, one;
+    uint32_t dm;      // match - mismatch
     uint32_t sub2;    // mismatch + g (Smith-Waterman) or + 2g, both halves
     uint32_t neg_g2;  // -g in both halves, mod 2^32
     uint32_t ge2;     // ge in both halves
@@ -122,15 +126,17 @@ __device__ __forceinline__ uint32_t nw_init(int32_t j, int32_t b, int32_t go, in
     return (uint32_t)(uint16_t)(int16_t)(ri < 0 || j > 2 * b ? kNwFloor : v);
 }
 
-// One step over the lane's R registers.  eq / bw: equality bits of row t' and,
-// shifted so column R + h sits where column h does, of row t'-1.  hl / el: the
+// One step over the lane's R registers.  cw: the equality bits of row t' and, one bit
+// above them, those of row t'-1 shifted so column R + h sits where column h does; tab, l16:
+// the score table and the lane's place in its rows.  hl / el: the
 // left neighbours of register 0.  Returns the last register's H and E' through
 // hl / el, and the row keys (Smith-Waterman) through klo / khi.  START
 // (Needleman-Wunsch): halves of rows before 0 are held at the initial row, and
 // row 0's cells left of the reference start set to the floor.
 template <int R, bool NW, bool START>
-__device__ __forceinline__ void split_step(uint32_t (&Hr)[R], const uint32_t *eq,
-                                           const uint32_t *bw, uint32_t &hl, uint32_t &el,
+__device__ __forceinline__ void split_step(uint32_t (&Hr)[R], const uint32_t *cw,
+                                           const char *tab, uint32_t l16, uint32_t &hl,
+                                           uint32_t &el,
                                            int32_t &klo, int32_t &khi, int G,
                                            uint32_t last_mask, const SplitConsts &c, int32_t row,
                                            int32_t b, int32_t c0)
@@ -138,29 +144,33 @@ __device__ __forceinline__ void split_step(uint32_t (&Hr)[R], const uint32_t *eq
     constexpr int NG = (R + 7) / 8;  // key groups: register h in group h % NG, tag 7 - h / NG
     const uint32_t floor2 = (uint32_t)(uint16_t)(int16_t)kNwFloor * 0x00010001u;
     uint32_t h0 = 0, nx = 0;
-    uint32_t gk[NG], pend[NG];
+    uint32_t gk[NG], pend[NG], sub[4];
     const uint32_t hold = START ? (row < 0 ? 0x0000FFFFu : 0u) | (row < 1 ? 0xFFFF0000u : 0u) : 0u;
 #pragma unroll
     for (int h = 0; h < R; ++h) {
-        const int k = h >> 4, j = h & 15, jj = h & 7;
-        // equality bits of the low and high cells at bits pos and pos + 16
-        const uint32_t wsel = (j < 8) ? __byte_perm(eq[k], bw[k], 0x7632)
-                                      : __byte_perm(eq[k], bw[k], 0x5410);
-        const uint32_t wv = (jj < 4) ? wsel : wsel * c.x256;
-        const int pos = 14 - 2 * (jj & 3);
-        const uint32_t sub =
-            mad_hi(wv & ((1u << pos) | (1u << (pos + 16))), c.dm[jj & 3], c.sub2);
+        if ((h & 3) == 0) {  // row of the table: the byte of these four columns
+            const char *const row =
+                tab + __byte_perm(cw[h >> 4], l16, 0x7704 | ((3 - ((h >> 2) & 3)) << 4));
+            if (h + 1 < R) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(row);
+                sub[0] = v.x;
+                sub[1] = v.y;
+                sub[2] = v.z;
+                sub[3] = v.w;
+            } else {
+                sub[0] = *reinterpret_cast<const uint32_t *>(row);
+            }
+        }
         const uint32_t up = (h + 1 < R) ? Hr[h + 1 < R ? h + 1 : h] : __byte_perm(h0, nx, 0x5432);
         uint32_t hn;
         const uint32_t old = Hr[h];
         if (!NW) {
             const uint32_t e = __viaddmax_s16x2(el, c.ge2, up);
             const uint32_t tt = __vimax3_s16x2(e, hl, c.ng2);
-            hn = __viaddmax_s16x2(Hr[h], sub, tt) * c.one + c.neg_g2;
+            hn = __viaddmax_s16x2(Hr[h], sub[h & 3], tt) * c.one + c.neg_g2;
             el = e;
         } else {
-            const uint32_t tt = __vimax3_s16x2(up, hl, floor2);
-            hn = __viaddmax_s16x2(Hr[h], sub, tt);
+            hn = __vimax3_s16x2(__viaddmax_s16x2(Hr[h], sub[h & 3], up), hl, floor2);
             if (START) {
                 hn = (hn & ~hold) | (old & hold);
                 // row 0, left of the reference start: outside, although the initial
@@ -207,8 +217,10 @@ __device__ __forceinline__ void split_step(uint32_t (&Hr)[R], const uint32_t *eq
     }
 }
 
+constexpr int kSplitThreads = 256;
+
 template <int R, bool NW>
-__global__ void __launch_bounds__(128, R <= 17 ? 5 : 4)
+__global__ void __launch_bounds__(kSplitThreads, 2)
 split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t *__restrict__ bands,
              int32_t band, gb2_sw_result *__restrict__ out)
 {
@@ -216,8 +228,14 @@ split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t 
     constexpr int NB = (R + 15) / 16;      // words of its high columns
     constexpr int NG = (R + 7) / 8;
     const int lane = threadIdx.x & 31;
+    constexpr int WARPS = kSplitThreads / 32;
     const uint32_t FULL = 0xffffffffu;
     const uint32_t floor2 = (uint32_t)(uint16_t)(int16_t)kNwFloor * 0x00010001u;
+    extern __shared__ uint4 smem_tab[];
+    score_table_fill(smem_tab, c.sub2, c.dm, kSplitThreads);
+    __syncthreads();
+    const char *const tab = (const char *)smem_tab;
+    const uint32_t l16 = (uint32_t)(lane & 15) * 16;
 
     // Tasks: the pairs of one warp, a run of a segment's queue (longest first).  The
     // first task of a warp is given by its place in the grid, the segments in turn: if
@@ -225,8 +243,8 @@ split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t 
     // pairs for itself (50,000 mixed pairs: SMs busy 0.6 to 4.2 M cycles).  After
     // that a warp takes from the segment whose next pair is longest, so that no long
     // pair starts last.
-    const int64_t rank = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const int64_t warps = (int64_t)gridDim.x * 4;
+    const int64_t rank = warp_rank();
+    const int64_t warps = (int64_t)gridDim.x * WARPS;
     bool first_task = true;
     {
         for (;;) {
@@ -358,17 +376,18 @@ split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t 
                 }
                 const uint32_t qrep = mad_hi(qw, c.x4, 0u) * 0x55555555u;
                 qw *= c.x4;
-                uint32_t bw[NB];
-#pragma unroll
-                for (int i = 0; i < NB; ++i) {
-                    constexpr int A = R / 16, S = 2 * (R % 16);
-                    const uint32_t nxt = (A + i + 1 < NE) ? ep[A + i + 1 < NE ? A + i + 1 : 0] : 0u;
-                    bw[i] = S ? __funnelshift_l(nxt, ep[A + i], S) : ep[A + i];
-                }
 #pragma unroll
                 for (int i = 0; i < NE; ++i) {
                     const uint32_t x = win[i] ^ qrep;
                     eq[i] = ~(x | mad_hi(x, c.half, 0u)) & em[i];
+                }
+                uint32_t cw[NB];
+#pragma unroll
+                for (int i = 0; i < NB; ++i) {
+                    constexpr int A = R / 16, S = 2 * (R % 16) + 1;
+                    static_assert(S < 32, "one word back");
+                    const uint32_t nxt = (A + i + 1 < NE) ? ep[A + i + 1 < NE ? A + i + 1 : 0] : 0u;
+                    cw[i] = __funnelshift_l(nxt, ep[A + i < NE ? A + i : 0], S) | eq[i];
                 }
 #pragma unroll
                 for (int i = 0; i < NE; ++i)
@@ -377,11 +396,11 @@ split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t 
                 rw *= c.x4;
                 int32_t klo = 0, khi = 0;
                 if (NW && t < 2 * G)
-                    split_step<R, NW, true>(Hr, eq, bw, hl, el, klo, khi, G, last_mask, c, row, b,
-                                            c0);
+                    split_step<R, NW, true>(Hr, cw, tab, l16, hl, el, klo, khi, G, last_mask, c,
+                                            row, b, c0);
                 else
-                    split_step<R, NW, false>(Hr, eq, bw, hl, el, klo, khi, G, last_mask, c, row, b,
-                                             c0);
+                    split_step<R, NW, false>(Hr, cw, tab, l16, hl, el, klo, khi, G, last_mask, c,
+                                             row, b, c0);
                 // hand the last column's high half to the next lane; the low half is the
                 // left neighbour of this lane's high columns
                 if (!NW) {
@@ -535,11 +554,20 @@ auto with_shape(int shape, F f)
     }
 }
 
+template <typename K>
+cudaError_t split_smem(K *kern, bool nw, int shape)
+{
+    static std::atomic<uint64_t> done[2][kSplitShapes];  // one pointer type for all shapes
+    return allow_smem(kern, kScoreTableBytes, done[nw ? 1 : 0][shape]);
+}
+
 int occupancy(bool nw, int shape)
 {
-    auto occ = [](auto kern) {
+    auto occ = [&](auto kern) {
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 128, 0) != cudaSuccess)
+        if (split_smem(kern, nw, shape) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kSplitThreads,
+                                                          kScoreTableBytes) != cudaSuccess)
             cudaGetLastError();
         return std::max(nb, 1);
     };
@@ -549,6 +577,15 @@ int occupancy(bool nw, int shape)
 }  // namespace
 
 int split_regs(int shape) { return kRegs[shape]; }
+
+int split_grid(bool nw, int shape, int lg, int64_t n, int sm_count)
+{
+    // a block per warp's work while there are SMs without one: the warps of a block take
+    // the first tasks of the grid in turn
+    const int64_t per = 32 >> lg;
+    return (int)std::min<int64_t>((n + per - 1) / per,
+                                  (int64_t)sm_count * split_blocks_per_sm(nw, shape));
+}
 
 int split_blocks_per_sm(bool nw, int shape)
 {
@@ -579,15 +616,27 @@ bool split_rebase(const SwParams &p, int shape, int lg, int32_t *low, int32_t *h
     return lo + 128 <= hi && (m == 0 || hi / m >= 2 * cols + 2 * G + 16);
 }
 
-// Fitted to 1,000,000 reads (150 vs 200 bp, band 32: 139, 226, 290, 368, 402, 487, 568,
-// 652 cycles per warp and row for the shapes in order; Needleman-Wunsch 128, 198, 303,
-// 545 for R = 5, 9, 17, 33) and to 300-1,000 pairs of 2-10 kbp, one warp per scheduler
-// (296, 443, 557, 632, 603, 741, 943, 1,022).  The larger of the two times bounds the
-// batch and about a third of the other shows beside it (4,000 pairs of 2-10 kbp, band
-// 128: R = 9 3.0 ms, 17 3.5, 33 5.2; 16,000: 8.4, 7.5, 8.0).
-double split_time(double issue, double chain, double warps, const SplitLoad &l)
+// Fitted to 400,000 reads (150 vs 200 bp, band 33: 125, 181, 220, 286, 324, 388, 434, 500
+// cycles per warp and row for the shapes in order; Needleman-Wunsch 7.1 R + 74) and to
+// 150-600 pairs of 3-9 kbp, one warp per scheduler (244, 318, 381, 464, 524, 606, 676,
+// 785).  `rows`: rows a warp runs beside those of its pairs.
+// Pairs of one length run in rounds of four warps per scheduler, the last round as long
+// as its fullest scheduler (150 bp, band 32: 20,000 pairs R = 9, 17, one thread per pair
+// 97, 81, 79 us; 40,000: 155, 146, 111).  Of ragged pairs the longest come first: the
+// larger of all the work and the longest pair bounds the batch and about a third of the
+// other shows beside it; while all warps are resident the schedulers with one warp more
+// set the pace (16,000 pairs of 2-10 kbp, band 128: R = 33, 2,000 warps, 7.5 ms; R = 17,
+// 4,000 warps, 6.0; 4,000 pairs: R = 9 2.8 ms, 17 2.9, 33 4.3).
+double split_time(double issue, double chain, double warps, double rows, const SplitLoad &l)
 {
-    const double total = warps * issue * l.mean_rows, longest = chain * l.max_rows;
+    if (l.max_rows <= 1.25 * l.mean_rows) {
+        const double full = std::floor(warps / 4), rest = std::ceil(warps - 4 * full);
+        const double row = full * std::max(4 * issue, chain) +
+                           (rest > 0 ? std::max(rest * issue, chain) : 0.0);
+        return row * (l.max_rows + rows);
+    }
+    const double busy = warps <= 4 ? std::ceil(warps) : warps;
+    const double total = busy * issue * (l.mean_rows + rows), longest = chain * l.max_rows;
     return std::max(total, longest) + 0.35 * std::min(total, longest);
 }
 
@@ -605,7 +654,9 @@ SplitChoice split_choose(const SwParams &p, int32_t band, const SplitLoad &l, bo
             (!nw && long_scores && !split_rebase(p, s, lg, &low, &high)))
             continue;
         const double warps = (double)l.pairs * (1 << lg) / 32 / (4.0 * l.sm_count);
-        const double t = split_time((nw ? 15.0 : 17.5) * R + 62, 24.5 * R + 190, warps, l);
+        // 15,000 cycles: the start of a pair, which the one-thread kernel has not
+        const double t = 15000 + split_time(nw ? 7.1 * R + 74 : 13.3 * R + 60, 19.2 * R + 148,
+                                            warps, 2.0 * (1 << lg), l);
         if (best.shape < 0 || t < best.cost)
             best = SplitChoice{s, lg, t};
     }
@@ -620,21 +671,22 @@ cudaError_t launch_split(bool nw, int shape, SeqView q, SeqView r, SwParams p, i
     SplitConsts c;
     c.x4 = 4;
     c.x8 = 8;
-    c.x256 = 256;
     c.x64k = 65536;
     c.half = 0x80000000u;
     c.one = 1;
-    for (int i = 0; i < 4; ++i)
-        c.dm[i] = dm << (18 + 2 * i);
+    c.dm = dm;
     c.sub2 = ((uint32_t)p.mismatch + (nw ? 2 * g : g)) * 0x00010001u;
     c.neg_g2 = 0u - g * 0x00010001u;
+    c.ng2 = g * 0x00010001u;
     c.ge2 = (uint32_t)(uint16_t)p.ge * 0x00010001u;
-    c.ng2 = (uint32_t)(uint16_t)g * 0x00010001u;
     c.go = p.go;
     c.ge = p.ge;
     c.g = (int32_t)g;
     auto go = [&](auto kern) {
-        kern<<<grid, 128, 0, st>>>(q, r, c, work, bands, band, out);
+        const cudaError_t e = split_smem(kern, nw, shape);
+        if (e != cudaSuccess)
+            return e;
+        kern<<<grid, kSplitThreads, kScoreTableBytes, st>>>(q, r, c, work, bands, band, out);
         return cudaGetLastError();
     };
     return nw ? with_shape<true>(shape, go) : with_shape<false>(shape, go);
