@@ -54,13 +54,13 @@ BAND = 32
 SW_OPS_PER_CELL = 11  # int32 ops per cell of the reference recurrence (align_cpu.mojo:270-296)
 SW_OPS_PER_CELL_PACKED = 5.5  # the same ops on int16x2 lanes: two cells per lane-op
 # dram__bytes_read.sum + dram__bytes_write.sum of the dominant kernel per step of this
-# workload, from one ncu capture (not measurable inside a timed run): a step runs as 4
-# launches of 262,144 pairs; the captured launch read 32.02 MB and wrote 0 B (its 3.1 MB
-# of results were still in L2 when it ended), times 4.
-SW_PACKED_TRAFFIC_BYTES = 128.1e6
+# workload, from one ncu capture (not measurable inside a timed run): a launch of 65,536
+# pairs read 8.41 MB and wrote 0 B (its results were still in L2 when it ended), 128.3 B
+# per pair; a step runs as 4 launches of 250,000 pairs.
+SW_PACKED_TRAFFIC_BYTES = 128.3e6
 SW_PACKED_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum of one "
-                            "262,144-pair launch of sw_pack16_kernel<32>, x 4 launches per step "
-                            "(capture of commit 78a5858)")
+                            "65,536-pair launch of sw_pack16_kernel<32>, per pair, x 1,000,000 "
+                            "(profiles/sw_pack16_kernel_b32_1M_reads.md)")
 
 
 def parse():
@@ -484,7 +484,7 @@ def extras(args, dev, peak_ops, hbm_peak):
     threads = os.cpu_count() or 1
     out = {}
     # each band class alone: the 1,000,000 reads of the headline workload with one band
-    # for every pair (bands 16/32 take the narrow-key packed kernel, 64/128 the wide-key one)
+    # for every pair (bands 16/32 take the one-thread packed kernel, 64/128 the lane-split one)
     q1, r1, _, _ = synth.generate(1, 1_000_000)
     d1q, d1r = dev.upload_batch(q1, with_nmask=False), dev.upload_batch(r1, with_nmask=False)
     own1 = _PinnedOwner()
@@ -496,8 +496,8 @@ def extras(args, dev, peak_ops, hbm_peak):
                           5, 3)
         cells_b = synth.sw_cells(q1, band)
         classes[f"band_{band}"] = {"gcups": round(cells_b / tcb / 1e6, 1), "ms": round(tcb, 3),
-                                   "kernel": f"sw_pack16_kernel<{band}, "
-                                             f"{'narrow' if band <= 32 else 'wide'} keys>"}
+                                   "kernel": f"sw_pack16_kernel<{band}>" if band <= 32
+                                             else "split_kernel"}
     out["sw_band_classes_1M_reads"] = {
         "workload": "the 1,000,000 reads of the headline workload (150 vs 200 bp, "
                     "+2/-4/-4/-2), one band for every pair, resident, results into "

@@ -221,8 +221,8 @@ int gb2_nw_pair(gb2_ctx *ctx, const uint64_t *q_words, int64_t qlen,
  * encoding (:603-621); run_offsets has n_pairs + 1 entries.  runs_cap is the
  * capacity of `runs`: sum(qlen + rlen) over the pairs always suffices; when
  * the runs do not fit, returns GB2_ERANGE with run_offsets[n_pairs] set to the
- * number needed.  Device history: 5 B per visited wavefront cell + 12 B per
- * score, in groups that fit half the free device memory (at most 64 GiB, or
+ * number needed.  Device history: 5 B per wavefront cell that a pair's cost
+ * allows + 12 B per score, in groups that fit half the free device memory (at most 64 GiB, or
  * GB2_FLAGS_ARENA_MIB); GB2_ENOMEM when one pair alone does not fit. */
 int gb2_wfa_cigar(gb2_ctx *ctx, const gb2_batch *q, const gb2_batch *r,
                   const gb2_wfa_cfg *cfg, int64_t n_pairs, int32_t *cost,
