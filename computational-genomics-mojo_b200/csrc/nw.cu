@@ -27,6 +27,7 @@
 // band, per-pair bands.
 #include <algorithm>
 
+#include "nw_range.cuh"
 #include "runtime.cuh"
 
 namespace gb2 {
@@ -194,28 +195,16 @@ int nw_blocks_per_sm()
 
 using namespace gb2;
 
-// The shape and lane count of the lane-split kernel (sw_split.cu) for bands up to
-// maxb, or -1: its right padding needs mismatch >= 2 * (go + ge) and gap terms that
-// are not gains, its packed score steps match - mismatch <= 255, and every value
-// H + g * (qi + ri), re-centred by 2g per row every 16 rows, must lie between the
-// 16-bit limit and the floor that stands for cells outside the matrix.
+// The shape and lane count of the lane-split kernel (sw_split.cu) for bands up to maxb, or
+// -1 when there is none or the call's values leave its 16-bit registers (nw_range.cuh).
 static int nw_split_shape(const SwParams &p, int64_t maxb, int64_t qmax, int64_t rmax,
                           const SplitLoad &load, int &lg)
 {
-    const int64_t g = -((int64_t)p.go + p.ge), mm = p.mismatch, m = p.match;
-    if (maxb > kSplitMaxBand || g < 0 || g > 255 || p.ge > 0 || mm < -2 * g || mm > 255 || m < mm ||
-        m - mm > 255)
+    if (maxb > kSplitMaxBand)
         return -1;
     const SplitChoice ch = split_choose(p, (int32_t)maxb, load, true, false);
-    if (ch.shape < 0)
-        return -1;
-    const int64_t G = 1 << ch.lg, cols = 2 * (int64_t)split_regs(ch.shape) * G;
-    const int64_t len = std::min(qmax, rmax) + 1, mp = std::max<int64_t>(m, 0);
-    const int64_t drift = g * (36 + 4 * G + 2 * maxb + cols);
-    const int64_t top = mp * len + drift;
-    const int64_t bottom = std::max<int64_t>(-mm, 0) * len + g * (maxb + 2) +
-                           std::abs((int64_t)p.go) - maxb * p.ge + drift + 18 * (mp + 2 * g);
-    if (top > 32000 || bottom > 30500)
+    if (ch.shape < 0 || !nw_split_fits(p.match, p.mismatch, p.go, p.ge, maxb, qmax, rmax,
+                                       split_regs(ch.shape), ch.lg))
         return -1;
     lg = ch.lg;
     return ch.shape;

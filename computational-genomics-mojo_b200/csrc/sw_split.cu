@@ -37,7 +37,8 @@
 // of equality bits per 16 columns is therefore all the boundary handling: the
 // step has no masked variant.  Needleman-Wunsch needs mismatch >= 2(go+ge) for
 // the same argument, and its cells left of the reference start sit at a floor
-// far below every real value.
+// below every real value: they are computed too, and nw_range.cuh shows how far they
+// rise.
 //
 // Scores of any length in 16 bits (Smith-Waterman).  Registers hold H - base
 // with base per pair, and the maximum is found by keys (H - base) * 8 + tag, so
@@ -49,7 +50,7 @@
 // S + 16 * -mismatch while base > 0, so the floor at H = base never binds.
 // Needleman-Wunsch: registers hold H + g * (qi + ri) less 2g per row (the up and
 // left moves then add nothing: two DPX instructions per two cells), re-centred
-// every 16 steps; the host checks that the values fit.
+// every 16 steps; the host checks that the values fit (nw_range.cuh).
 //
 // What bounds it: instructions, which issue at about 0.65 per cycle and scheduler (see
 // sw_kernels.cu), 5.5 per register of two cells and 0.5 for its substitution term, one
@@ -75,12 +76,12 @@
 #include <cmath>
 
 #include "gb2_internal.cuh"
+#include "nw_range.cuh"
 
 namespace gb2 {
 namespace {
 
 constexpr uint32_t kSent = 0xC000u;          // -16384: start of the E chain
-constexpr int32_t kNwFloor = -31000;         // Needleman-Wunsch: cells outside the matrix
 constexpr int32_t kNwNeg = -1000000;
 
 struct SplitConsts {
@@ -219,7 +220,9 @@ __device__ __forceinline__ void split_step(uint32_t (&Hr)[R], const uint32_t *cw
 
 constexpr int kSplitThreads = 256;
 
-template <int R, bool NW>
+// WIDE_G: Needleman-Wunsch with g above kNwWrapFree (a kernel of its own: the branch alone
+// costs the others 1.4%, band 64).
+template <int R, bool NW, bool WIDE_G>
 __global__ void __launch_bounds__(kSplitThreads, 2)
 split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t *__restrict__ bands,
              int32_t band, gb2_sw_result *__restrict__ out)
@@ -456,6 +459,14 @@ split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t 
                 rr1 = word16(rp, rlen, ++rk);
                 if (NW && t0 > 0) {  // re-centre: 2g per row
                     const uint32_t d2 = (uint32_t)(uint16_t)(int16_t)(-32 * c.g) * 0x00010001u;
+                    if (WIDE_G) {  // the sum below wraps: no cell under floor + 32g
+                        const uint32_t lim2 =
+                            (uint32_t)(uint16_t)(int16_t)(kNwFloor + 32 * c.g) * 0x00010001u;
+#pragma unroll
+                        for (int h = 0; h < R; ++h)
+                            Hr[h] = __vmaxs2(Hr[h], lim2);
+                        hl = __vmaxs2(hl, lim2);
+                    }
 #pragma unroll
                     for (int h = 0; h < R; ++h)
                         Hr[h] = __viaddmax_s16x2(Hr[h], d2, floor2);
@@ -539,39 +550,47 @@ split_kernel(SeqView q, SeqView r, SplitConsts c, SplitWork work, const int32_t 
 
 constexpr int kRegs[kSplitShapes] = {5, 9, 13, 17, 21, 25, 29, 33};
 
-template <bool NW, typename F>
+template <bool NW, bool WIDE_G, typename F>
 auto with_shape(int shape, F f)
 {
     switch (shape) {
-    case 0: return f(split_kernel<kRegs[0], NW>);
-    case 1: return f(split_kernel<kRegs[1], NW>);
-    case 2: return f(split_kernel<kRegs[2], NW>);
-    case 3: return f(split_kernel<kRegs[3], NW>);
-    case 4: return f(split_kernel<kRegs[4], NW>);
-    case 5: return f(split_kernel<kRegs[5], NW>);
-    case 6: return f(split_kernel<kRegs[6], NW>);
-    default: return f(split_kernel<kRegs[7], NW>);
+    case 0: return f(split_kernel<kRegs[0], NW, WIDE_G>);
+    case 1: return f(split_kernel<kRegs[1], NW, WIDE_G>);
+    case 2: return f(split_kernel<kRegs[2], NW, WIDE_G>);
+    case 3: return f(split_kernel<kRegs[3], NW, WIDE_G>);
+    case 4: return f(split_kernel<kRegs[4], NW, WIDE_G>);
+    case 5: return f(split_kernel<kRegs[5], NW, WIDE_G>);
+    case 6: return f(split_kernel<kRegs[6], NW, WIDE_G>);
+    default: return f(split_kernel<kRegs[7], NW, WIDE_G>);
     }
 }
 
-template <typename K>
-cudaError_t split_smem(K *kern, bool nw, int shape)
+template <typename F>
+auto with_kernel(bool nw, bool wide_g, int shape, F f)
 {
-    static std::atomic<uint64_t> done[2][kSplitShapes];  // one pointer type for all shapes
-    return allow_smem(kern, kScoreTableBytes, done[nw ? 1 : 0][shape]);
+    return !nw      ? with_shape<false, false>(shape, f)
+           : wide_g ? with_shape<true, true>(shape, f)
+                    : with_shape<true, false>(shape, f);
+}
+
+template <typename K>
+cudaError_t split_smem(K *kern, bool nw, bool wide_g, int shape)
+{
+    static std::atomic<uint64_t> done[3][kSplitShapes];  // one pointer type for all shapes
+    return allow_smem(kern, kScoreTableBytes, done[wide_g ? 2 : nw ? 1 : 0][shape]);
 }
 
 int occupancy(bool nw, int shape)
 {
     auto occ = [&](auto kern) {
         int nb = 0;
-        if (split_smem(kern, nw, shape) != cudaSuccess ||
+        if (split_smem(kern, nw, false, shape) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kSplitThreads,
                                                           kScoreTableBytes) != cudaSuccess)
             cudaGetLastError();
         return std::max(nb, 1);
     };
-    return nw ? with_shape<true>(shape, occ) : with_shape<false>(shape, occ);
+    return with_kernel(nw, false, shape, occ);
 }
 
 }  // namespace
@@ -682,14 +701,15 @@ cudaError_t launch_split(bool nw, int shape, SeqView q, SeqView r, SwParams p, i
     c.go = p.go;
     c.ge = p.ge;
     c.g = (int32_t)g;
+    const bool wide_g = nw && c.g > kNwWrapFree;
     auto go = [&](auto kern) {
-        const cudaError_t e = split_smem(kern, nw, shape);
+        const cudaError_t e = split_smem(kern, nw, wide_g, shape);
         if (e != cudaSuccess)
             return e;
         kern<<<grid, kSplitThreads, kScoreTableBytes, st>>>(q, r, c, work, bands, band, out);
         return cudaGetLastError();
     };
-    return nw ? with_shape<true>(shape, go) : with_shape<false>(shape, go);
+    return with_kernel(nw, wide_g, shape, go);
 }
 
 }  // namespace gb2
