@@ -24,8 +24,10 @@ constexpr int32_t kNwWrapFree = (32768 + kNwFloor) / 32;
 //   re-centred, put on the register beside that.
 // The floor's life: cells left of the reference start and above row 0 start at it.  They
 // are computed like the others, with no matches, so a row adds mismatch + 2g to them and
-// 16 rows, which the next re-centring takes back.  So such a cell is at most
-//   floor + 18 * (mismatch + 2g)
+// 16 rows, which the next re-centring takes back but for 16 * mismatch.  Only a diagonal
+// move gains, and it brings a cell left of the start one position nearer to it: at most
+// maxb of them before the cell is a neighbour of a real one.  So such a cell is at most
+//   floor + 18 * (mismatch + 2g) + maxb * max(mismatch, 0)
 // at any time, and at least the floor; 500 are to spare below the lowest real cell.
 inline bool nw_split_fits(int64_t match, int64_t mismatch, int64_t go, int64_t ge, int64_t maxb,
                           int64_t qmax, int64_t rmax, int regs, int lg)
@@ -40,7 +42,7 @@ inline bool nw_split_fits(int64_t match, int64_t mismatch, int64_t go, int64_t g
     const int64_t top = mp * len + drift;
     const int64_t bottom = std::max<int64_t>(-mismatch, 0) * len + g * (maxb + 2) + std::abs(go) -
                            maxb * ge + drift;
-    const int64_t climb = 18 * (mp + 2 * g);
+    const int64_t climb = 18 * (mp + 2 * g) + maxb * std::max<int64_t>(mismatch, 0);
     return top <= 32000 && bottom + climb + 500 <= -kNwFloor;
 }
 

@@ -1,5 +1,6 @@
 """The 16-bit range of the lane-split Needleman-Wunsch kernel: large gap costs, whose
-re-centring must not wrap the floor that stands for cells outside the matrix.
+re-centring must not wrap the floor that stands for cells outside the matrix, and positive
+mismatch scores, which make cells left of the reference start climb from it.
 
 On the CPU the kernel's arithmetic (nw_split_model.cpp, with the library's own admission
 rule) against the oracle; on the GPU the calls themselves.  Whether a case runs on the
@@ -76,12 +77,14 @@ def _model_scores(model, qs, rs, sc, band, regs, lg, wrapping=0):
 
 
 # match, mismatch, gap open, gap extend: g = -(open + extend) on both sides of 55, up to which
-# the floor of -31000 less 32g fits 16 bits
+# the floor of -31000 less 32g fits 16 bits; and mismatches above 0
 GAPS = [(2, -4, -50, -4), (2, -4, -50, -5), (2, -4, -54, -2), (5, -4, -60, -1), (2, -4, -60, -10),
         (20, -60, -50, -20), (10, -40, -40, -16), (10, -20, -100, -10), (1, 0, -150, 0)]
+GAINS = [(5, 2, -4, -2), (20, 10, -4, -2), (70, 60, -2, -1), (150, 120, -2, -1), (255, 255, 0, 0),
+         (60, 30, -58, -2)]
 
 
-@pytest.mark.parametrize("sc", GAPS)
+@pytest.mark.parametrize("sc", GAPS + GAINS)
 def test_model_is_exact_where_the_rule_admits(model, oracle, sc):
     rng = np.random.default_rng(abs(sc[1]) + abs(sc[2]))
     admitted = 0
@@ -100,14 +103,40 @@ def test_model_is_exact_where_the_rule_admits(model, oracle, sc):
     assert admitted >= 20, (sc, admitted)
 
 
+def test_model_of_short_references(model, oracle):
+    """Queries much longer than their references inside a wide band: the most rows of cells
+    left of the reference start, with gains for mismatches."""
+    rng = np.random.default_rng(5)
+    seen = {True: 0, False: 0}
+    for band in (100, 250, 400, 543):
+        for sc in GAINS + [(2, -4, -4, -2), (2, -4, -4, -60)]:
+            qs = [rng.integers(0, 4, 100 + int(rng.integers(0, band))).astype(np.uint8)
+                  for _ in range(4)]
+            rs = [rng.integers(0, 4, 100).astype(np.uint8) for _ in range(4)]
+            want = _want(oracle, _batch(qs), _batch(rs), sc, band).tolist()
+            fits = _fits(model, sc, band, max(map(len, qs)), 100)
+            for ok, (regs, lg) in zip(fits, _shapes(band)):
+                seen[ok] += 1
+                if ok:
+                    assert _model_scores(model, qs, rs, sc, band, regs, lg) == want
+    assert min(seen.values()) >= 10, seen
+
+
 def test_a_floor_that_wraps_is_seen(model, oracle):
-    """The model finds the fault: a floor that wraps at g = 56."""
+    """The model finds both faults: a floor that wraps at g = 56, and a climb that the rule
+    refuses."""
     rng = np.random.default_rng(1)
     qs, rs = _pairs(rng, 40, 9, 4)
     sc = (2, -4, -54, -2)
     want = _want(oracle, _batch(qs), _batch(rs), sc, 4).tolist()
     assert _model_scores(model, qs, rs, sc, 4, 5, 0) == want
     assert _model_scores(model, qs, rs, sc, 4, 5, 0, wrapping=1) != want
+    sc = (150, 120, -2, -1)
+    qs = [rng.integers(0, 4, 420).astype(np.uint8)]
+    rs = [rng.integers(0, 4, 100).astype(np.uint8)]
+    want = _want(oracle, _batch(qs), _batch(rs), sc, 400).tolist()
+    assert not any(_fits(model, sc, 400, 420, 100))
+    assert _model_scores(model, qs, rs, sc, 400, 13, 5) != want
 
 
 def _gpu_check(device, oracle, qs, rs, sc, band):
@@ -128,15 +157,17 @@ ADMITTED = [(sc, band, qlen) for sc in ((2, -4, -50, -5), (2, -4, -54, -2), (2, 
             if (sc[2], band) != (-60, 64)] + [
     ((2, -4, -20, -5), 131, 33), ((10, -40, -40, -16), 16, 60), ((5, -4, -60, -1), 32, 150),
     ((10, -20, -100, -10), 4, 60)]
+ADMITTED_GAINS = [((20, 10, -4, -2), 64, 150), ((20, 10, -4, -2), 400, 33),
+                  ((5, 2, -4, -2), 400, 150), ((60, 30, -58, -2), 16, 60)]
 
 
 def test_the_cases_of_the_lane_split_kernel_are_its_own(model):
-    for sc, band, qlen in ADMITTED:
+    for sc, band, qlen in ADMITTED + ADMITTED_GAINS:
         assert all(_fits(model, sc, band, qlen, qlen + 4)), (sc, band, qlen)
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("sc,band,qlen", ADMITTED)
+@pytest.mark.parametrize("sc,band,qlen", ADMITTED + ADMITTED_GAINS)
 def test_gpu_cases_of_the_lane_split_kernel(device, oracle, model, sc, band, qlen):
     """Few pairs and many (the shapes with the most lanes, and with the most columns)."""
     rng = np.random.default_rng(band + qlen)
@@ -160,3 +191,15 @@ def test_gpu_largest_gap_costs(device, oracle, model, band, qlen):
     assert every > 55 or band >= 64, (every, some)
     for g in sorted({every, every + 1, some, some + 1}):
         _gpu_check(device, oracle, qs * 40, rs * 40, (2, -4, -(g - 2), -2), band)
+
+
+@pytest.mark.gpu
+def test_gpu_positive_mismatch_in_a_wide_band(device, oracle, model):
+    """Queries longer than their references by most of the band: refused by the rule where
+    cells left of the reference start could pass real ones, exact either way."""
+    rng = np.random.default_rng(9)
+    qs = [rng.integers(0, 4, 420 - i).astype(np.uint8) for i in range(40)]
+    rs = [rng.integers(0, 4, 100).astype(np.uint8) for _ in range(40)]
+    for sc, admitted in (((150, 120, -2, -1), False), ((5, 2, -4, -2), True)):
+        assert all(f == admitted for f in _fits(model, sc, 400, 420, 100)), sc
+        _gpu_check(device, oracle, qs, rs, sc, 400)
