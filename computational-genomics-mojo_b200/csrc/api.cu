@@ -758,7 +758,7 @@ static int wfa_block_warps(int64_t qmax, int64_t rmax, int64_t n, int variant)
 // The first tier: one warp per pair costs the least work, more warps the least time for
 // the longest pair.  What decides is how many pairs as long as the longest the batch
 // amounts to, by the square of the length (the mean over the longest to the power 1.5
-// estimates that from the packed words).  Measured, 1 / 4 / 8 warps first (ms):
+// estimates that).  Measured, 1 / 4 / 8 warps first (ms):
 //   100-10,000 bp, 300 pairs (30 such)  4.39 / 2.87 / 2.58;  4,000 (400) 6.26 / 4.56 / 4.48
 //   8,000 (800) 7.5 / 7.5 / 8.9;  12,000 (1,200) 8.9 / 10.4 / 13.2
 //   100-1,500 bp, 3,000 (610) 0.57 / 0.44 / 0.69;  8,000 (1,600) 0.73 / 0.95 / 1.62
@@ -777,7 +777,8 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         pl.usable[1] = false;
     constexpr int G = kWfaShared;  // the global-memory tier
     const double longest = (double)std::max<int64_t>({qmax, rmax, 1});
-    const double mean = std::min(32.0 * (double)std::max(qv.n_words, rv.n_words) / (double)n, longest);
+    const double mean = std::max(mean_length(qv, n, (int64_t)longest),
+                                 mean_length(rv, n, (int64_t)longest));
     const double alike = (double)n * std::pow(mean / longest, 1.5) / (double)sms;
     int first = alike > 6.0 ? 0 : (alike > 2.7 ? 2 : 3);
     while (first < G && !pl.usable[first])
@@ -1053,9 +1054,10 @@ int wfa_end(gb2_ctx *c, Exec &x)
 // ---------------------------------------------------------------------------
 // blocking helpers of the context's own executor
 // ---------------------------------------------------------------------------
-static SeqView view_of(const gb2_batch *b)
+static SeqView view_of(const gb2_batch *b, int64_t n)
 {
-    return SeqView{b->d_packed, b->d_offsets, b->d_lengths, 0, std::max<int64_t>(b->n_words, 1)};
+    return SeqView{b->d_packed, b->d_offsets, b->d_lengths, 0, std::max<int64_t>(b->n_words, 1),
+                   bases_share(b->bases, n, b->count)};
 }
 
 static int sync_and_check(gb2_ctx *c)
@@ -1247,16 +1249,17 @@ struct HostSide {
 // as int32 into pinned staging, and the device rebuilds both int64 arrays).
 // Large chunks are split over two threads.
 struct ChunkScan {
-    int64_t qw0, qw1, rw0, rw1, qmaxlen, rmaxlen;
+    int64_t qw0, qw1, rw0, rw1, qmaxlen, rmaxlen, qbases, rbases;
     bool negative, narrow;  // narrow: every length within narrow_range
     bool dense;             // both sides contiguous, lengths staged as int32
 };
 
 static void scan_side(const HostSide &h, int64_t i0, int64_t i1, int64_t &w0, int64_t &w1,
-                      int64_t &minlen, int64_t &maxlen, int64_t &bits, bool &contig,
-                      int32_t *len32)
+                      int64_t &minlen, int64_t &maxlen, int64_t &bases, int64_t &bits,
+                      bool &contig, int32_t *len32)
 {
     int64_t lo = INT64_MAX, hi = 0, mn = INT64_MAX, mx = 0, b = 0;
+    uint64_t sum = 0;  // (lengths that are no lengths may wrap it)
     int64_t expect = i1 > i0 ? h.offsets[i0] : 0;
     bool ct = true;
     for (int64_t i = i0; i < i1; ++i) {
@@ -1264,6 +1267,7 @@ static void scan_side(const HostSide &h, int64_t i0, int64_t i1, int64_t &w0, in
         b |= o | l;
         mx = l > mx ? l : mx;
         mn = l < mn ? l : mn;
+        sum += (uint64_t)l;
         lo = o < lo ? o : lo;
         const int64_t e = o + ((l + 31) >> 5);
         hi = e > hi ? e : hi;
@@ -1275,13 +1279,14 @@ static void scan_side(const HostSide &h, int64_t i0, int64_t i1, int64_t &w0, in
     w1 = hi;
     minlen = mn;
     maxlen = mx;
+    bases = (int64_t)sum;
     bits = b;
     contig = ct;
 }
 
 // One side's part of a chunk scan.
 struct SideScan {
-    int64_t w0 = 0, w1 = 0, minlen = 0, maxlen = 0, bits = 0;
+    int64_t w0 = 0, w1 = 0, minlen = 0, maxlen = 0, bases = 0, bits = 0;
     bool contig = true;
 };
 
@@ -1295,6 +1300,8 @@ static ChunkScan combine(const SideScan &q, const SideScan &r)
     o.rw1 = std::max(r.w1, r.w0);
     o.qmaxlen = q.maxlen;
     o.rmaxlen = r.maxlen;
+    o.qbases = q.bases;
+    o.rbases = r.bases;
     o.narrow = narrow_range(q.minlen, q.maxlen) && narrow_range(r.minlen, r.maxlen);
     o.dense = q.contig && r.contig && q.maxlen < (1ll << 31) && r.maxlen < (1ll << 31);
     return o;
@@ -1468,8 +1475,8 @@ static int pipeline(gb2_ctx *c, const HostSide &hq, const HostSide &hr, const in
         for (int64_t ci = 0; ci < nchunks; ++ci) {
             const int64_t p0 = bounds[(size_t)ci], p1 = bounds[(size_t)ci + 1];
             SideScan &sc = (*out)[(size_t)ci];
-            scan_side(h, p0, p1, sc.w0, sc.w1, sc.minlen, sc.maxlen, sc.bits, sc.contig,
-                      stage + 2 * p0 + (side ? p1 - p0 : 0));
+            scan_side(h, p0, p1, sc.w0, sc.w1, sc.minlen, sc.maxlen, sc.bases, sc.bits,
+                      sc.contig, stage + 2 * p0 + (side ? p1 - p0 : 0));
             done->store(ci + 1, std::memory_order_release);
         }
     };
@@ -1557,9 +1564,9 @@ static int pipeline(gb2_ctx *c, const HostSide &hq, const HostSide &hr, const in
             CU(c, cudaStreamWaitEvent(x.st, ps.copied, 0));
         }
         const SeqView qv{(const uint64_t *)ps.qw.p, (const int64_t *)ps.qo.p,
-                         (const int64_t *)ps.ql.p, cs.qw0, qn};
+                         (const int64_t *)ps.ql.p, cs.qw0, qn, cs.qbases};
         const SeqView rv{(const uint64_t *)ps.rw.p, (const int64_t *)ps.ro.p,
-                         (const int64_t *)ps.rl.p, cs.rw0, rn};
+                         (const int64_t *)ps.rl.p, cs.rw0, rn, cs.rbases};
         if ((r = run_chunk(x, qv, rv, cs.qmaxlen, cs.rmaxlen, cs.narrow,
                            bands ? (const int32_t *)ps.bands.p : nullptr,
                            bands ? bands + p0 : nullptr, m, ps.out.p)))
@@ -1774,18 +1781,20 @@ static int gb2_batch_upload_impl(gb2_ctx *c, const uint64_t *packed, int64_t n_w
     if (count < 0 || n_words < 0 || (count > 0 && (!offsets || !lengths)) ||
         (n_words > 0 && !packed))
         return set_err(c, GB2_EINVAL, "batch arrays missing or sizes negative");
-    int64_t maxlen = 0, minlen = count > 0 ? INT64_MAX : 0;
+    int64_t maxlen = 0, minlen = count > 0 ? INT64_MAX : 0, bases = 0;
     for (int64_t i = 0; i < count; ++i) {
         if (lengths[i] < 0 || offsets[i] < 0 || offsets[i] + words_for(lengths[i]) > n_words)
             return set_err(c, GB2_EINVAL, "sequence %lld lies outside the packed words",
                            (long long)i);
         maxlen = std::max(maxlen, lengths[i]);
         minlen = std::min(minlen, lengths[i]);
+        bases += lengths[i];
     }
     gb2_batch *b = new gb2_batch();
     b->owner = c;
     b->count = count;
     b->n_words = n_words;
+    b->bases = bases;
     b->max_len = maxlen;
     b->min_len = minlen;
     const size_t wb = (size_t)std::max<int64_t>(n_words, 1) * 8;
@@ -1903,7 +1912,7 @@ static int gb2_sw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
                            cfg->band_width, n, flags, bands ? 1 : 0, pi.max_band});
     if (parts == 1) {
         rc = run_graphed(c, c->g_sw, key, flags, nullptr, [&](bool capturing) -> int {
-            return sw_core(c, c->x, view_of(q), view_of(r), q->max_len, r->max_len, cfg,
+            return sw_core(c, c->x, view_of(q, n), view_of(r, n), q->max_len, r->max_len, cfg,
                            d_bands, pi, n, (gb2_sw_result *)c->out_sw.p, flags, !capturing);
         });
         if (rc) {
@@ -1936,11 +1945,8 @@ static int gb2_sw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
         for (int k = 0; k < parts && r2 == GB2_OK; ++k) {
             const int64_t p0 = k * per, m = std::min(per, n - p0);
             Exec &ex = (k & 1) ? c->x2 : c->x;
-            SeqView qv = view_of(q), rv = view_of(r);
-            qv.offsets += p0;
-            qv.lengths += p0;
-            rv.offsets += p0;
-            rv.lengths += p0;
+            const SeqView qv = part_of(view_of(q, n), p0, m, n);
+            const SeqView rv = part_of(view_of(r, n), p0, m, n);
             r2 = sw_core(c, ex, qv, rv, q->max_len, r->max_len, cfg,
                          d_bands ? d_bands + p0 : nullptr, pi, m, dres + p0, flags, false);
             if (!r2 && !capturing && cudaEventRecord(c->kdone[k], ex.st) != cudaSuccess)
@@ -2062,8 +2068,8 @@ static int pair_upload(gb2_ctx *c, const uint64_t *q_words, int64_t qlen, const 
     memcpy(h + 4 + qn, r_words, (size_t)words_for(rlen) * 8);
     CU(c, cudaMemcpyAsync(c->pair_in.p, h, bytes, cudaMemcpyHostToDevice, c->x.st));
     const int64_t *const d = (const int64_t *)c->pair_in.p;
-    qv = SeqView{(const uint64_t *)d + 4, d, d + 1, 0, qn};
-    rv = SeqView{(const uint64_t *)d + 4 + qn, d + 2, d + 3, 0, rn};
+    qv = SeqView{(const uint64_t *)d + 4, d, d + 1, 0, qn, qlen};
+    rv = SeqView{(const uint64_t *)d + 4 + qn, d + 2, d + 3, 0, rn, rlen};
     return GB2_OK;
 }
 
@@ -2137,7 +2143,7 @@ static int gb2_wfa_affine_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *
         int r2;
         if ((r2 = wfa_begin(c, c->x)))
             return r2;
-        return wfa_core(c, c->x, view_of(q), view_of(r), q->max_len, r->max_len, cfg, n,
+        return wfa_core(c, c->x, view_of(q, n), view_of(r, n), q->max_len, r->max_len, cfg, n,
                         (int32_t *)c->out_wfa.p, run_flags);
     });
     if (rc) {
@@ -2347,7 +2353,7 @@ int gb2_autotune(gb2_ctx *c, int kind, const gb2_batch *q, const gb2_batch *r, c
         // classes of the mix run with their installed variants
         run = [=](int v) {
             *slot = v;
-            return sw_core(c, c->x, view_of(q), view_of(r), q->max_len, r->max_len, cfg, d_bands,
+            return sw_core(c, c->x, view_of(q, n), view_of(r, n), q->max_len, r->max_len, cfg, d_bands,
                            pi, n, (gb2_sw_result *)c->out_sw.p, GB2_FLAG_BATCHED | GB2_FLAG_INT32,
                            false);
         };
@@ -2366,7 +2372,7 @@ int gb2_autotune(gb2_ctx *c, int kind, const gb2_batch *q, const gb2_batch *r, c
             int r2;
             if ((r2 = wfa_begin(c, c->x)))
                 return r2;
-            return wfa_core(c, c->x, view_of(q), view_of(r), q->max_len, r->max_len, cfg, n,
+            return wfa_core(c, c->x, view_of(q, n), view_of(r, n), q->max_len, r->max_len, cfg, n,
                             (int32_t *)c->out_wfa.p, GB2_FLAG_BATCHED | (v << 8));
         };
     } else {

@@ -5,17 +5,9 @@
 #include <stdint.h>
 
 #include "genomics_b200.h"
+#include "seq_view.cuh"
 
 namespace gb2 {
-
-// Device view of one SequenceBatch side of a pair list.
-struct SeqView {
-    const uint64_t *packed;  // packed words resident on the device
-    const int64_t *offsets;  // word offset of each sequence (SequenceBatch.offsets)
-    const int64_t *lengths;  // bases of each sequence (SequenceBatch.lengths)
-    int64_t word_base;       // offsets[i] - word_base indexes `packed`
-    int64_t n_words;         // words in `packed` (reads are clamped to it)
-};
 
 // Which pairs a launch processes: queue[start .. start+n) of pair indices
 // (queue == nullptr: pairs [0, n)).  When seg != nullptr the device array
@@ -147,9 +139,7 @@ struct SplitLoad {
 };
 inline SplitLoad split_load(const SeqView &q, int64_t qmax, int64_t n, int sm_count)
 {
-    // the packed words bound the mean length (a layout with gaps or shared words: qmax)
-    const double mean = 32.0 * (double)q.n_words / (double)n;
-    return SplitLoad{n, mean < (double)qmax ? mean : (double)qmax, (double)qmax, sm_count};
+    return SplitLoad{n, mean_length(q, n, qmax), (double)qmax, sm_count};
 }
 // Estimated cycles of a batch whose warps issue for `issue` cycles per row, or whose
 // longest pair takes `chain` cycles per row; warps per scheduler.

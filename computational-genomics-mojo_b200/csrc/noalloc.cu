@@ -132,8 +132,8 @@ extern "C" int gb2_wfa_affine_noalloc(const uint64_t *q_packed, int64_t q_words,
         cudaGetLastError();
         return GB2_ECUDA;
     }
-    gb2::SeqView qv{q_packed, q_offsets, q_lengths, 0, q_words};
-    gb2::SeqView rv{r_packed, r_offsets, r_lengths, 0, r_words};
+    gb2::SeqView qv{q_packed, q_offsets, q_lengths, 0, q_words, 0};
+    gb2::SeqView rv{r_packed, r_offsets, r_lengths, 0, r_words, 0};
     gb2::WfaParams p{cfg->x, cfg->o, cfg->e, cfg->max_error};
     const gb2::PairList none{nullptr, 0, nullptr, counter};
     const gb2::PairList pl{nullptr, n_pairs, nullptr, counter};

@@ -321,8 +321,10 @@ static int gb2_nw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
     if ((rc = nw_validate(c, cfg, bands, n, q->max_len, r->max_len, maxb)) ||
         (rc = ensure(c, c->out_sw, (size_t)n * sizeof(gb2_sw_result), c->x.st)))
         return rc;
-    const SeqView qv{q->d_packed, q->d_offsets, q->d_lengths, 0, q->n_words};
-    const SeqView rv{r->d_packed, r->d_offsets, r->d_lengths, 0, r->n_words};
+    const SeqView qv{q->d_packed, q->d_offsets, q->d_lengths, 0, q->n_words,
+                     bases_share(q->bases, n, q->count)};
+    const SeqView rv{r->d_packed, r->d_offsets, r->d_lengths, 0, r->n_words,
+                     bases_share(r->bases, n, r->count)};
     const bool narrow = narrow_range(q->min_len, q->max_len) && narrow_range(r->min_len, r->max_len);
     const int32_t *d_bands = nullptr;
     if (bands) {
@@ -340,7 +342,8 @@ static int gb2_nw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
         return (flags & GB2_FLAG_GENERIC)
                    ? -1
                    : nw_split_shape(p, maxb, q->max_len, r->max_len,
-                                    split_load(qv, q->max_len, m, c->sm_count), lg);
+                                    split_load(part_of(qv, 0, m, n), q->max_len, m, c->sm_count),
+                                    lg);
     };
     int parts = n >= kResidentSplit ? kResidentParts : 1, lg = 0;
     int shape = shape_for((n + parts - 1) / parts, lg);
@@ -361,11 +364,7 @@ static int gb2_nw_banded_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
     for (int k = 0; k < parts; ++k) {
         const int64_t p0 = k * per, m = std::min(per, n - p0);
         Exec &x = (k & 1) ? c->x2 : c->x;
-        SeqView qk = qv, rk = rv;
-        qk.offsets += p0;
-        qk.lengths += p0;
-        rk.offsets += p0;
-        rk.lengths += p0;
+        const SeqView qk = part_of(qv, p0, m, n), rk = part_of(rv, p0, m, n);
         if ((rc = nw_core(c, x, qk, rk, p, cfg->band_width, d_bands ? d_bands + p0 : nullptr,
                           maxb, shape, lg, m, dres + p0, flags, narrow)))
             return rc;

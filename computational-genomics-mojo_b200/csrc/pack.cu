@@ -77,13 +77,14 @@ static int gb2_batch_from_ascii_impl(gb2_ctx *c, const uint8_t *ascii, int64_t a
         (ascii_bytes > 0 && !ascii))
         return set_err(c, GB2_EINVAL, "ascii batch arrays missing or sizes negative");
     std::vector<int64_t> woff((size_t)std::max<int64_t>(count, 1));
-    int64_t words = 0, maxlen = 0, minlen = count > 0 ? INT64_MAX : 0;
+    int64_t words = 0, bases = 0, maxlen = 0, minlen = count > 0 ? INT64_MAX : 0;
     for (int64_t i = 0; i < count; ++i) {
         if (lengths[i] < 0 || starts[i] < 0 || starts[i] + lengths[i] > ascii_bytes)
             return set_err(c, GB2_EINVAL, "sequence %lld lies outside the ascii buffer",
                            (long long)i);
         woff[(size_t)i] = words;
         words += words_for(lengths[i]);
+        bases += lengths[i];
         maxlen = std::max(maxlen, lengths[i]);
         minlen = std::min(minlen, lengths[i]);
     }
@@ -91,6 +92,7 @@ static int gb2_batch_from_ascii_impl(gb2_ctx *c, const uint8_t *ascii, int64_t a
     b->owner = c;
     b->count = count;
     b->n_words = words;
+    b->bases = bases;
     b->max_len = maxlen;
     b->min_len = minlen;
     uint8_t *d_ascii = nullptr;

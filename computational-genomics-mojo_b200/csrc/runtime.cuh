@@ -150,7 +150,7 @@ struct gb2_batch {
     uint64_t *d_nmask = nullptr;
     int64_t *d_offsets = nullptr;
     int64_t *d_lengths = nullptr;
-    int64_t count = 0, n_words = 0, max_len = 0, min_len = 0;
+    int64_t count = 0, n_words = 0, max_len = 0, min_len = 0, bases = 0;
     gb2_ctx *owner = nullptr;
 };
 

@@ -287,9 +287,9 @@ int launch_group(gb2_server *s, Slot &sl)
     const int flags = s->cfg.flags | GB2_FLAG_BATCHED;
     if (L.n_sw) {
         SeqView qv{(const uint64_t *)(d + L.o_sqw), (const int64_t *)(d + L.o_sqo),
-                   (const int64_t *)(d + L.o_sql), 0, std::max<int64_t>(L.sw_qw, 1)};
+                   (const int64_t *)(d + L.o_sql), 0, std::max<int64_t>(L.sw_qw, 1), L.sw_qw * 32};
         SeqView rv{(const uint64_t *)(d + L.o_srw), (const int64_t *)(d + L.o_sro),
-                   (const int64_t *)(d + L.o_srl), 0, std::max<int64_t>(L.sw_rw, 1)};
+                   (const int64_t *)(d + L.o_srl), 0, std::max<int64_t>(L.sw_rw, 1), L.sw_rw * 32};
         // bands come per pair from the staged array; the config's own band is unused
         gb2_sw_cfg cfg = R0.sw_cfg;
         cfg.band_width = L.max_band;
@@ -305,9 +305,9 @@ int launch_group(gb2_server *s, Slot &sl)
     }
     if (L.n_wfa) {
         SeqView qv{(const uint64_t *)(d + L.o_wqw), (const int64_t *)(d + L.o_wqo),
-                   (const int64_t *)(d + L.o_wql), 0, std::max<int64_t>(L.wfa_qw, 1)};
+                   (const int64_t *)(d + L.o_wql), 0, std::max<int64_t>(L.wfa_qw, 1), L.wfa_qw * 32};
         SeqView rv{(const uint64_t *)(d + L.o_wrw), (const int64_t *)(d + L.o_wro),
-                   (const int64_t *)(d + L.o_wrl), 0, std::max<int64_t>(L.wfa_rw, 1)};
+                   (const int64_t *)(d + L.o_wrl), 0, std::max<int64_t>(L.wfa_rw, 1), L.wfa_rw * 32};
         if ((rc = wfa_begin(c, x)) ||
             (rc = wfa_core(c, x, qv, rv, L.wfa_qmax, L.wfa_rmax, &R0.wfa_cfg, L.n_wfa,
                            (int32_t *)(dout + L.o_wout), flags)))

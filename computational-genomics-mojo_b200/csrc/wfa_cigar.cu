@@ -270,8 +270,10 @@ static int gb2_wfa_cigar_impl(gb2_ctx *c, const gb2_batch *q, const gb2_batch *r
     GB2_CU(c, cudaMemcpyAsync(rl.data(), r->d_lengths, (size_t)n * 8, cudaMemcpyDeviceToHost,
                               c->x.st));
     GB2_CU(c, cudaStreamSynchronize(c->x.st));
-    const SeqView qv{q->d_packed, q->d_offsets, q->d_lengths, 0, q->n_words};
-    const SeqView rv{r->d_packed, r->d_offsets, r->d_lengths, 0, r->n_words};
+    const SeqView qv{q->d_packed, q->d_offsets, q->d_lengths, 0, q->n_words,
+                     bases_share(q->bases, n, q->count)};
+    const SeqView rv{r->d_packed, r->d_offsets, r->d_lengths, 0, r->n_words,
+                     bases_share(r->bases, n, r->count)};
     return wfa_cigar_run(c, qv, rv, ql.data(), rl.data(), q->max_len, r->max_len, cfg, n, cost,
                          runs, runs_cap, run_offsets, flags);
 }
