@@ -65,8 +65,11 @@ int exec_init(Exec &x)
 {
     bool ok = cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&x.ev_fork, cudaEventDisableTiming) == cudaSuccess;
+    int least = 0, greatest = 0;
+    ok = ok && cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess;
     for (int i = 0; ok && i < kAux; ++i)
-        ok = cudaStreamCreateWithFlags(&x.aux[i], cudaStreamNonBlocking) == cudaSuccess &&
+        ok = cudaStreamCreateWithPriority(&x.aux[i], cudaStreamNonBlocking,
+                                          i < kAuxFirst ? greatest : least) == cudaSuccess &&
              cudaEventCreateWithFlags(&x.ev_join[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok)
         cudaGetLastError();
@@ -518,7 +521,6 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
     memset(lut.v, kNoSplit, sizeof lut.v);
     bool present[kSplitShapes][6] = {};
     int32_t seg_low[kSplitShapes][6] = {}, seg_high[kSplitShapes][6] = {};
-    bool all_split = split && b_hi <= kSplitMaxBand;  // no pair needs an int32 or literal kernel
     // One thread per pair for the short pairs of a uniform band only: beside other bands
     // its launch would wait for, or hold up, the lane-split one.
     bool narrow = pack && (pi.uniform_band || !split);
@@ -554,8 +556,6 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
             present[ch.shape][ch.lg] = true;
             seg_low[ch.shape][ch.lg] = low;
             seg_high[ch.shape][ch.lg] = any_score ? high : -1;
-            if (long_scores && !any_score)
-                all_split = false;
             if (pi.uniform_band && (b == 16 || b == 32) && !narrow_wins(b, ch))
                 narrow = false;
         }
@@ -571,65 +571,59 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
     static const int cls_band[kSwSplit0] = {16, 32, 64, 128, 0, 16 | kPack16, 32 | kPack16};
     static_assert(kSwClasses * kCounterStride * 4 <= (int)kCounterBytes, "counter space");
     bool need[kSwSplit0] = {};
+    // a band some of whose pairs the lane-split kernel does not take
+    const auto left = [&](int32_t b) {
+        return !split || b > kSplitMaxBand || (long_scores && !(lut.v[b] & kSplitLong));
+    };
     for (int k = 0; k < 4; ++k)
-        need[k] = fast && !all_split && cls_band[k] >= b_lo && cls_band[k] <= b_hi;
-    need[4] = !all_split;
+        need[k] = fast && cls_band[k] >= b_lo && cls_band[k] <= b_hi && left(cls_band[k]);
+    for (int32_t b = b_lo; b <= std::min(b_hi, kSplitMaxBand + 1) && !need[4]; ++b)
+        need[4] = left(b) && !(fast && lengths_ok && classify_band(b) > 0);
     need[5] = narrow && b_lo <= 16 && b_hi >= 16;
     need[6] = narrow && b_lo <= 32 && b_hi >= 32;
     if (pi.uniform_band) {
         // when the batch's longest sequences qualify, every pair lands in one class
-        const int cb = classify_band(cfg->band_width);
         if ((need[5] || need[6]) && pack_lengths) {
             for (int k = 0; k < 5; ++k)
                 need[k] = false;
             memset(present, 0, sizeof present);
         }
-        if (fast && cb > 0 && lengths_ok)
-            need[4] = false;
     }
     if (need[4] && (rc = ensure_lit()))
         return rc;
     CU(c, cudaEventRecord(x.ev_fork, x.st));
-    int used = 0;
     cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
-    auto next_stream = [&](cudaStream_t &s) -> int {
-        s = x.aux[used % kAux];
+    bool used[kAux] = {};
+    int at = 0;  // the launch's stream
+    auto next_stream = [&](int i, cudaStream_t &s) -> int {
+        at = i;
+        s = x.aux[at];
         CU(c, cudaStreamWaitEvent(s, x.ev_fork, 0));
         return GB2_OK;
     };
     auto launched = [&](cudaStream_t s) -> int {
-        CU(c, cudaEventRecord(x.ev_join[used % kAux], s));
-        ++used;
+        CU(c, cudaEventRecord(x.ev_join[at], s));
+        used[at] = true;
         c->launches += 1;
         return GB2_OK;
     };
     cudaStream_t s;
-    for (int shape = kSplitShapes - 1; shape >= 0; --shape) {
-        SplitWork w{};
-        for (int lg = 5; lg >= 0; --lg) {
-            if (!present[shape][lg])
-                continue;
-            const int k = kSwSplit0 + shape * 6 + lg, i = w.count++;
-            w.lg[i] = lg;
-            w.low[i] = seg_low[shape][lg];
-            w.high[i] = seg_high[shape][lg];
-            w.list[i] = PairList{(const int32_t *)x.queue.p, 0, (const int64_t *)x.seg.p + 2 * k,
-                                 (int *)x.counters.p + kCounterStride * k};
-        }
-        if (w.count == 0)
-            continue;
-        if ((rc = next_stream(s)))
-            return rc;
-        // for the segment with the most lanes per pair
-        const int grid = split_grid(false, shape, w.lg[0], n, c->sm_count);
-        CU(c, launch_split(false, shape, qv, rv, p, cfg->band_width, d_bands, w, d_out, grid, s));
-        if ((rc = launched(s)))
-            return rc;
-    }
-    for (int k = 0; k < kSwSplit0; ++k) {
+    bool splits = false, others = false;
+    for (const auto &of_shape : present)
+        for (bool b : of_shape)
+            splits |= b;
+    for (bool b : need)
+        others |= b;
+    // The int32 and literal kernels go first, on the streams of higher priority: beside the
+    // lane-split one they hold the pairs of the highest scores, at the most time per row.
+    // (6,000 pairs of 100-2,000 bp, band 128, +5/-4/-10/-1: 2.15-3.5 ms when the lane-split
+    // kernel takes the SMs first, 1.55 after them.)
+    for (int i = 0, nth = 0; i < kSwSplit0; ++i) {
+        static const int order[kSwSplit0] = {4, 3, 2, 1, 0, 5, 6};
+        const int k = order[i];
         if (!need[k])
             continue;
-        if ((rc = next_stream(s)))
+        if ((rc = next_stream(nth++ % (splits ? kAux - 1 : kAux), s)))
             return rc;
         PairList pl{(const int32_t *)x.queue.p, 0, (const int64_t *)x.seg.p + 2 * k,
                     (int *)x.counters.p + kCounterStride * k};
@@ -647,8 +641,31 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
         if ((rc = launched(s)))
             return rc;
     }
-    for (int i = 0; i < std::min(used, kAux); ++i)
-        CU(c, cudaStreamWaitEvent(x.st, x.ev_join[i], 0));
+    for (int shape = kSplitShapes - 1, nth = 0; shape >= 0; --shape) {
+        SplitWork w{};
+        for (int lg = 5; lg >= 0; --lg) {
+            if (!present[shape][lg])
+                continue;
+            const int k = kSwSplit0 + shape * 6 + lg, i = w.count++;
+            w.lg[i] = lg;
+            w.low[i] = seg_low[shape][lg];
+            w.high[i] = seg_high[shape][lg];
+            w.list[i] = PairList{(const int32_t *)x.queue.p, 0, (const int64_t *)x.seg.p + 2 * k,
+                                 (int *)x.counters.p + kCounterStride * k};
+        }
+        if (w.count == 0)
+            continue;
+        if ((rc = next_stream(kAux - 1 - nth++ % (others ? kAux - kAuxFirst : kAux), s)))
+            return rc;
+        // for the segment with the most lanes per pair
+        const int grid = split_grid(false, shape, w.lg[0], n, c->sm_count);
+        CU(c, launch_split(false, shape, qv, rv, p, cfg->band_width, d_bands, w, d_out, grid, s));
+        if ((rc = launched(s)))
+            return rc;
+    }
+    for (int i = 0; i < kAux; ++i)
+        if (used[i])
+            CU(c, cudaStreamWaitEvent(x.st, x.ev_join[i], 0));
     prof_end(c, e0, x.st);
     return GB2_OK;
 }

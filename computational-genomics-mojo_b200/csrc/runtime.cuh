@@ -11,7 +11,8 @@
 
 namespace gb2 {
 
-constexpr int kAux = 4;            // auxiliary streams for concurrent band classes
+constexpr int kAux = 4;            // auxiliary streams for concurrent band classes,
+constexpr int kAuxFirst = 2;       // the first two of higher priority
 // 16, 32, 64, 128 (int32 registers), literal, packed 16, packed 32 (one thread per
 // pair), then the lane-split packed kernel: shape * 6 + log2(lanes)
 constexpr int kSwSplit0 = 7;

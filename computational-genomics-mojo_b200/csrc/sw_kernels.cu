@@ -552,7 +552,8 @@ sw_literal_kernel(SeqView q, SeqView r, SwParams p, int32_t band, const int32_t 
 {
     int64_t n;
     const int32_t *__restrict__ queue = pairs_resolve(pl, n);
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // few pairs: their warps spread over the blocks (each takes its own cache)
+    const int64_t tid = warp_rank() * 32 + (threadIdx.x & 31);
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
     int64_t *hp = scratch + tid * stride;
     for (int64_t slot = tid; slot < n; slot += nth) {
