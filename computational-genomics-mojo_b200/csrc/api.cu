@@ -479,22 +479,23 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
             cls |= kPack16;
         PairList pl{nullptr, n, nullptr, nullptr};
         int grid = 0;  // one pair per thread, pairs in input order
-        if (batched && cls > 0) {  // persistent blocks taking pairs from a counter
-            int rc;
-            if ((rc = ensure(c, x.counters, kCounterBytes, x.st)))
-                return rc;
-            CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
-            pl.counter = (int *)x.counters.p;
-            // no more blocks than pairs need: in a batch smaller than one wave the warps of
-            // the SMs that start first would otherwise take every pair (50,000 reads,
-            // band 32: 281 -> 193 us).  The packed kernel's warps then go by
-            // their place in the grid (40,000 reads, band 32: 134 -> 111 us).
+        if (cls > 0 && (batched || (cls & kPack16))) {
             const int64_t per = sw_pairs_per_block(cls, var_of(cls));
             const int64_t blocks = (int64_t)c->sm_count * sw_blocks_per_sm(cls, var_of(cls));
-            grid = (int)std::min(blocks, (n + per - 1) / per);
             if ((cls & kPack16) && n <= blocks * per) {
-                pl.counter = nullptr;
+                // less than one wave: the packed kernel's warps go by their place in the grid,
+                // one to an SM first (40,000 reads, band 32: 134 -> 111 us)
                 grid = (int)std::min(blocks, (n + 31) / 32);
+            } else if (batched) {
+                // persistent blocks taking pairs from a counter, no more of them than pairs
+                // need: the warps of the SMs that start first would otherwise take every pair
+                // (50,000 reads, band 32: 281 -> 193 us)
+                int rc;
+                if ((rc = ensure(c, x.counters, kCounterBytes, x.st)))
+                    return rc;
+                CU(c, cudaMemsetAsync(x.counters.p, 0, 64, x.st));
+                pl.counter = (int *)x.counters.p;
+                grid = (int)std::min(blocks, (n + per - 1) / per);
             }
         }
         cudaEvent_t e0 = profile ? prof_begin(c, x.st) : nullptr;
