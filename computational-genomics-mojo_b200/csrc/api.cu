@@ -776,13 +776,23 @@ static int wfa_block_warps(int64_t qmax, int64_t rmax, int64_t n, int variant)
 // The first tier: one warp per pair costs the least work, more warps the least time for
 // the longest pair.  What decides is how many pairs as long as the longest the batch
 // amounts to, by the square of the length (the mean over the longest to the power 1.5
-// estimates that).  Measured, 1 / 4 / 8 warps first (ms):
-//   100-10,000 bp, 300 pairs (30 such)  4.39 / 2.87 / 2.58;  4,000 (400) 6.26 / 4.56 / 4.48
-//   8,000 (800) 7.5 / 7.5 / 8.9;  12,000 (1,200) 8.9 / 10.4 / 13.2
-//   100-1,500 bp, 3,000 (610) 0.57 / 0.44 / 0.69;  8,000 (1,600) 0.73 / 0.95 / 1.62
-//   8,000-10,000 bp, 2,000 (1,700) 10.1 / 11.6 / 13.5
-// so one warp above 6 per SM, four above 2.7, else eight (a single pair, the per-call
-// drop-in: sixteen warps took 0.68 ms for 4,000 bp, eight 0.62).
+// estimates that).  Measured, 1 / 4 / 8 warps first (us, x4 o6 e2):
+//   1,000 bp, 12% divergence, 148 pairs  410 / 271 / 258;  300  394 / 294 / 409;
+//     600  468 / 465 / 603;  1,200  534 / 702 / 1,034
+//   250 bp, 3%, 100 pairs  49 / 50 / 51;  600  51 / 58 / 71;  2,500  63 / 118 / 177
+//   100-1,500 bp, 12%, 600 pairs (120 as long as the longest)  617 / 424 / 412;
+//     1,200 (240)  641 / 477 / 533;  2,500 (500)  679 / 599 / 994;  4,000 (810)  771 / 974
+//   500-8,000 bp, 12%, 600 pairs (118)  5,560 / 3,898 / 3,620
+//   4,000 bp, 3%, 600 pairs  586 / 540 / 689;  1,200  687 / 828 / 1,211
+//   100-3,000 bp, 8%, 5,000 pairs (760), with their CIGARs  3,040 / 2,820
+//   100-10,000 bp, 4,000 pairs (400)  6,260 / 4,560 / 4,480;  8,000 (800)  7,500 / 7,500
+// so one warp above 4 per SM (6 for sequences over 2,000 bases), four above 1.4, else eight
+// (a single pair, the per-call drop-in: sixteen warps took 0.68 ms for 4,000 bp, eight 0.62).
+//
+// Pairs of at most kWfaShortLen bases start on eight lanes each, but a pair's steps then
+// take longer: only from kWfaShortMinPairsPerSm per SM on, where the warps of the one-warp
+// tier are many rounds behind (one warp / eight lanes, us: 100-150 bp, 3%, 2,500 pairs
+// 59 / 96;  9,000  94 / 109;  14,000  106 / 123;  20,000  135 / 130;  40,000  204 / 154).
 static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t rmax,
                      const WfaParams &p, int64_t n, int32_t *d_out, int flags, int32_t *d_ub)
 {
@@ -798,7 +808,7 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     const double mean = std::max(mean_length(qv, n, (int64_t)longest),
                                  mean_length(rv, n, (int64_t)longest));
     const double alike = (double)n * std::pow(mean / longest, 1.5) / (double)sms;
-    int first = alike > 6.0 ? 0 : (alike > 2.7 ? 2 : 3);
+    int first = alike > (longest > 2000 ? 6.0 : 4.0) ? 0 : (alike > 1.4 ? 2 : 3);
     while (first < G && !pl.usable[first])
         ++first;
     auto next_of = [&](int t) {
@@ -817,9 +827,8 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         if (pl.usable[t] && reach + 4 <= pl.H[t] && reach + 6 + pl.H[t] <= pl.W[t] &&
             steps <= 32767 - std::max<int64_t>(qmax, pl.H[t] + 8))
             last = t;
-    // short pairs start on eight lanes each, when there are enough to fill the warps
-    const bool shorts = first == 0 && std::max(qmax, rmax) <= kWfaShortLen &&
-                        wfa_short_usable(pl);
+    const bool shorts = first == 0 && n >= kWfaShortMinPairsPerSm * sms &&
+                        std::max(qmax, rmax) <= kWfaShortLen && wfa_short_usable(pl);
     // dump records of the transitions out of each tier
     int64_t dcap[G] = {}, doff[G] = {}, dbytes = 0;
     for (int t = first; t < std::min(last, G); ++t) {

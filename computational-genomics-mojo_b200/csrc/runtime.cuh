@@ -40,6 +40,8 @@ constexpr int64_t kTierDumpCap = 1ll << 30;    // bytes of suspended-pair record
 constexpr int64_t kWfaBoundMinLen = 1024;
 // WFA: batches of fewer pairs per SM than this skip the two-warp tier
 constexpr int64_t kWfaTwoWarpMinPairsPerSm = 160;
+// WFA: batches of fewer pairs per SM than this start short pairs on the one-warp tier
+constexpr int64_t kWfaShortMinPairsPerSm = 100;
 constexpr int32_t kWfaBoundBand = 56;  // 113 diagonals and the lengths' difference: one round of a warp
 
 // Grow-only device buffer.

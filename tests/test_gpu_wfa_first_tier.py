@@ -1,0 +1,61 @@
+"""Where a WFA batch starts -- eight, four or one warp per pair, or eight lanes -- changes
+with the number of pairs as long as the longest: the same costs on both sides of each line,
+for even and ragged lengths, and batches between the lines of few launches."""
+import numpy as np
+import pytest
+
+from genomics_b200 import SequenceBatch, WFAConfig
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(rng, n, lo, hi):
+    qs, rs = [], []
+    for i in range(n):
+        t = rng.integers(0, 4, hi if i == 0 else int(rng.integers(lo, hi + 1)))
+        q = t.copy()
+        hit = rng.random(len(q)) < (0.02, 0.1, 1.0)[i % 3]
+        q[hit] = rng.integers(0, 4, int(hit.sum()))
+        cut = int(rng.integers(0, len(q)))
+        qs.append("".join("ACGT"[c] for c in np.delete(q, slice(cut, cut + i % 4))))
+        rs.append("".join("ACGT"[c] for c in t))
+    return SequenceBatch.from_strings(qs), SequenceBatch.from_strings(rs)
+
+
+def _copies(b, n):
+    """n sequences with words of their own: the batch's over and over."""
+    p, m, o, ln = b.arrays()
+    times = -(-n // len(ln))
+    offs = np.concatenate([o + k * p.size for k in range(times)])
+    return SequenceBatch.from_arrays(np.tile(p, times), np.tile(m, times), offs[:n],
+                                     np.tile(ln, times)[:n])
+
+
+@pytest.mark.parametrize("lo,hi", [(150, 150), (1, 512), (300, 700)])
+@pytest.mark.parametrize("per_sm", [1.4, 4.0, 100.0])
+def test_costs_on_both_sides_of_a_line(device, oracle, lo, hi, per_sm):
+    rng = np.random.default_rng(lo + hi)
+    q, r = _pairs(rng, 60, lo, hi)
+    qp, _, qo, ql = q.arrays()
+    rp, _, ro, rl = r.arrays()
+    cfg = WFAConfig(4, 6, 2, 900)
+    want, _ = oracle.wfa_batch(qp, qo, ql, rp, ro, rl, 4, 6, 2, 900, envelope=True)
+    alike = (np.mean(rl) / rl.max()) ** 1.5 if per_sm < 100 else 1.0
+    line = int(148 * per_sm / alike)
+    for n in (line - 3, line + 3):
+        got = device.wfa_affine(_copies(q, n), _copies(r, n), cfg)
+        assert (got == np.resize(want, n)).all(), n
+
+
+def test_a_small_batch_of_reads_starts_on_one_warp_per_pair(device):
+    """2,500 reads: one launch, without the eight-lane kernel and its second one."""
+    rng = np.random.default_rng(1)
+    q, r = _pairs(rng, 60, 150, 150)
+    dq, dr = device.upload_batch(_copies(q, 2500)), device.upload_batch(_copies(r, 2500))
+    try:
+        device.stats_reset()
+        device.wfa_affine(dq, dr, WFAConfig(4, 6, 2, 100), batched=False)
+        assert device.stats()["launches"] == 1
+    finally:
+        dq.close()
+        dr.close()
