@@ -697,10 +697,11 @@ cudaError_t launch_sw_naive(SeqView q, SeqView r, SwParams p, int32_t band, cons
         return cudaSuccess;
     if (n > 0x7fffffff || max_band > kSwNaiveMaxBand)
         return cudaErrorInvalidValue;
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        sw_naive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        (int)(2 * (2 * kSwNaiveMaxBand + 1) * sizeof(int32_t)));
-    (void)attr;
+    static std::atomic<uint64_t> done{0};
+    const cudaError_t attr = allow_smem(
+        sw_naive_kernel, (int)(2 * (2 * kSwNaiveMaxBand + 1) * sizeof(int32_t)), done);
+    if (attr != cudaSuccess)
+        return attr;
     const size_t smem = (size_t)2 * (2 * (size_t)max_band + 1) * sizeof(int32_t);
     sw_naive_kernel<<<(unsigned)n, 128, smem, st>>>(q, r, p, band, bands, n, out);
     return cudaGetLastError();

@@ -780,21 +780,20 @@ int wfa_cigar_blocks_per_sm()
 
 static size_t wfa_smem_bytes(int bw) { return (size_t)bw * 4 * kWfaSeqWords * 4; }
 
-// One-time opt-in to the kernel's dynamic shared memory (above 48 KB for BW = 16).
+// Opt-in to the kernel's dynamic shared memory (above 48 KB for BW = 16).
 template <int U, int BW>
-static void wfa_prepare()
+static cudaError_t wfa_prepare()
 {
-    static const cudaError_t e = cudaFuncSetAttribute(
-        wfa_kernel<U, BW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wfa_smem_bytes(BW));
-    (void)e;
+    static std::atomic<uint64_t> done{0};
+    return allow_smem(wfa_kernel<U, BW>, (int)wfa_smem_bytes(BW), done);
 }
 
 template <int U, int BW>
 static int wfa_occupancy()
 {
-    wfa_prepare<U, BW>();
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wfa_kernel<U, BW>, 32 * BW,
+    if (wfa_prepare<U, BW>() != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wfa_kernel<U, BW>, 32 * BW,
                                                       wfa_smem_bytes(BW)) != cudaSuccess) {
         cudaGetLastError();
         return BW == 4 ? 4 : 1;
@@ -821,25 +820,20 @@ cudaError_t launch_wfa(int variant, int block_warps, SeqView q, SeqView r, WfaPa
     // block_warps kWfaWideWarps: the wide kernel (4 diagonals per thread per
     // round); otherwise variant bits 4-5: diagonals per thread per round 4
     // (default), 2 or 1
-    if (block_warps == kWfaWideWarps) {
-        wfa_prepare<4, kWfaWideWarps>();
-        wfa_kernel<4, kWfaWideWarps><<<grid, 32 * kWfaWideWarps, wfa_smem_bytes(kWfaWideWarps),
-                                       st>>>(q, r, p, longs, shorts, out, scratch, slot_width,
-                                             err_flag, work);
-    } else if (variant & 0x20) {
-        wfa_prepare<1, 4>();
-        wfa_kernel<1, 4><<<grid, 128, wfa_smem_bytes(4), st>>>(
-            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work);
-    } else if (variant & 0x10) {
-        wfa_prepare<2, 4>();
-        wfa_kernel<2, 4><<<grid, 128, wfa_smem_bytes(4), st>>>(
-            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work);
-    } else {
-        wfa_prepare<4, 4>();
-        wfa_kernel<4, 4><<<grid, 128, wfa_smem_bytes(4), st>>>(
-            q, r, p, longs, shorts, out, scratch, slot_width, err_flag, work);
-    }
-    return cudaGetLastError();
+    const auto go = [&](cudaError_t prepared, auto kern, int bw) {
+        if (prepared != cudaSuccess)
+            return prepared;
+        kern<<<grid, 32 * bw, wfa_smem_bytes(bw), st>>>(q, r, p, longs, shorts, out, scratch,
+                                                        slot_width, err_flag, work);
+        return cudaGetLastError();
+    };
+    if (block_warps == kWfaWideWarps)
+        return go(wfa_prepare<4, kWfaWideWarps>(), wfa_kernel<4, kWfaWideWarps>, kWfaWideWarps);
+    if (variant & 0x20)
+        return go(wfa_prepare<1, 4>(), wfa_kernel<1, 4>, 4);
+    if (variant & 0x10)
+        return go(wfa_prepare<2, 4>(), wfa_kernel<2, 4>, 4);
+    return go(wfa_prepare<4, 4>(), wfa_kernel<4, 4>, 4);
 }
 
 // ---- integer throughput probe -------------------------------------------------
