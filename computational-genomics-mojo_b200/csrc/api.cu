@@ -829,6 +829,9 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
             last = t;
     const bool shorts = first == 0 && n >= kWfaShortMinPairsPerSm * sms &&
                         std::max(qmax, rmax) <= kWfaShortLen && wfa_short_usable(pl);
+    if (last == G && 2 * std::max(qmax, rmax) + 16 > INT32_MAX)
+        return set_err(c, GB2_ENOMEM, "no rings for a WFA sequence of %lld bases",
+                       (long long)std::max(qmax, rmax));
     // dump records of the transitions out of each tier
     int64_t dcap[G] = {}, doff[G] = {}, dbytes = 0;
     for (int t = first; t < std::min(last, G); ++t) {
@@ -842,7 +845,7 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     if ((rc = ensure(c, x.tierq, (size_t)n * 8 * (G + 1), x.st)) ||
         (rc = ensure(c, x.dumps, (size_t)std::max<int64_t>(dbytes, 256), x.st)) ||
         (last == G &&
-         (rc = ensure(c, x.scratch32, (size_t)(sms * pl.gring_block_bytes), x.st))) ||
+         (rc = ensure(c, x.scratch32, (size_t)wfa_gring_bytes(pl, n, sms), x.st))) ||
         (rc = ensure(c, x.counters, kCounterBytes, x.st)))
         return rc;
     CU(c, cudaMemsetAsync(x.counters.p, 0, kCounterBytes, x.st));
@@ -928,7 +931,9 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
         io.ubound = (d_ub && t > 0) ? d_ub : nullptr;
         // a team's first pair is the one of its place in the grid: as many blocks as there
         // are pairs spread a small batch over the SMs
-        const int grid = (int)(t == first ? std::min<int64_t>(sms, n) : sms);
+        const int grid = (int)(t == G       ? wfa_gring_blocks(pl, n, sms)
+                               : t == first ? std::min<int64_t>(sms, n)
+                                            : sms);
         cudaEvent_t e0 = prof_begin(c, x.st);
         CU(c, launch_wfa_tier(pl, t, grid, qv, rv, p, io, d_out, wfa_work(x),
                               (int *)x.errflag.p, x.st));

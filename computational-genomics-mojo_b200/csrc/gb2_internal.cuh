@@ -203,6 +203,18 @@ struct WfaTierPlan {
     int64_t gring_block_bytes; // G tier ring region of one block
 };
 WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax);
+// Blocks of the G tier for n pairs: no more than pairs, nor than kWfaGringCap bytes of rings
+// (one always; a pair of 20,000,000 bases takes 1.6 GB).
+constexpr int64_t kWfaGringCap = 64ll << 30;
+inline int64_t wfa_gring_blocks(const WfaTierPlan &pl, int64_t n, int64_t sm_count)
+{
+    const int64_t fit = kWfaGringCap / pl.gring_block_bytes, want = n < sm_count ? n : sm_count;
+    return fit < 1 ? 1 : fit < want ? fit : want;
+}
+inline int64_t wfa_gring_bytes(const WfaTierPlan &pl, int64_t n, int64_t sm_count)
+{
+    return wfa_gring_blocks(pl, n, sm_count) * pl.gring_block_bytes;
+}
 
 // Inputs and outputs of one tier launch.  Input: list (int32 pair indices,
 // nullptr = 0..n-1) or ents ({pair, dump record or -1}); n, or *n_dev when set,

@@ -732,11 +732,12 @@ __device__ __forceinline__ int32_t tier_pair32(const SeqView &q, const SeqView &
     team.sync();  // the previous pair's reads of the shared copies and the ring are done
     const SeqWin qs = stage_seq<SMEM_SEQ>(q, qoff, qnw, sq, tt, TW, 0u);
     const SeqWin rs = stage_seq<SMEM_SEQ>(r, roff, rnw, sr, tt, TW, 0xFFFFFFFFu);
-    for (int32_t i = tt; i < (w.nslot + 1) * W; i += TW)  // the slots and the NEG row
+    // the slots and the NEG row; more than 2^31 elements for sequences of some 10^8 bases
+    for (int64_t i = tt; i < (int64_t)(w.nslot + 1) * W; i += TW)
         ring[i] = NEG;
     const int32_t target = qlen - rlen;
     RT *const base = ring + H;
-    auto slot = [&](int j) { return base + j * W; };
+    auto slot = [&](int j) { return base + (int64_t)j * W; };
     // per-slot intervals: lane j holds M slot j's and I/D slot j's
     int32_t mlo = 1, mhi = 0, ilo = 1, ihi = 0;
     int ms = 0, is = 0;
