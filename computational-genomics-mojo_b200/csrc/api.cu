@@ -578,7 +578,8 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
     };
     for (int k = 0; k < 4; ++k)
         need[k] = fast && cls_band[k] >= b_lo && cls_band[k] <= b_hi && left(cls_band[k]);
-    for (int32_t b = b_lo; b <= std::min(b_hi, kSplitMaxBand + 1) && !need[4]; ++b)
+    need[4] = b_hi > kSplitMaxBand;
+    for (int32_t b = b_lo; b <= std::min(b_hi, kSplitMaxBand) && !need[4]; ++b)
         need[4] = left(b) && !(fast && lengths_ok && classify_band(b) > 0);
     need[5] = narrow && b_lo <= 16 && b_hi >= 16;
     need[6] = narrow && b_lo <= 32 && b_hi >= 32;

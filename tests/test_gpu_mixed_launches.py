@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from genomics_b200 import AlignConfig, SequenceBatch
+from genomics_b200._lib import FLAG_INT32
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +49,24 @@ def test_launches_beside_the_lane_split_kernel(device, oracle, pairs, top, only,
     finally:
         dq.close()
         dr.close()
+
+
+@pytest.mark.parametrize("band", [16, 64, 65, 128, 543, 544, 600])
+@pytest.mark.parametrize("scores", [SCORES, (2, -4, -4, -2), (1, -8, -2, -1)])
+def test_one_band_of_ragged_pairs(device, oracle, pairs, band, scores):
+    """Every pair is taken by some kernel: bands on both sides of the lane-split kernel's
+    widest, scores inside and past its range, and a scoring that no packed kernel takes."""
+    q, r = pairs
+    qp, _, qo, ql = q.arrays()
+    rp, _, ro, rl = r.arrays()
+    want = np.stack(oracle.sw_batch(qp, qo, ql, rp, ro, rl, *scores, band), 1)
+    out = np.full(24 * 3, -77, np.int32).view([("score", "<i4"), ("query_end", "<i4"),
+                                               ("ref_end", "<i4")])
+    for flags in (0, FLAG_INT32):
+        for batched in (True, False):
+            dq, dr = device.upload_batch(q), device.upload_batch(r)
+            got = device.sw_banded(dq, dr, AlignConfig(*scores, band), batched=batched,
+                                   flags=flags, out=out)
+            assert (got.view(np.int32).reshape(-1, 3) == want).all(), (band, flags, batched)
+            dq.close()
+            dr.close()
