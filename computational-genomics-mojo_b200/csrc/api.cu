@@ -787,8 +787,15 @@ static int wfa_block_warps(int64_t qmax, int64_t rmax, int64_t n, int variant)
 //   4,000 bp, 3%, 600 pairs  586 / 540 / 689;  1,200  687 / 828 / 1,211
 //   100-3,000 bp, 8%, 5,000 pairs (760), with their CIGARs  3,040 / 2,820
 //   100-10,000 bp, 4,000 pairs (400)  6,260 / 4,560 / 4,480;  8,000 (800)  7,500 / 7,500
-// so one warp above 4 per SM (6 for sequences over 2,000 bases), four above 1.4, else eight
-// (a single pair, the per-call drop-in: sixteen warps took 0.68 ms for 4,000 bp, eight 0.62).
+// so one warp above 4 per SM (6 for sequences over 2,000 bases, or longer than that tier's
+// shared copy), four above 1.4, else eight (a single pair, the per-call drop-in: sixteen
+// warps took 0.68 ms for 4,000 bp, eight 0.62).
+// Pairs that max_error stops after as many steps are alike however long they are: lengths
+// count up to four bases per step.
+//   100-3,000 bp, 12%, max_error 400 (200 steps), 600 pairs  217 / 203 / 319;
+//     1,200  245 / 343 / 507;  5,000  503 / 996 / 1,820
+//   3,000 bp, 12%, max_error 200, 600 pairs  101 / 173 / 250
+//   500-10,000 bp, 12%, max_error 1,000, 600 pairs  974 / 498 / 823
 //
 // Pairs of at most kWfaShortLen bases start on eight lanes each, but a pair's steps then
 // take longer: only from kWfaShortMinPairsPerSm per SM on, where the warps of the one-warp
@@ -805,11 +812,13 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     if (n < kWfaTwoWarpMinPairsPerSm * sms)
         pl.usable[1] = false;
     constexpr int G = kWfaShared;  // the global-memory tier
-    const double longest = (double)std::max<int64_t>({qmax, rmax, 1});
-    const double mean = std::max(mean_length(qv, n, (int64_t)longest),
-                                 mean_length(rv, n, (int64_t)longest));
-    const double alike = (double)n * std::pow(mean / longest, 1.5) / (double)sms;
-    int first = alike > (longest > 2000 ? 6.0 : 4.0) ? 0 : (alike > 1.4 ? 2 : 3);
+    const int64_t steps = p.max_error / gcd_h(p.x, gcd_h(p.o, p.e));
+    const int64_t lmax = std::max<int64_t>({qmax, rmax, 1});
+    const int64_t longest = std::min(lmax, std::max<int64_t>(4 * steps, 1));
+    const double mean = std::max(mean_length(qv, n, longest), mean_length(rv, n, longest));
+    const double alike = (double)n * std::pow(mean / (double)longest, 1.5) / (double)sms;
+    const double one_warp = longest > 2000 || lmax > kWfaOneWarpCopy ? 6.0 : 4.0;
+    int first = alike > one_warp ? 0 : (alike > 1.4 ? 2 : 3);
     while (first < G && !pl.usable[first])
         ++first;
     auto next_of = [&](int t) {
@@ -821,7 +830,6 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     // The last tier that can get pairs: a diagonal is at most as far out as the longer
     // sequence is long and as there are steps, and a tier whose window holds that, for
     // steps that int16 rows are proven for, passes nothing on.
-    const int64_t steps = p.max_error / gcd_h(p.x, gcd_h(p.o, p.e));
     const int64_t reach = std::min(std::max(qmax, rmax), steps);
     int last = G;
     for (int t = G - 1; t >= first; --t)

@@ -248,6 +248,7 @@ struct WfaTierIo {
 // Short pairs, eight lanes each (before tier 0): whether the penalties' rows leave a
 // window, and the launch (list or seg, n, ctr in; next out).
 constexpr int32_t kWfaShortLen = 512;
+constexpr int32_t kWfaOneWarpCopy = 6144;  // bases of a sequence the one-warp tier copies
 bool wfa_short_usable(const WfaTierPlan &pl);
 cudaError_t launch_wfa_short(const WfaTierPlan &pl, int sm_count, SeqView q, SeqView r, WfaParams p,
                              const WfaTierIo &io, int32_t *out, int64_t *work, cudaStream_t st);

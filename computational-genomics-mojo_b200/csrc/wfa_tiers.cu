@@ -1245,7 +1245,7 @@ struct TierSpec {
     int32_t seq_bases;  // longest sequence copied to shared memory
 };
 // S, M, L tiers
-static const TierSpec kTiers[kWfaShared] = {{1, 16, 6144}, {2, 8, 12288}, {4, 4, 16384}, {8, 2, 32768}, {16, 1, 32768}};
+static const TierSpec kTiers[kWfaShared] = {{1, 16, kWfaOneWarpCopy}, {2, 8, 12288}, {4, 4, 16384}, {8, 2, 32768}, {16, 1, 32768}};
 
 WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax)
 {

@@ -47,6 +47,37 @@ def test_costs_on_both_sides_of_a_line(device, oracle, lo, hi, per_sm):
         assert (got == np.resize(want, n)).all(), n
 
 
+def test_lengths_count_no_further_than_max_error_lets_them(device, oracle):
+    """1,200 pairs of 100-3,000 bases, few of them long: with a small max_error they are as
+    good as alike, and one warp per pair is all that is launched."""
+    rng = np.random.default_rng(3)
+    qs, rs = [], []
+    for i in range(60):
+        t = rng.integers(0, 4, int(100 * 30 ** (i / 59)))
+        q = t.copy()
+        hit = rng.random(len(q)) < 0.1
+        q[hit] = rng.integers(0, 4, int(hit.sum()))
+        qs.append("".join("ACGT"[c] for c in q))
+        rs.append("".join("ACGT"[c] for c in t))
+    q, r = SequenceBatch.from_strings(qs), SequenceBatch.from_strings(rs)
+    qp, _, qo, ql = q.arrays()
+    rp, _, ro, rl = r.arrays()
+    want, _ = oracle.wfa_batch(qp, qo, ql, rp, ro, rl, 4, 6, 2, 200, envelope=True)
+    seen = set()
+    for batched in (True, False):
+        dq, dr = device.upload_batch(_copies(q, 1200)), device.upload_batch(_copies(r, 1200))
+        try:
+            device.stats_reset()
+            got = device.wfa_affine(dq, dr, WFAConfig(4, 6, 2, 200), batched=batched)
+            assert (got == np.resize(want, 1200)).all()
+            seen.add((batched, device.stats()["launches"]))
+        finally:
+            dq.close()
+            dr.close()
+    # (three kernels order a batched call's pairs)
+    assert seen == {(True, 4), (False, 1)}, seen
+
+
 def test_a_small_batch_of_reads_starts_on_one_warp_per_pair(device):
     """2,500 reads: one launch, without the eight-lane kernel and its second one."""
     rng = np.random.default_rng(1)
