@@ -619,7 +619,7 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
     // The int32 and literal kernels go first, on the streams of higher priority: beside the
     // lane-split one they hold the pairs of the highest scores, at the most time per row.
     // (6,000 pairs of 100-2,000 bp, band 128, +5/-4/-10/-1: 2.15-3.5 ms when the lane-split
-    // kernel takes the SMs first, 1.55 after them.)
+    // kernel takes the SMs first, 1.3 after them.)
     for (int i = 0, nth = 0; i < kSwSplit0; ++i) {
         static const int order[kSwSplit0] = {4, 3, 2, 1, 0, 5, 6};
         const int k = order[i];
