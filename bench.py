@@ -59,8 +59,7 @@ SW_OPS_PER_CELL_PACKED = 5.5  # the same ops on int16x2 lanes: two cells per lan
 # per pair; a step runs as 4 launches of 250,000 pairs.
 SW_PACKED_TRAFFIC_BYTES = 128.3e6
 SW_PACKED_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum of one "
-                            "65,536-pair launch of sw_pack16_kernel<32>, per pair, x 1,000,000 "
-                            "(profiles/sw_pack16_kernel_b32_1M_reads.md)")
+                            "65,536-pair launch of sw_pack16_kernel<32>, per pair, x 1,000,000")
 
 
 def parse():

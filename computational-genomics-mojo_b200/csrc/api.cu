@@ -527,8 +527,8 @@ int sw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, int64_t r
     bool narrow = pack && (pi.uniform_band || !split);
     if (split) {
         // Per-pair bands run as one launch, so that its warps can take the longest pair
-        // of any band next: the shape with the least time summed over the register
-        // kernels' bands (the host does not know which bands the pairs have).
+        // of any band next: the shape with the least time summed over bands 16, 32, 64, 128
+        // and the widest, an assumed mix (which bands the pairs have is not counted).
         int shape = -1;
         if (!pi.uniform_band) {
             double least = 0;
@@ -2129,7 +2129,7 @@ static int gb2_sw_pair_impl(gb2_ctx *c, const uint64_t *q_words, int64_t qlen, c
         int rc;
         if ((rc = sw_validate(c, cfg, nullptr, 1, qlen, rlen, pi)))
             return rc;
-        pi.narrow_lengths = narrow_range(qlen, qlen) && narrow_range(rlen, rlen);
+        pi.narrow_lengths = true;  // one pair
         if ((rc = ensure(c, c->out_sw, sizeof(gb2_sw_result), c->x.st)) ||
             (rc = pair_upload(c, q_words, qlen, r_words, rlen, qv, rv)) ||
             (rc = sw_core(c, c->x, qv, rv, qlen, rlen, cfg, nullptr, pi, 1,

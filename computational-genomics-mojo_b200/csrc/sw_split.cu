@@ -637,8 +637,8 @@ bool split_rebase(const SwParams &p, int shape, int lg, int32_t *low, int32_t *h
 
 // Fitted to 400,000 reads (150 vs 200 bp, band 33: 125, 181, 220, 286, 324, 388, 434, 500
 // cycles per warp and row for the shapes in order; Needleman-Wunsch 7.1 R + 74) and to
-// 150-600 pairs of 3-9 kbp, one warp per scheduler (244, 318, 381, 464, 524, 606, 676,
-// 785).  `rows`: rows a warp runs beside those of its pairs.
+// 150-600 Smith-Waterman pairs of 3-9 kbp, one warp per scheduler (244, 318, 381, 464, 524,
+// 606, 676, 785; Needleman-Wunsch is priced with the same, its own chain not measured).  `rows`: rows a warp runs beside those of its pairs.
 // Pairs of one length run in rounds of four warps per scheduler, the last round as long
 // as its fullest scheduler (150 bp, band 32: 20,000 pairs R = 9, 17, one thread per pair
 // 97, 81, 79 us; 40,000: 155, 146, 111).  Of ragged pairs the longest come first: the

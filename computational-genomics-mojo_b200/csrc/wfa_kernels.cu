@@ -243,8 +243,8 @@ __device__ __forceinline__ int32_t wfa_align_pair(const SeqView &q, const SeqVie
     // optimal alignments, whose prefixes all stay inside, so their values, and the values
     // of every source that ties with the one taken, are those of the whole wavefront.
     const int32_t known = HREC ? (hsteps - 1) * w.g : 0;
-    // through a shuffle: the assembler of CUDA 12.9 otherwise merges
-    // max(max(lo, -max_err), target - R) below into a 3-way maximum of +max_err
+    // through a shuffle: with -max_err in max(max(lo, -max_err), target - R) below, a build
+    // with CUDA 12.9 was seen to clip the low side at +max_err
     const int32_t neg_err = __shfl_sync(FULL, -max_err, 0);
     const int64_t qoff = q.offsets[pi] - q.word_base;
     const int64_t roff = r.offsets[pi] - r.word_base;

@@ -48,10 +48,10 @@
 // any position is two neighbouring words and one funnel shift; pairs longer than a
 // tier's copy capacity read their windows from the packed words in global memory.
 //
-// Bound: instruction issue.  Per warp and step about 100 instructions of bookkeeping,
-// 139 per round of four diagonals a lane (82 of two) of which the extension's two window
-// loads, shifts, compare and clamps are 80, and about 100 for the lanes whose whole first
-// window matched.  At the sizes above T1 issues 69% of its slots, T4 62%.
+// Bound: instruction issue: 77 thread instructions per cell, most of them the extension's
+// two window loads, shifts, compare and clamps and a step's bookkeeping.  20,000 pairs of
+// 100-10,000 bp (2.7e9 cells, by counters): T1 2.5 ms at 71% of the issue slots, the bound
+// pass 2.0 at 64%, T4 5.9 at 63%, sixteen warps per SM each.
 #include <algorithm>
 #include <type_traits>
 
@@ -514,8 +514,8 @@ __device__ __forceinline__ int32_t tier_pair16(
     const int32_t tc = cut(target);
     const uint32_t lim_matrix = pack2(-min(rlen, kFar), -min(qlen, kFar));
     const uint32_t lim_target = pack2(tc, -tc);
-    // (through a shuffle: the assembler of CUDA 12.9 can lose the sign of a negated kernel
-    // argument when it merges maxima into a 3-way one)
+    // (through a shuffle: where maxima met a negated kernel argument, a build with CUDA 12.9
+    // was seen to clip at +max_err)
     int32_t flo = __shfl_sync(FULL, -min(max_err, kFar), 0), fnhi = flo;
     if (band_w > 0) {
         flo = max(flo, cut(min(0, target) - band_w));

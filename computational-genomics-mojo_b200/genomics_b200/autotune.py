@@ -6,7 +6,9 @@ at 3-5 resident blocks per SM; every shape computes the same results.  `tune`
 times each shape on a sample of the caller's own pairs, installs the fastest
 in the device's context, and returns the table; `save` / `load` keep it in a
 JSON file so a service tunes once per machine and restores the table at
-start-up.
+start-up.  The table applies to calls that run these kernels: for
+Smith-Waterman FLAG_INT32, and scores or pairs past what the packed kernels
+take; for WFA FLAG_NAIVE.  Other calls choose their kernels by themselves.
 """
 from __future__ import annotations
 

@@ -366,7 +366,12 @@ int gb2_server_stop(gb2_server *srv);
  * GB2_TUNE_WFA: the batched WFA kernel), `reps` timed runs each after one
  * warm-up, checks that every candidate gives the first candidate's results
  * (GB2_EKERNEL otherwise), and installs the fastest in the context: later calls
- * whose flags leave the variant field (bits 8-15) at 0 use it.  Tune on the
+ * whose flags leave the variant field (bits 8-15) at 0 use it where they run that
+ * kernel.  Since the packed kernels take every band to 543, a Smith-Waterman call
+ * runs the int32 kernels only with GB2_FLAG_INT32, with scores the packed kernels
+ * cannot take (mismatch < gap_open + gap_extend, terms over 255), or for pairs whose
+ * scores pass the packed kernels' range; a WFA call runs the single kernel only with
+ * GB2_FLAG_NAIVE or a variant.  The table changes no other call.  Tune on the
  * batch size that will run: a small batch that leaves SMs idle favours more
  * lanes per pair than a full one.  bands (GB2_TUNE_SW, optional, host): the
  * per-pair bands of a mixed batch; each candidate of the class then runs inside
