@@ -1239,6 +1239,7 @@ wfa_short_kernel(SeqView q, SeqView r, WfaParams p, TierIn in, int2 *next, int *
 // Shared memory of one block (the device maximum per block, less a margin for
 // the kernel's static shared variables).
 constexpr int64_t kTierBlockSmem = 227 * 1024 - 256;
+constexpr int64_t kTierMinWindow = 64;  // diagonals
 
 struct TierSpec {
     int team_warps, nteams;
@@ -1265,16 +1266,25 @@ WfaTierPlan wfa_tier_plan(const WfaParams &p, int64_t qmax, int64_t rmax)
     for (int t = 0; t < kWfaShared; ++t) {
         const TierSpec &s = kTiers[t];
         const int64_t team_bytes = kTierBlockSmem / s.nteams;
-        const int64_t seq_entries = 2 * ((s.seq_bases + 31) / 32) + 2;  // and the guard
-        const int64_t seq_bytes = 2 * seq_entries * 4;
-        int64_t W = (team_bytes - seq_bytes) / (nslot * 2);
+        int64_t seq_entries = 2 * ((s.seq_bases + 31) / 32) + 2;  // and the guard
+        int64_t W = (team_bytes - 2 * seq_entries * 4) / (nslot * 2);
         W = W / 8 * 8;  // 16-byte rows: the NEG fill uses 16-byte stores
+        // Many slots (up to 96) leave the one-warp tier less than 64 diagonals: it keeps 64
+        // and copies shorter sequences (x1 o0 e31, 400,000 pairs of 100 bp: 126 ms without
+        // that tier, 96 so).
+        if (W < kTierMinWindow && team_bytes > kTierMinWindow * nslot * 2) {
+            const int64_t words = (team_bytes - kTierMinWindow * nslot * 2) / 8 & ~int64_t(1);
+            if (words >= 4) {
+                W = kTierMinWindow;
+                seq_entries = std::min(seq_entries, words);
+            }
+        }
         plan.W[t] = (int32_t)W;
         plan.H[t] = (int32_t)(W / 2 - 1);
         plan.seq_cap[t] = (int32_t)seq_entries;
         plan.team_bytes[t] = team_bytes & ~int64_t(15);
         plan.ring_bytes[t] = (int64_t)nslot * W * 2;
-        plan.usable[t] = W >= 64;
+        plan.usable[t] = W >= kTierMinWindow;
         plan.dump_stride[t] = (kDumpHeader + (int64_t)nslot * W * 2 + 255) & ~int64_t(255);
     }
     // G: int32 rings covering [-max(qlen, rlen) - 3, max(qlen, rlen) + 3]

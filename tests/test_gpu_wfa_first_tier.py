@@ -78,6 +78,45 @@ def test_lengths_count_no_further_than_max_error_lets_them(device, oracle):
     assert seen == {(True, 4), (False, 1)}, seen
 
 
+@pytest.mark.parametrize("pen", [(1, 0, 31), (31, 0, 31), (1, 1, 30), (2, 1, 30)])
+def test_penalties_of_many_slots_keep_the_one_warp_tier(device, oracle, pen):
+    """Up to 96 wavefront rows: the one-warp tier's window is 64 diagonals at least, beside
+    sequence copies that then hold no more than some 4,000 bases."""
+    rng = np.random.default_rng(pen[1])
+    q, r = _pairs(rng, 60, 100, 200)
+    lq, lr = _pairs(rng, 4, 4300, 4500)
+    both = []
+    for a, b in ((q, lq), (r, lr)):
+        p, m, o, ln = a.arrays()
+        p2, m2, o2, ln2 = b.arrays()
+        both.append(SequenceBatch.from_arrays(np.concatenate((p, p2)), np.concatenate((m, m2)),
+                                              np.concatenate((o, o2 + p.size)),
+                                              np.concatenate((ln, ln2))))
+    for (a, b), times in (((q, r), 42), (both, 40)):
+        qp, _, qo, ql = a.arrays()
+        rp, _, ro, rl = b.arrays()
+        n = len(ql) * times
+        for me in (100, 400, 3000):
+            want, _ = oracle.wfa_batch(qp, qo, ql, rp, ro, rl, *pen, me, envelope=True)
+            got = device.wfa_affine(_copies(a, n), _copies(b, n), WFAConfig(*pen, me))
+            assert (got == np.resize(want, n)).all(), (pen, me)
+
+
+def test_reads_at_many_slots_start_on_one_warp(device):
+    """100 steps leave the one-warp tier's 64 diagonals, not the four-warp one's: two
+    launches, where one means that the first was left out."""
+    rng = np.random.default_rng(4)
+    q, r = _pairs(rng, 60, 150, 150)
+    dq, dr = device.upload_batch(_copies(q, 2500)), device.upload_batch(_copies(r, 2500))
+    try:
+        device.stats_reset()
+        device.wfa_affine(dq, dr, WFAConfig(1, 0, 31, 100), batched=False)
+        assert device.stats()["launches"] == 2
+    finally:
+        dq.close()
+        dr.close()
+
+
 def test_a_small_batch_of_reads_starts_on_one_warp_per_pair(device):
     """2,500 reads: one launch, without the eight-lane kernel and its second one."""
     rng = np.random.default_rng(1)
