@@ -796,6 +796,8 @@ static int wfa_block_warps(int64_t qmax, int64_t rmax, int64_t n, int variant)
 //     1,200  245 / 343 / 507;  5,000  503 / 996 / 1,820
 //   3,000 bp, 12%, max_error 200, 600 pairs  101 / 173 / 250
 //   500-10,000 bp, 12%, max_error 1,000, 600 pairs  974 / 498 / 823
+// And one warp always where no wavefront passes 64 diagonals, two to a lane (100-3,000 bp,
+// 12%, max_error 50, 150 pairs  57 / 62 / 68;  600  59 / 82 / 104).
 //
 // Pairs of at most kWfaShortLen bases start on eight lanes each, but a pair's steps then
 // take longer: only from kWfaShortMinPairsPerSm per SM on, where the warps of the one-warp
@@ -812,13 +814,15 @@ static int wfa_tiers(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, int64_t qmax, 
     if (n < kWfaTwoWarpMinPairsPerSm * sms)
         pl.usable[1] = false;
     constexpr int G = kWfaShared;  // the global-memory tier
-    const int64_t steps = p.max_error / gcd_h(p.x, gcd_h(p.o, p.e));
+    const int64_t g = gcd_h(p.x, gcd_h(p.o, p.e)), steps = p.max_error / g;
     const int64_t lmax = std::max<int64_t>({qmax, rmax, 1});
     const int64_t longest = std::min(lmax, std::max<int64_t>(4 * steps, 1));
     const double mean = std::max(mean_length(qv, n, longest), mean_length(rv, n, longest));
     const double alike = (double)n * std::pow(mean / (double)longest, 1.5) / (double)sms;
     const double one_warp = longest > 2000 || lmax > kWfaOneWarpCopy ? 6.0 : 4.0;
     int first = alike > one_warp ? 0 : (alike > 1.4 ? 2 : 3);
+    if (2 * std::min(lmax, steps / (p.e / g)) + 1 <= 64)
+        first = 0;
     while (first < G && !pl.usable[first])
         ++first;
     auto next_of = [&](int t) {
