@@ -291,6 +291,8 @@ static int nw_core(gb2_ctx *c, Exec &x, SeqView qv, SeqView rv, const SwParams &
         const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)c->sm_count * 4);
         if ((rc = ensure(c, x.scratch64, (size_t)grid * 128 * stride * 8, x.st)))
             return rc;
+        static std::atomic<uint64_t> done{0};
+        GB2_CU(c, prefer_l1(nw_literal_kernel, done));
         nw_literal_kernel<<<grid, 128, 0, x.st>>>(qv, rv, p, band, d_bands, n, d_out,
                                                   (int64_t *)x.scratch64.p, stride);
         GB2_CU(c, cudaGetLastError());

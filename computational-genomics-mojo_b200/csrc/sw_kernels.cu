@@ -850,6 +850,10 @@ cudaError_t launch_sw(int band_class, int variant, SeqView q, SeqView r, SwParam
     default: {
         if (grid <= 0)
             return cudaErrorInvalidValue;  // the literal kernel needs a sized scratch grid
+        static std::atomic<uint64_t> done{0};
+        const cudaError_t attr = prefer_l1(sw_literal_kernel, done);
+        if (attr != cudaSuccess)
+            return attr;
         sw_literal_kernel<<<grid, 128, 0, st>>>(q, r, p, band, bands, pl, out, scratch,
                                                 scratch_stride);
         return cudaGetLastError();
